@@ -295,24 +295,83 @@ cp::FusedArgs fused_args(cp_instance* I, int precond) {
     return a;
 }
 
-// FP64 CG, one launch per iteration (cg_fused.cu), or the whole solve in one
-// thread-block cluster where the instance fits.
-void cg_fp64_fused(cp_instance* I, double eps, long long max_iter, int precond) {
-    cp::FusedArgs a = fused_args(I, precond);
-    if (I->cluster_fp64) {
-        if (!I->cluster_planned) {
-            I->cluster_plan = cp::cluster_cg_plan(a, I->csr.max_width);
-            I->cluster_planned = 1;
+// The on-chip CG's plan of this instance, built on first use; false when the
+// instance does not fit.
+bool chip_ready(cp_instance* I) {
+    if (!I->on_chip) return false;
+    if (I->chip_planned) return I->chip.ctas > 0;
+    I->chip_planned = 1;
+    for (const bool grid : {false, true}) {
+        const cp::ChipShape sh = cp::chip_shape(I->n_nodes, I->csr.max_width, I->sms(), grid);
+        if (sh.ctas == 0) continue;
+        void* mem = I->alloc<unsigned char>(cp::chip_plan_bytes(sh, I->n_nodes));
+        cp::chip_build_plan(I->chip, sh, mem, I->n_nodes, I->mesh.xy, I->csr.slice_ptr, I->csr.scol, I->sms(), I->s());
+        if (I->chip.ctas == 0) continue;
+        if (grid) {
+            I->chip_ll_bytes = cp::chip_ll_bytes(sh);
+            I->chip_ll = I->alloc<unsigned char>(I->chip_ll_bytes);
+            I->chip_seq = I->alloc<unsigned int>(1);
+            CP_CUDA(cudaMemsetAsync(I->chip_ll, 0, I->chip_ll_bytes, I->s()));
+            CP_CUDA(cudaMemsetAsync(I->chip_seq, 0, sizeof(unsigned int), I->s()));
         }
-        if (I->cluster_plan.ctas > 0) {
-            // one cluster holds the whole solve
-            cp::cluster_cg_launch(a, I->cluster_plan, eps * eps, max_iter, I->s());
-            I->launches += 1;
-            CP_CUDA(cudaMemcpyAsync(I->sc_h, I->sc, sizeof(cp::CgScalars), cudaMemcpyDeviceToHost, I->s()));
-            CP_CUDA(cudaStreamSynchronize(I->s()));
-            return;
-        }
+        break;
     }
+    return I->chip.ctas > 0;
+}
+
+template <typename T>
+cp::ChipArgs<T> chip_args(cp_instance* I, double eps2, long long max_iter, int precond) {
+    cp::ChipArgs<T> a;
+    a.plan = I->chip;
+    a.slice_ptr = I->csr.slice_ptr;
+    a.scol = I->csr.scol;
+    a.val64 = I->csr.val64;
+    a.b = I->b;
+    a.mask = I->mask;
+    a.x = I->u;
+    a.precond = precond;
+    a.sc = I->sc;
+    a.eps2 = eps2;
+    a.max_iter = max_iter;
+    if (I->chip.grid) cp::chip_ll_carve(I->chip, I->chip_ll, &a.ll_rec, &a.ll_part, &a.ll_step);
+    a.seq = I->chip_seq;
+    if (I->test_barrier_ns) {
+        a.poll_limit = 1000;
+        a.seq_skew = 1;
+    }
+    return a;
+}
+
+// After an on-chip solve whose scalars are in sc_h: a CTA that gave up
+// waiting leaves the exchange buffers mid-sequence, so they start afresh.
+void chip_check(cp_instance* I) {
+    if (!I->sc_h->chip_err) return;
+    CP_CUDA(cudaMemsetAsync(I->sc, 0, sizeof(cp::CgScalars), I->s()));
+    if (I->chip.grid) {
+        CP_CUDA(cudaMemsetAsync(I->chip_ll, 0, I->chip_ll_bytes, I->s()));
+        CP_CUDA(cudaMemsetAsync(I->chip_seq, 0, sizeof(unsigned int), I->s()));
+    }
+    throw Error{CP_ERR_TIMEOUT, "on-chip CG: an exchange timed out"};
+}
+
+// One on-chip solve; its scalars end in sc_h.
+template <typename T>
+void run_chip(cp_instance* I, const cp::ChipArgs<T>& a) {
+    cp::chip_launch(a, I->s());
+    I->launches += 1;
+    CP_CUDA(cudaMemcpyAsync(I->sc_h, I->sc, sizeof(cp::CgScalars), cudaMemcpyDeviceToHost, I->s()));
+    CP_CUDA(cudaStreamSynchronize(I->s()));
+    chip_check(I);
+}
+
+// FP64 CG: on chip where the instance fits, else one launch per iteration
+// (cg_fused.cu).
+void cg_fp64_fused(cp_instance* I, double eps, long long max_iter, int precond) {
+    if (chip_ready(I)) {
+        run_chip(I, chip_args<double>(I, eps * eps, max_iter, precond));
+        return;
+    }
+    cp::FusedArgs a = fused_args(I, precond);
     if (I->persistent_fp64 && cp::fused_persistent_fits(a)) {
         // one cooperative launch for the whole solve
         if (I->test_barrier_ns) {
@@ -605,14 +664,14 @@ CP_API int cp_instance_create(cp_context* ctx, const cp_mesh_view* mv, const cp_
     if (!I) return CP_ERR_NOMEM;
     I->ctx = ctx;
     if (const char* g = std::getenv("CUPLAST_NO_GRAPH")) I->use_graph = !(g[0] == '1');
-    // FP64 CG form: one thread-block cluster when the instance fits (default),
-    // else one launch per iteration in a graph; CUPLAST_FP64_CG=fused keeps
-    // the graph loop, =persistent makes it one cooperative launch, =classic
-    // selects the two-kernel loop of cg.cu.
+    // CG form: on chip (cg_chip.cu) when the instance fits (default, or
+    // CUPLAST_FP64_CG=cluster), else one launch per iteration in a graph;
+    // CUPLAST_FP64_CG=fused keeps the graph loop, =persistent makes it one
+    // cooperative launch, =classic selects the two-kernel loop of cg.cu.
     if (const char* g = std::getenv("CUPLAST_FP64_CG")) {
         I->fused_fp64 = std::strcmp(g, "classic") != 0;
         I->persistent_fp64 = std::strcmp(g, "persistent") == 0;
-        I->cluster_fp64 = std::strcmp(g, "cluster") == 0;
+        I->on_chip = std::strcmp(g, "cluster") == 0;
     }
     if (const char* g = std::getenv("CUPLAST_TEST_BARRIER_NS")) I->test_barrier_ns = std::strtoull(g, nullptr, 10);
     int rc = guarded(ctx, [&] {

@@ -85,16 +85,55 @@ bool fused_persistent_fits(const FusedArgs& a);
 void fused_launch_persistent(const FusedArgs& a, double eps2, long long max_iter, cudaStream_t s);
 cudaGraphExec_t fused_build_while_graph(const FusedArgs& a, int body_iters, cudaStream_t s);
 
-// The same solve inside one thread-block cluster (cg_cluster.cu), for
-// instances whose blocks of K and records fit the cluster's shared memory.
-struct ClusterPlan {
-    int ctas = 0;      // cluster size (0: does not fit)
-    int spc = 0;       // slices of 32 nodes per CTA (one warp each)
-    int wmax = 0;      // widest node row, in blocks
-    size_t smem = 0;   // dynamic shared memory per CTA
+// The whole linear solve on chip (cg_chip.cu): one thread-block cluster, or
+// a cooperative grid of up to one CTA per SM.
+struct ChipShape {
+    bool grid = false;
+    int ctas = 0;  // 0: the instance does not fit
+    int spc = 0;   // slices of 32 nodes per CTA (one warp each)
+    int wmax = 0;  // widest node row, in blocks
 };
-ClusterPlan cluster_cg_plan(const FusedArgs& a, int max_width);
-void cluster_cg_launch(const FusedArgs& a, const ClusterPlan& plan, double eps2, long long max_iter, cudaStream_t s);
+struct ChipPlan {
+    bool grid = false;
+    int ctas = 0, spc = 0, wmax = 0;
+    int halo_cap = 0;                // most halo nodes of a CTA (rounded up)
+    int* order = nullptr;            // per slot (CTA, thread): its node, or -1
+    unsigned short* lidx = nullptr;  // per block of a slot's row: index of its column in the CTA's U
+    int* halo = nullptr;             // per CTA: the slots of its halo nodes
+    int* halo_cnt = nullptr;         // per CTA
+    unsigned char* pub = nullptr;    // per slot: in another CTA's halo
+};
+template <typename T>
+struct ChipArgs {
+    ChipPlan plan;
+    const int* slice_ptr = nullptr;
+    const int* scol = nullptr;
+    const double* val64 = nullptr;
+    const double2* b = nullptr;
+    const uchar2* mask = nullptr;
+    double2* x = nullptr;
+    int precond = 0;
+    CgScalars* sc = nullptr;
+    double eps2 = 0.0, outer_eps2 = -1.0;  // as cg_launch_init
+    long long max_iter = 0;
+    int relative_to_r0 = 0;
+    // grid exchange: records, sums and steps by parity, the last sequence
+    // number in use; rounds a poll takes before it gives up, and what is
+    // added to the posted sequence numbers (0; 1 makes every poll run out:
+    // the time-out path's test)
+    uint4 *ll_rec = nullptr, *ll_part = nullptr, *ll_step = nullptr;
+    unsigned int* seq = nullptr;
+    unsigned int poll_limit = 1u << 22;
+    unsigned int seq_skew = 0;
+};
+ChipShape chip_shape(int n, int wmax, int sm_count, bool grid);
+size_t chip_plan_bytes(const ChipShape& s, int n);
+size_t chip_ll_bytes(const ChipShape& s);
+void chip_ll_carve(const ChipPlan& p, void* mem, uint4** rec, uint4** part, uint4** step);
+void chip_build_plan(ChipPlan& p, const ChipShape& s, void* mem, int n, const double2* xy, const int* slice_ptr,
+                     const int* scol, int sm_count, cudaStream_t st);
+template <typename T>
+void chip_launch(const ChipArgs<T>& a, cudaStream_t s);
 
 template <typename T>
 void cg_launch_init(const CgArgs<T>& a, const void* valA, bool valA_is_fp64, double eps2, long long max_iter,

@@ -63,8 +63,7 @@ struct cp_instance {
     // never released, so every wait runs out and the solve ends with
     // CP_ERR_TIMEOUT
     unsigned long long test_barrier_ns = 0;
-    bool cluster_fp64 = true;      // one thread-block cluster when the instance fits (CUPLAST_FP64_CG other than cluster: off)
-    int cluster_planned = 0;       // cluster_plan below is computed (once per instance)
+    bool on_chip = true;           // the on-chip CG when the instance fits (CUPLAST_FP64_CG other than cluster: off)
     double2* pred_u = nullptr;     // level predictor (cp_solve_opts.predict): the last level's u and psi
     double* pred_psi = nullptr;
     // initial guesses from the level's solution increments (cp_solve_opts.recycle, recycle.h), allocated on
@@ -74,7 +73,11 @@ struct cp_instance {
     double *rec_part = nullptr, *rec_y = nullptr;
     unsigned int* rec_ticket = nullptr;
     int rec_cnt = 0, rec_head = 0;
-    cp::ClusterPlan cluster_plan;
+    int chip_planned = 0;          // chip below is computed (once per instance)
+    cp::ChipPlan chip;             // the on-chip CG's plan (cg_chip.cu); chip.ctas = 0: does not fit
+    unsigned char* chip_ll = nullptr;  // its exchange buffers (grid form)
+    size_t chip_ll_bytes = 0;
+    unsigned int* chip_seq = nullptr;
     double2 *f_r = nullptr, *f_w = nullptr, *f_p = nullptr, *f_kp = nullptr, *f_g = nullptr;
     double* f_partials = nullptr;
     cudaGraphExec_t gf[2] = {nullptr, nullptr};  // [precond]

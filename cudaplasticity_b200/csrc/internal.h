@@ -96,6 +96,7 @@ struct CgScalars {
     int lin_done;       // init found the FP64 residual already below the caller's tolerance
     unsigned int ticket;
     unsigned int gen;   // persistent CG: grid-barrier steps released so far
+    int chip_err;       // on-chip CG: a CTA gave up waiting (cleared by the host)
 };
 
 struct OuterScalars {

@@ -17,7 +17,7 @@
 // FP64 (and floatBoost) requests take the same admission path but are solved
 // by cp_solve, one request per lane thread; each lane has its own context
 // (stream), so the lanes' solves and the batch run concurrently. A small
-// request's CG occupies one 16-SM cluster, so several of them share the GPU.
+// request's CG occupies one cluster of up to 16 SMs, so several of them share the GPU.
 #include <cuda_runtime.h>
 
 #include <algorithm>

@@ -85,6 +85,10 @@ bool fused_persistent_fits(const FusedArgs& a);
 void fused_launch_persistent(const FusedArgs& a, double eps2, long long max_iter, cudaStream_t s);
 cudaGraphExec_t fused_build_while_graph(const FusedArgs& a, int body_iters, cudaStream_t s);
 
+// CgScalars.status of an FP32 on-chip solve whose step lost its curvature
+// (internal: never returned to a caller).
+constexpr int CP_ERR_DEGENERATE = 100;
+
 // The whole linear solve on chip (cg_chip.cu): one thread-block cluster, or
 // a cooperative grid of up to one CTA per SM.
 struct ChipShape {

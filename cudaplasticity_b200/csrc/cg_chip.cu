@@ -590,8 +590,7 @@ __global__ void __launch_bounds__(kChipWarps * 32, 1) k_chip(ChipArgs<T> a) {
             else if (!(rho_inv > 0.0) || !(rho > 0.0)) {
                 // in FP32 the step may degenerate before the residual does: the
                 // solve ends there and the caller takes the FP64 residual
-                if (sizeof(T) == 4) converged = 1;
-                else status = CP_ERR_BREAKDOWN;
+                status = sizeof(T) == 4 ? CP_ERR_DEGENERATE : CP_ERR_BREAKDOWN;
             }
             if (!(rr == rr)) status = CP_ERR_BREAKDOWN;
         }

@@ -78,6 +78,7 @@ struct cp_instance {
     unsigned char* chip_ll = nullptr;  // its exchange buffers (grid form)
     size_t chip_ll_bytes = 0;
     unsigned int* chip_seq = nullptr;
+    double2* mix_u0 = nullptr;         // mixed mode on chip: u before the linear solve
     double2 *f_r = nullptr, *f_w = nullptr, *f_p = nullptr, *f_kp = nullptr, *f_g = nullptr;
     double* f_partials = nullptr;
     cudaGraphExec_t gf[2] = {nullptr, nullptr};  // [precond]

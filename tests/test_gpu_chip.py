@@ -104,6 +104,30 @@ def test_wide_rows(n_c, n_r, form, ctx, monkeypatch):
     check(p, *solve(ctx, p), 1e-11)
 
 
+@pytest.mark.parametrize("nx, ny", [(2, 2), (16, 2), (127, 2), (64, 26), (96, 64), (1229, 5), (331, 99)])
+def test_mixed_precision(nx, ny, ctx):
+    """FP32 recurrences inside FP64 defect correction: the solve ends on the FP64 residual itself."""
+    p = strip(nx, ny)
+    for precond in (0, 1):
+        u, rep, csr = solve(ctx, p, precond=precond, precision=cp.CP_PREC_MIXED, inner_tol=1e-3)
+        res, gap = residual(p, u, csr)
+        # one evaluation of b - K u in each arithmetic order: the rounding of a row's at most 18 products
+        assert rep["cg_rel_res"] <= 1e-11 and abs(res - rep["cg_rel_res"]) <= 2 * 20 * EPS64 * gap
+
+
+def test_mixed_precision_falls_back(ctx, monkeypatch):
+    """Where FP32 cannot carry the system (a column 900 elements high and two wide, kappa eps32 >> 1), the on-chip form
+    hands over to the two-kernel loop from the same start: the same outcome as that loop alone."""
+    p = strip(3, 900)
+    out = []
+    for form in ("classic", "cluster"):
+        monkeypatch.setenv("CUPLAST_FP64_CG", form)
+        with pytest.raises(cp.CuplastError) as e:
+            solve(ctx, p, precision=cp.CP_PREC_MIXED, inner_tol=1e-3)
+        out.append(e.value.status)
+    assert out == [cp._capi.CP_ERR_BREAKDOWN] * 2
+
+
 def test_result_is_reproducible_and_independent_of_the_instance(ctx):
     p = strip(120, 80)
     a, b = solve(ctx, p)[0], solve(ctx, p)[0]

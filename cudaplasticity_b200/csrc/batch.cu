@@ -634,14 +634,14 @@ __global__ void __launch_bounds__(kThreads) k_batch_probe(const BDesc* __restric
 template <bool Q8>
 __global__ void __launch_bounds__(kThreads) k_batch_asm(const BDesc* __restrict__ D, BState* SS,
                                                         const int4* __restrict__ tiles, BCtl* c, int max_width) {
-    extern __shared__ double sacc[];
+    extern __shared__ double2 sacc[];
     __shared__ int shf, shp;
     {
         const volatile int* pop = c->pop;
         if (pop[PH_ASM] == 0) return;
     }
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    double* acc = sacc + (size_t)w * 128 * max_width;
+    double2* acc = sacc + (size_t)w * 64 * max_width;
     const int nt = c->n_tiles;
     for (int t = blockIdx.x; t < nt; t += gridDim.x) {
         const int4 tl = tiles[t];
@@ -651,12 +651,12 @@ __global__ void __launch_bounds__(kThreads) k_batch_asm(const BDesc* __restrict_
         const int sl0 = tl.y * tl.z, sl1 = min(sl0 + tl.z, d.n_slices);
         for (int sl = sl0 + w; sl < sl1; sl += kWarps) {
             const int base = d.slice_ptr[sl], wd = (d.slice_ptr[sl + 1] - base) >> 5;
-            const int len = 128 * wd;
-            for (int i = lane; i < len; i += 32) acc[i] = 0.0;
+            const int len = 64 * wd;
+            for (int i = lane; i < len; i += 32) acc[i] = make_double2(0.0, 0.0);
             __syncwarp();
             const int n = 32 * sl + lane;
             if (n < d.m.n_nodes) {
-                double* nb = acc + 4 * lane;
+                const RowAcc nb = row_acc(acc, lane);
                 for (int q = d.inc_pos[n]; q < d.inc_pos[n + 1]; ++q) {
                     const int code = d.inc[q];
                     const int e = code >> 3, i = code & 7;
@@ -665,12 +665,12 @@ __global__ void __launch_bounds__(kThreads) k_batch_asm(const BDesc* __restrict_
                 }
             }
             __syncwarp();
-            double* o64 = d.val64 + 4LL * base;
-            float* o32 = d.val32 + 4LL * base;
+            double2* o64 = reinterpret_cast<double2*>(d.val64 + 4LL * base);
+            float2* o32 = reinterpret_cast<float2*>(d.val32 + 4LL * base);
             for (int i = lane; i < len; i += 32) {
-                const double v = acc[i];
+                const double2 v = acc[row_unit(i)];
                 o64[i] = v;
-                o32[i] = (float)v;
+                o32[i] = make_float2((float)v.x, (float)v.y);
             }
             __syncwarp();
         }

@@ -22,37 +22,57 @@ constexpr int kAsmThreads = 128;  // = 4 slices of 32 nodes
 // One thread per node, one block per tile of 4 slices. The tile's blocks are
 // one contiguous range of values in the sliced layout, accumulated in shared
 // memory (each thread only touches its own node's blocks: no atomics, and the
-// summation order is the element order) and written out coalesced, once.
+// summation order is the element order) and written out coalesced, once. The
+// next incidence's element is loaded ahead of the current one's arithmetic.
+// On the 1,048,576-quad plate 135 us (2.86 TB/s of its 386 MB) against 238
+// before the moment form of the element rows, the bank-conflict-free
+// accumulators and one block per tile in place of 8 per SM (6 fit: a second
+// wave a third full); 4096 quads 8.3 against 12.4 us. It is bound by the
+// latency of its gathers; fewer registers (6 or 8 blocks per SM) lose: 156,
+// 191 us.
 template <bool W64, bool W32, bool Q8>
-__global__ void __launch_bounds__(kAsmThreads) k_assemble(DevMesh m, DevCsr csr, MaterialDev M, const double* E_c,
-                                                          const double* nu_c) {
-    extern __shared__ double sacc[];
-    const int ntiles = (m.n_nodes + kAsmThreads - 1) / kAsmThreads;
-    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        const int s0 = 4 * tile, s1 = min(s0 + 4, csr.n_slices);
-        const long long B0 = csr.slice_ptr[s0], B1 = csr.slice_ptr[s1];
-        const int len = (int)(4 * (B1 - B0));
-        for (int t = threadIdx.x; t < len; t += blockDim.x) sacc[t] = 0.0;
-        __syncthreads();
-        const int n = tile * kAsmThreads + threadIdx.x;
-        if (n < m.n_nodes) {
-            double* nb = sacc + 4 * (csr.slice_ptr[n >> 5] - B0 + (n & 31));
-            for (int q = csr.inc_pos[n]; q < csr.inc_pos[n + 1]; ++q) {
-                const int code = csr.inc[q];
-                const int e = code >> 3, i = code & 7;
-                const Dmat d = form_d(M.plane, E_c[e], nu_c[e]);
-                element_rows<Q8>(m, e, i, csr.inc_k[q], Q8 ? csr.inc_k8[q] : 0u, d, M.h, nb);
+__global__ void __launch_bounds__(kAsmThreads) k_assemble(DevMesh m, DevCsr csr, MaterialDev M,
+                                                          const double* __restrict__ E_c,
+                                                          const double* __restrict__ nu_c) {
+    extern __shared__ double2 sacc[];
+    const int s0 = 4 * blockIdx.x, s1 = min(s0 + 4, csr.n_slices);
+    const long long B0 = csr.slice_ptr[s0], B1 = csr.slice_ptr[s1];
+    const int len = (int)(2 * (B1 - B0));
+    const int n = blockIdx.x * kAsmThreads + threadIdx.x;
+    int q = 0, q1 = 0, code = 0;
+    double Ec = 1.0, nuc = 0.0;
+    if (n < m.n_nodes) {
+        q = csr.inc_pos[n];
+        q1 = csr.inc_pos[n + 1];
+        if (q < q1) {
+            code = csr.inc[q];
+            Ec = E_c[code >> 3];
+            nuc = nu_c[code >> 3];
+        }
+    }
+    for (int t = threadIdx.x; t < len; t += blockDim.x) sacc[t] = make_double2(0.0, 0.0);
+    __syncthreads();
+    if (n < m.n_nodes) {
+        const RowAcc nb = row_acc(sacc + 2 * (csr.slice_ptr[n >> 5] - B0), n & 31);
+        while (q < q1) {
+            const int e = code >> 3, i = code & 7;
+            const Dmat d = form_d(M.plane, Ec, nuc);
+            const uint32_t kk = csr.inc_k[q], kk8 = Q8 ? csr.inc_k8[q] : 0u;
+            if (++q < q1) {
+                code = csr.inc[q];
+                Ec = E_c[code >> 3];
+                nuc = nu_c[code >> 3];
             }
+            element_rows<Q8>(m, e, i, kk, kk8, d, M.h, nb);
         }
-        __syncthreads();
-        double* out64 = csr.val64 + 4 * B0;
-        float* out32 = W32 ? csr.val32 + 4 * B0 : nullptr;
-        for (int t = threadIdx.x; t < len; t += blockDim.x) {
-            double v = sacc[t];
-            if (W64) out64[t] = v;
-            if (W32) out32[t] = (float)v;
-        }
-        __syncthreads();
+    }
+    __syncthreads();
+    double2* out64 = reinterpret_cast<double2*>(csr.val64 + 4 * B0);
+    float2* out32 = W32 ? reinterpret_cast<float2*>(csr.val32 + 4 * B0) : nullptr;
+    for (int t = threadIdx.x; t < len; t += blockDim.x) {
+        const double2 v = sacc[row_unit(t)];
+        if (W64) out64[t] = v;
+        if (W32) out32[t] = make_float2((float)v.x, (float)v.y);
     }
 }
 
@@ -65,8 +85,12 @@ constexpr int kElemThreads = 256;
 // last assembly, stress intensity, secant update, and the two exit-norm sums
 // (reduced deterministically by the last block). With Aitken on, the raw
 // secant target psi is stored as a residual and the relax kernel moves psi.
+// 4 blocks per SM (64 registers) for the latency of the gathers, and a grid
+// that fits once, so that the block sums and their fence are paid once per
+// block: 1,048,576 quads with Hollomon hardening, whole call 128 us before
+// the moment form, 85 at 2 blocks per SM, 74 now (floor 26: 168 MB).
 template <bool Q8>
-__global__ void __launch_bounds__(kElemThreads) k_update(DevMesh m, MaterialDev M, const double2* __restrict__ u,
+__global__ void __launch_bounds__(kElemThreads, 4) k_update(DevMesh m, MaterialDev M, const double2* __restrict__ u,
                                                          ElemState st, OuterScalars* sc, double* partials, int aitken) {
     __shared__ double sh[2 * kElemThreads / 32];
     __shared__ bool last;
@@ -141,8 +165,7 @@ void launch_assemble(const DevMesh& m, const DevCsr& csr, const MaterialDev& mat
     const int ntiles = (m.n_nodes + kAsmThreads - 1) / kAsmThreads;
     const size_t smem = (size_t)kAsmThreads * 4 * csr.max_width * sizeof(double);
     CP_CHECK(smem <= 200 * 1024, CP_ERR_UNSUPPORTED, "node degree too large for the assembly tile");
-    int grid = ntiles < sm_count * 8 ? ntiles : sm_count * 8;
-    if (grid < 1) grid = 1;
+    const int grid = std::max(ntiles, 1);
     if (m.c8)
         assemble_as<true>(m, csr, mat, E_c, nu_c, want64, want32, grid, smem, s);
     else
@@ -150,8 +173,13 @@ void launch_assemble(const DevMesh& m, const DevCsr& csr, const MaterialDev& mat
     CP_CUDA(cudaGetLastError());
 }
 
+// Threads per block of the element kernels: small meshes in small blocks, so
+// that they spread over the SMs (4096 quads: 64 blocks of 64).
+int elem_threads(int ne, int sm_count) { return ne <= 2 * 64 * sm_count ? 64 : kElemThreads; }
+
 int update_grid(int ne, int sm_count) {
-    int g = (ne + kElemThreads - 1) / kElemThreads;
+    const int t = elem_threads(ne, sm_count);
+    int g = (ne + t - 1) / t;
     int cap = sm_count * 4;
     return g < 1 ? 1 : (g < cap ? g : cap);
 }
@@ -160,22 +188,22 @@ void launch_update(const DevMesh& m, const MaterialDev& mat, const double2* u, E
                    double* partials, int aitken, cudaStream_t s, int sm_count) {
     const int ne = m.c3 + m.c4 + m.c8;
     if (m.c8)
-        k_update<true><<<update_grid(ne, sm_count), kElemThreads, 0, s>>>(m, mat, u, st, sc, partials, aitken);
+        k_update<true><<<update_grid(ne, sm_count), elem_threads(ne, sm_count), 0, s>>>(m, mat, u, st, sc, partials, aitken);
     else
-        k_update<false><<<update_grid(ne, sm_count), kElemThreads, 0, s>>>(m, mat, u, st, sc, partials, aitken);
+        k_update<false><<<update_grid(ne, sm_count), elem_threads(ne, sm_count), 0, s>>>(m, mat, u, st, sc, partials, aitken);
     CP_CUDA(cudaGetLastError());
 }
 
 void launch_aitken_relax(const DevMesh& m, const MaterialDev& mat, ElemState& st, const OuterScalars* sc, double w,
                          cudaStream_t s, int sm_count) {
     const int ne = m.c3 + m.c4 + m.c8;
-    k_aitken<<<update_grid(ne, sm_count), kElemThreads, 0, s>>>(m, mat, st, sc, w);
+    k_aitken<<<update_grid(ne, sm_count), elem_threads(ne, sm_count), 0, s>>>(m, mat, st, sc, w);
     CP_CUDA(cudaGetLastError());
 }
 
 void launch_plastic(const DevMesh& m, const MaterialDev& mat, ElemState& st, cudaStream_t s, int sm_count) {
     const int ne = m.c3 + m.c4 + m.c8;
-    k_plastic<<<update_grid(ne, sm_count), kElemThreads, 0, s>>>(ne, mat, st);
+    k_plastic<<<update_grid(ne, sm_count), elem_threads(ne, sm_count), 0, s>>>(ne, mat, st);
     CP_CUDA(cudaGetLastError());
 }
 
@@ -261,8 +289,9 @@ extern "C" CP_API int cp_secant_update_noalloc(void* stream, const cp_material* 
     es.sxx = d_fields + 4 * ne; es.syy = d_fields + 5 * ne; es.tau = d_fields + 6 * ne; es.sig_i = d_fields + 7 * ne;
     es.table_s = d_fields + 8 * ne;
     es.psi = d_psi; es.E_c = d_E_c; es.nu_c = d_nu_c;
-    const int grid = (count4 + cp::kElemThreads - 1) / cp::kElemThreads;  // <= kNoAllocMaxBlocks
-    cp::k_update<false><<<grid, cp::kElemThreads, 0, s>>>(m, M, reinterpret_cast<const double2*>(d_uv), es, sc, partials, 0);
+    const int threads = cp::elem_threads(count4, 148);
+    const int grid = cp::update_grid(count4, 148);  // <= kNoAllocMaxBlocks
+    cp::k_update<false><<<grid, threads, 0, s>>>(m, M, reinterpret_cast<const double2*>(d_uv), es, sc, partials, 0);
     if (cudaGetLastError() != cudaSuccess) return CP_ERR_CUDA;
     double host_err = 0.0;
     if (cudaMemcpyAsync(&host_err, &sc->rel_err, sizeof(double), cudaMemcpyDeviceToHost, s) != cudaSuccess)

@@ -37,26 +37,35 @@ __device__ __forceinline__ Dmat form_d(int plane, double E, double nu) {
     return d;
 }
 
-// calcB4 (src/PlasticitySolver.cu:26-64) at Gauss point (r, s): shape-function
-// gradients bx[k] = dN_k/dx, by[k] = dN_k/dy and detJ.
-__device__ __forceinline__ double q4_grad(const double* x, const double* y, double r, double s, double* bx,
-                                          double* by) {
-    double J0 = 0.25 * ((1. + s) * x[0] - (1. + s) * x[1] - (1. - s) * x[2] + (1. - s) * x[3]);
-    double J2 = 0.25 * ((1. + r) * x[0] + (1. - r) * x[1] - (1. - r) * x[2] - (1. + r) * x[3]);
-    double J1 = 0.25 * ((1. + s) * y[0] - (1. + s) * y[1] - (1. - s) * y[2] + (1. - s) * y[3]);
-    double J3 = 0.25 * ((1. + r) * y[0] + (1. - r) * y[1] - (1. - r) * y[2] - (1. + r) * y[3]);
-    double det = J0 * J3 - J1 * J2;
-    double inv = 1. / det;
-    double i0 = J3 * inv, i1 = -J1 * inv, i2 = -J2 * inv, i3 = J0 * inv;
-    bx[0] = 0.25 * ((1. + s) * i0 + (1. + r) * i1);
-    by[0] = 0.25 * ((1. + s) * i2 + (1. + r) * i3);
-    bx[1] = 0.25 * ((-1. - s) * i0 + (1. - r) * i1);
-    by[1] = 0.25 * ((-1. - s) * i2 + (1. - r) * i3);
-    bx[2] = 0.25 * ((-1. + s) * i0 - (1. - r) * i1);
-    by[2] = 0.25 * ((-1. + s) * i2 - (1. - r) * i3);
-    bx[3] = 0.25 * ((1. - s) * i0 - (1. + r) * i1);
-    by[3] = 0.25 * ((1. - s) * i2 - (1. + r) * i3);
-    return det;
+// The 4-node quad (calcB4, src/PlasticitySolver.cu:26-64) in the basis of its
+// nodes' signs r = (1, -1, -1, 1), s = (1, 1, -1, -1), h = r s: for a nodal
+// field f, with f_a = r.f, f_b = s.f, f_h = h.f, four times its derivatives at
+// the Gauss point (sr q, ss q), sr, ss = +-1, are
+//   f_r = f_a + ss q f_h,  f_s = f_b + sr q f_h
+// two values each over the four points, so the whole element costs 7 sums and
+// 4 fused operations per field instead of a Jacobian and 8 gradients per
+// point. All factors of 4 cancel or go into the weights.
+struct QuadField {
+    double rp, rm, sp, sm;  // f_r at ss = +, -; f_s at sr = +, -
+};
+__device__ __forceinline__ QuadField quad_field(double f0, double f1, double f2, double f3) {
+    const double p = f0 - f2, q = f1 - f3;
+    const double fa = p - q, fb = p + q, fh = kGp * ((f0 + f2) - (f1 + f3));
+    return {fa + fh, fa - fh, fb + fh, fb - fh};
+}
+// 1 / x and 1 / y by one division.
+__device__ __forceinline__ void inv2(double x, double y, double& ix, double& iy) {
+    const double t = 1.0 / (x * y);
+    ix = y * t;
+    iy = x * t;
+}
+// Reciprocals of the four determinants (16 times the true ones) at (sr, ss) =
+// (+,+), (+,-), (-,+), (-,-).
+__device__ __forceinline__ void quad_inv_det(const QuadField& x, const QuadField& y, double* w) {
+    const double d0 = x.rp * y.sp - y.rp * x.sp, d1 = x.rm * y.sp - y.rm * x.sp;
+    const double d2 = x.rp * y.sm - y.rp * x.sm, d3 = x.rm * y.sm - y.rm * x.sm;
+    inv2(d0, d1, w[0], w[1]);
+    inv2(d2, d3, w[2], w[3]);
 }
 
 // calcB8 (src/PlasticitySolver.cu:67-134) at (r, s): gradients and detJ of the
@@ -134,22 +143,40 @@ __device__ __forceinline__ int nth(const int4& v, int j) {
     return j == 0 ? v.x : (j == 1 ? v.y : (j == 2 ? v.z : v.w));
 }
 
-// Row-block (i, all j) of element e's stiffness, scaled by h, added into the
-// owning node's 2x2 blocks through the slot bytes kk (block index k of local
-// node j; kk8 for local nodes 4..7 of an 8-node element); block k of the node
-// starts at nb + 128 k (sliced layout, 32 nodes x 4 values per block row).
-// Q8 = false compiles the 8-node branch out (it needs about 50 registers
-// more), for meshes without 8-node elements.
-__device__ __forceinline__ void add_scaled(double* b, const double* blk, double h) {
-    b[0] = __dadd_rn(b[0], __dmul_rn(blk[0], h));
-    b[1] = __dadd_rn(b[1], __dmul_rn(blk[1], h));
-    b[2] = __dadd_rn(b[2], __dmul_rn(blk[2], h));
-    b[3] = __dadd_rn(b[3], __dmul_rn(blk[3], h));
+// A node's row of 2x2 blocks in the assembly's shared memory. A slice of 32
+// nodes takes 64 double2 per block row k: the upper row of node l's block at
+// unit 64 k + l, the lower one at 64 k + 32 + (l ^ 4). Both the lanes' updates
+// (one half, consecutive nodes) and the copy out (halves in turn) then touch
+// every bank once; with a node's four values side by side each 16-byte access
+// of a warp took twice its wavefronts.
+struct RowAcc {
+    double2 *lo, *hi;
+};
+__device__ __forceinline__ RowAcc row_acc(double2* slice, int lane) { return {slice + lane, slice + 32 + (lane ^ 4)}; }
+// Unit of the t-th double2 of a slice's values in memory order (block row,
+// node, half).
+__device__ __forceinline__ int row_unit(int t) {
+    const int half = t & 1, l = (t >> 1) & 31;
+    return (t & ~63) + 32 * half + (l ^ (half << 2));
+}
+__device__ __forceinline__ void add_to(const RowAcc& a, int k, double k00, double k01, double k10, double k11) {
+    double2 &l = a.lo[64 * k], &h = a.hi[64 * k];
+    const double2 lo = l, hi = h;
+    l = make_double2(__dadd_rn(lo.x, k00), __dadd_rn(lo.y, k01));
+    h = make_double2(__dadd_rn(hi.x, k10), __dadd_rn(hi.y, k11));
+}
+__device__ __forceinline__ void add_scaled(const RowAcc& a, int k, const double* blk, double h) {
+    add_to(a, k, __dmul_rn(blk[0], h), __dmul_rn(blk[1], h), __dmul_rn(blk[2], h), __dmul_rn(blk[3], h));
 }
 
+// Row-block (i, all j) of element e's stiffness, scaled by h, added into the
+// owning node's blocks through the slot bytes kk (block index k of local node
+// j; kk8 for local nodes 4..7 of an 8-node element). Q8 = false compiles the
+// 8-node branch out (it needs about 50 registers more), for meshes without
+// 8-node elements.
 template <bool Q8>
 __device__ __forceinline__ void element_rows(const DevMesh& m, int e, int i, uint32_t kk, uint32_t kk8, const Dmat& d,
-                                             double h, double* nb) {
+                                             double h, const RowAcc& nb) {
     if (Q8 && e >= m.c3 + m.c4) {
         // formKe8 (src/PlasticitySolver.cu:189-224), one Gauss point at a
         // time: each point's block h (B_i^T D B_j) w detJ goes straight into
@@ -178,13 +205,13 @@ __device__ __forceinline__ void element_rows(const DevMesh& m, int e, int i, uin
                 double blk[4] = {0.0, 0.0, 0.0, 0.0};
                 add_block(blk, bxi, byi, bx[j], by[j], d, w);
                 const uint32_t k = j < 4 ? (kk >> (8 * j)) & 0xffu : (kk8 >> (8 * (j - 4))) & 0xffu;
-                add_scaled(nb + 128 * (int)k, blk, h);
+                add_scaled(nb, (int)k, blk, h);
             }
         }
         return;
     }
-    double x[4], y[4];
     if (e < m.c3) {
+        double x[3], y[3];
         int4 el = m.e3[e];
         for (int a = 0; a < 3; ++a) {
             double2 p = m.xy[nth(el, a)];
@@ -197,31 +224,77 @@ __device__ __forceinline__ void element_rows(const DevMesh& m, int e, int i, uin
 #pragma unroll
         for (int j = 0; j < 3; ++j) add_block(blk[j], bx[i], by[i], bx[j], by[j], d, area);
 #pragma unroll
-        for (int j = 0; j < 3; ++j) add_scaled(nb + 128 * (int)((kk >> (8 * j)) & 0xffu), blk[j], h);
+        for (int j = 0; j < 3; ++j) add_scaled(nb, (int)((kk >> (8 * j)) & 0xffu), blk[j], h);
     } else {
-        int4 el = m.e4[e - m.c3];
-        for (int a = 0; a < 4; ++a) {
-            double2 p = m.xy[nth(el, a)];
-            x[a] = p.x;
-            y[a] = p.y;
-        }
-        double blk[4][4] = {};
-#pragma unroll
-        for (int gi = 0; gi < 2; ++gi)
-#pragma unroll
-            for (int gj = 0; gj < 2; ++gj) {
-                double bx[4], by[4];
-                double r = gi ? kGp : -kGp, s = gj ? kGp : -kGp;
-                double det = q4_grad(x, y, r, s, bx, by);
-                double bxi = bx[0], byi = by[0];
-                if (i == 1) { bxi = bx[1]; byi = by[1]; }
-                else if (i == 2) { bxi = bx[2]; byi = by[2]; }
-                else if (i == 3) { bxi = bx[3]; byi = by[3]; }
-#pragma unroll
-                for (int j = 0; j < 4; ++j) add_block(blk[j], bxi, byi, bx[j], by[j], d, det);
-            }
-#pragma unroll
-        for (int j = 0; j < 4; ++j) add_scaled(nb + 128 * (int)((kk >> (8 * j)) & 0xffu), blk[j], h);
+        // formKe4 (src/PlasticitySolver.cu:157-186): the block of nodes i, j is
+        // a bilinear form in their signs (r_i, s_i, h_i), (r_j, s_j, h_j), so
+        // the element is the 21 moments of its Gauss points' weights with the
+        // three coefficient vectors, and a row is a few signed sums of them:
+        // about 280 FP64 operations per incidence, where the Jacobian,
+        // gradients and products of every point took 800. The moments do not
+        // depend on i, and the sums change only by exact signs under i <-> j,
+        // so K is bitwise symmetric.
+        const int4 el = m.e4[e - m.c3];
+        const double2 p0 = m.xy[el.x], p1 = m.xy[el.y], p2 = m.xy[el.z], p3 = m.xy[el.w];
+        const QuadField X = quad_field(p0.x, p1.x, p2.x, p3.x), Y = quad_field(p0.y, p1.y, p2.y, p3.y);
+        double w[4];
+        quad_inv_det(X, Y, w);
+        const double hw = h * 0.0625;
+        const double w0 = hw * w[0], w1 = hw * w[1], w2 = hw * w[2], w3 = hw * w[3];
+        // 16 det dN/dx = al r - be s + et h with al = y_s, be = y_r, et = ss q al - sr q be;
+        // 16 det dN/dy the same with ax = -x_s, bx = -x_r
+        const double alp = Y.sp, alm = Y.sm, bep = Y.rp, bem = Y.rm;
+        const double axp = -X.sp, axm = -X.sm, bxp = -X.rp, bxm = -X.rm;
+        // et at (+,+) = -at (-,-), at (-,+) = -at (+,-)
+        const double ya = 0.5 * (bep + bem), yb = 0.5 * (alp + alm), xa = 0.5 * (bxp + bxm), xb = 0.5 * (axp + axm);
+        const double e1 = kGp * (yb - ya), e2 = kGp * (yb + ya), f1 = kGp * (xb - xa), f2 = kGp * (xb + xa);
+        const double wrp = w0 + w1, wrm = w2 + w3, wsp = w0 + w2, wsm = w1 + w3, u1 = w0 + w3, u2 = w1 + w2;
+        // moments: xx, yy symmetric (rr, ss, hh, rs, rh, sh), xy full
+        const double arp = alp * wrp, arm = alm * wrm, brp = axp * wrp, brm = axm * wrm;
+        const double xx_rr = alp * arp + alm * arm, xy_rr = axp * arp + axm * arm, yy_rr = axp * brp + axm * brm;
+        const double asp = bep * wsp, asm_ = bem * wsm, bsp = bxp * wsp, bsm = bxm * wsm;
+        const double xx_ss = bep * asp + bem * asm_, xy_ss = bxp * asp + bxm * asm_, yy_ss = bxp * bsp + bxm * bsm;
+        const double g1 = e1 * u1, g2 = e2 * u2, g3 = f1 * u1, g4 = f2 * u2;
+        const double xx_hh = e1 * g1 + e2 * g2, xy_hh = f1 * g1 + f2 * g2, yy_hh = f1 * g3 + f2 * g4;
+        // sums over ss of w be, w et at sr = +, -; over sr of w et at ss = +, -
+        const double Bp = w0 * bep + w1 * bem, Bm = w2 * bep + w3 * bem;
+        const double Cp = w0 * bxp + w1 * bxm, Cm = w2 * bxp + w3 * bxm;
+        const double Ep = w0 * e1 - w1 * e2, Em = w2 * e2 - w3 * e1;
+        const double Fp = w0 * f1 - w1 * f2, Fm = w2 * f2 - w3 * f1;
+        const double Gp = w0 * e1 + w2 * e2, Gm = w1 * e2 + w3 * e1;
+        const double Hp = w0 * f1 + w2 * f2, Hm = w1 * f2 + w3 * f1;
+        const double xx_rs = -(alp * Bp + alm * Bm), yy_rs = -(axp * Cp + axm * Cm);
+        const double xy_rs = -(alp * Cp + alm * Cm), xy_sr = -(axp * Bp + axm * Bm);
+        const double xx_rh = alp * Ep + alm * Em, yy_rh = axp * Fp + axm * Fm;
+        const double xy_rh = alp * Fp + alm * Fm, xy_hr = axp * Ep + axm * Em;
+        const double xx_sh = -(bep * Gp - bem * Gm), yy_sh = -(bxp * Hp - bxm * Hm);
+        const double xy_sh = -(bep * Hp - bem * Hm), xy_hs = -(bxp * Gp - bxm * Gm);
+        // signs of node i; its row's columns: i, same s (i ^ 1), same r (3 - i), opposite (i ^ 2)
+        const double ri = (i == 0 || i == 3) ? 1.0 : -1.0, si = i < 2 ? 1.0 : -1.0, hi = ri * si;
+        double K00[4], K11[4];
+        auto sym_row = [&](double rr, double ss, double hh, double rs, double rh, double sh, double* K) {
+            const double a2 = 2.0 * hi * rs, b2 = 2.0 * si * rh, c2 = 2.0 * ri * sh;
+            K[0] = (rr + ss + hh) + (a2 + b2 + c2);
+            K[1] = (ss - (rr + hh)) - b2;
+            K[2] = (rr - (ss + hh)) - c2;
+            K[3] = (hh - (rr + ss)) - a2;
+        };
+        sym_row(d.c00 * xx_rr + d.c22 * yy_rr, d.c00 * xx_ss + d.c22 * yy_ss, d.c00 * xx_hh + d.c22 * yy_hh,
+                d.c00 * xx_rs + d.c22 * yy_rs, d.c00 * xx_rh + d.c22 * yy_rh, d.c00 * xx_sh + d.c22 * yy_sh, K00);
+        sym_row(d.c11 * yy_rr + d.c22 * xx_rr, d.c11 * yy_ss + d.c22 * xx_ss, d.c11 * yy_hh + d.c22 * xx_hh,
+                d.c11 * yy_rs + d.c22 * xx_rs, d.c11 * yy_rh + d.c22 * xx_rh, d.c11 * yy_sh + d.c22 * xx_sh, K11);
+        // c01 xy + c22 xy^T: symmetric and antisymmetric parts
+        const double cs = d.c01 + d.c22, ca = d.c01 - d.c22;
+        const double rr = cs * xy_rr, ss = cs * xy_ss, hh = cs * xy_hh;
+        const double q0 = hi * cs * (xy_rs + xy_sr), q1 = si * cs * (xy_rh + xy_hr), q2 = ri * cs * (xy_sh + xy_hs);
+        const double d0 = hi * ca * (xy_rs - xy_sr), d1 = si * ca * (xy_rh - xy_hr), d2 = ri * ca * (xy_sh - xy_hs);
+        const double b0 = (rr + ss + hh) + (q0 + q1 + q2), b1 = (ss - (rr + hh)) - q1, b2 = (rr - (ss + hh)) - q2,
+                     b3 = (hh - (rr + ss)) - q0;
+        const double t1 = d0 - d2, t2 = -(d0 + d1), t3 = d1 + d2;
+        add_to(nb, (int)((kk >> (8 * i)) & 0xffu), K00[0], b0, b0, K11[0]);
+        add_to(nb, (int)((kk >> (8 * (i ^ 1))) & 0xffu), K00[1], b1 + t1, b1 - t1, K11[1]);
+        add_to(nb, (int)((kk >> (8 * (3 - i))) & 0xffu), K00[2], b2 + t2, b2 - t2, K11[2]);
+        add_to(nb, (int)((kk >> (8 * (i ^ 2))) & 0xffu), K00[3], b3 + t3, b3 - t3, K11[3]);
     }
 }
 
@@ -243,18 +316,20 @@ __device__ double diagram_f(const MaterialDev& M, double eps) {
                                 A * pow(E / (A * mm), mm / (mm - 1.));
     }
     case CP_DIAGRAM_HOLLOMON: {
-        // eps = s/E + eps0((s/sy)^(1/n) - 1), inverted by Newton from s = sy
-        double sy = M.sigma_t, e0 = M.eps0, n = M.n, s = sy;
-        if (eps < sy / E) return eps * E;
+        // eps = s/E + eps0((s/sy)^(1/n) - 1) for s, by Newton in y = ln(s/sy):
+        // two exponentials per step. It starts from above (s/E taken at s =
+        // sy), where the convex function brings every step down towards the
+        // root, quadratically: 3 or 4 steps.
+        const double sy = M.sigma_t, e0 = M.eps0, in = 1.0 / M.n, ey = sy / E;
+        if (eps < ey) return eps * E;
+        double y = M.n * log1p((eps - ey) / e0);
         for (int it = 0; it < 200; ++it) {
-            double t = pow(s / sy, 1.0 / n);
-            double g = s / E + e0 * (t - 1.0) - eps;
-            double dg = 1.0 / E + e0 * t / (n * s);
-            double ds = g / dg;
-            s -= ds;
-            if (fabs(ds) <= 1e-15 * s) break;
+            const double a = ey * exp(y), b = e0 * exp(y * in);
+            const double dy = ((a + b) - (e0 + eps)) / (a + b * in);
+            y -= dy;
+            if (!(fabs(dy) > 1e-10)) break;
         }
-        return s;
+        return sy * exp(y);
     }
     case CP_DIAGRAM_PIECEWISE: {
         if (eps < M.pw_eps[0]) return eps * E;
@@ -280,6 +355,7 @@ __device__ __forceinline__ void update_element(const DevMesh& m, const MaterialD
                                                const ElemState& st, int e, int aitken, double& s_num, double& s_den,
                                                double& s_an, double& s_ad) {
     const double E0 = M.E, nu0 = M.nu;
+    const double Ec = st.E_c[e], nuc = st.nu_c[e];
     double ex, ey, g;
     if (e < m.c3) {
         int4 el = m.e3[e];
@@ -323,29 +399,27 @@ __device__ __forceinline__ void update_element(const DevMesh& m, const MaterialD
         }
         ex *= 0.25; ey *= 0.25; g *= 0.25;
     } else {
-        int4 el = m.e4[e - m.c3];
-        double x[4], y[4], uu[4], vv[4];
-        for (int a = 0; a < 4; ++a) {
-            int nd = nth(el, a);
-            double2 p = m.xy[nd], w = u[nd];
-            x[a] = p.x; y[a] = p.y; uu[a] = w.x; vv[a] = w.y;
-        }
+        // the mean over the Gauss points, from the fields' derivatives there
+        const int4 el = m.e4[e - m.c3];
+        const double2 p0 = m.xy[el.x], p1 = m.xy[el.y], p2 = m.xy[el.z], p3 = m.xy[el.w];
+        const double2 w0 = u[el.x], w1 = u[el.y], w2 = u[el.z], w3 = u[el.w];
+        const QuadField X = quad_field(p0.x, p1.x, p2.x, p3.x), Y = quad_field(p0.y, p1.y, p2.y, p3.y);
+        const QuadField U = quad_field(w0.x, w1.x, w2.x, w3.x), V = quad_field(w0.y, w1.y, w2.y, w3.y);
+        double w[4];
+        quad_inv_det(X, Y, w);
         ex = 0.0; ey = 0.0; g = 0.0;
 #pragma unroll
-        for (int gi = 0; gi < 2; ++gi)
-#pragma unroll
-            for (int gj = 0; gj < 2; ++gj) {
-                double bx[4], by[4];
-                q4_grad(x, y, gi ? kGp : -kGp, gj ? kGp : -kGp, bx, by);
-                ex += uu[0] * bx[0] + uu[1] * bx[1] + uu[2] * bx[2] + uu[3] * bx[3];
-                ey += vv[0] * by[0] + vv[1] * by[1] + vv[2] * by[2] + vv[3] * by[3];
-                g += uu[0] * by[0] + uu[1] * by[1] + uu[2] * by[2] + uu[3] * by[3] + vv[0] * bx[0] +
-                     vv[1] * bx[1] + vv[2] * bx[2] + vv[3] * bx[3];
-            }
+        for (int q = 0; q < 4; ++q) {
+            const double xr = q & 1 ? X.rm : X.rp, xs = q & 2 ? X.sm : X.sp, yr = q & 1 ? Y.rm : Y.rp,
+                         ys = q & 2 ? Y.sm : Y.sp, ur = q & 1 ? U.rm : U.rp, us = q & 2 ? U.sm : U.sp,
+                         vr = q & 1 ? V.rm : V.rp, vs = q & 2 ? V.sm : V.sp;
+            ex += (ur * ys - us * yr) * w[q];
+            ey += (vs * xr - vr * xs) * w[q];
+            g += ((us * xr - ur * xs) + (vr * ys - vs * yr)) * w[q];
+        }
         ex *= 0.25; ey *= 0.25; g *= 0.25;
     }
-    const double Ec = st.E_c[e];
-    const Dmat d = form_d(M.plane, Ec, st.nu_c[e]);
+    const Dmat d = form_d(M.plane, Ec, nuc);
     const double sx = d.c00 * ex + d.c01 * ey;
     const double sy = d.c01 * ex + d.c11 * ey;
     const double t = d.c22 * g;
@@ -360,9 +434,10 @@ __device__ __forceinline__ void update_element(const DevMesh& m, const MaterialD
     s_num += diff * diff;
     s_den += tab * tab;
     if (!aitken) {
+        const double ips = 1.0 / ps;
         st.psi[e] = ps;
-        st.E_c[e] = E0 / ps;
-        st.nu_c[e] = 0.5 * (1. - (1. - 2. * nu0) / ps);
+        st.E_c[e] = E0 * ips;
+        st.nu_c[e] = 0.5 * (1. - (1. - 2. * nu0) * ips);
     } else {
         const double r = (ps == ps) ? ps - st.psi[e] : 0.0;
         const double dr = r - st.res_prev[e];

@@ -94,12 +94,13 @@ constexpr int CP_ERR_DEGENERATE = 100;
 struct ChipShape {
     bool grid = false;
     int ctas = 0;  // 0: the instance does not fit
-    int spc = 0;   // slices of 32 nodes per CTA (one warp each)
+    int spc = 0;   // slices of 32 nodes per CTA
+    int npt = 1;   // nodes per thread
     int wmax = 0;  // widest node row, in blocks
 };
 struct ChipPlan {
     bool grid = false;
-    int ctas = 0, spc = 0, wmax = 0;
+    int ctas = 0, spc = 0, npt = 1, wmax = 0;
     int halo_cap = 0;                // most halo nodes of a CTA (rounded up)
     int* order = nullptr;            // per slot (CTA, thread): its node, or -1
     unsigned short* lidx = nullptr;  // per block of a slot's row: index of its column in the CTA's U

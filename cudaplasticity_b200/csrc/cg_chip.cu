@@ -35,6 +35,7 @@
 #include <cstdlib>
 
 #include "cg.h"
+#include "chip.cuh"
 #include "common.cuh"
 #include "internal.h"
 
@@ -42,12 +43,6 @@ namespace cp {
 
 namespace {
 
-constexpr int kRegBlocks = 9;        // blocks of a row in registers (a 4-node mesh's interior row)
-constexpr int kChipWarps = 12;       // slices per CTA: 384 threads of 168 registers
-constexpr int kMaxCluster = 16;
-constexpr int kSums = 5;
-constexpr int kMaxPolls = 8;         // warps that poll the CTAs' sums (grid): up to 256 CTAs
-constexpr int kHaloMax = 4096;       // halo nodes per CTA
 constexpr size_t kSmemCap = 220 * 1024;
 constexpr int kPlanThreads = 256;
 constexpr int kOrderThreads = 1024;
@@ -222,328 +217,110 @@ __global__ void __launch_bounds__(kPlanThreads) k_chip_plan(int slots, int own, 
     }
 }
 
-// --------------------------------------------------------------- helpers --
-
-__device__ __forceinline__ unsigned int smem_addr(const void* p) {
-    return (unsigned int)__cvta_generic_to_shared(p);
-}
-__device__ __forceinline__ unsigned int mapa(unsigned int addr, int rank) {
-    unsigned int r;
-    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
-    return r;
-}
-__device__ __forceinline__ void ld_cluster(unsigned int a, double2& v) {
-    asm volatile("ld.shared::cluster.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "r"(a) : "memory");
-}
-__device__ __forceinline__ void ld_cluster(unsigned int a, float2& v) {
-    asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a) : "memory");
-}
-// Two doubles into another CTA's shared memory; they count 16 bytes towards
-// the phase of the mbarrier there.
-__device__ __forceinline__ void st_async(unsigned int a, unsigned int bar, double x, double y) {
-    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.b64 [%0], {%1, %2}, [%3];" ::"r"(a),
-                 "l"(__double_as_longlong(x)), "l"(__double_as_longlong(y)), "r"(bar)
-                 : "memory");
-}
-__device__ __forceinline__ void bar_init(unsigned int bar) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void bar_expect(unsigned int bar, unsigned int bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ bool bar_try(unsigned int bar, unsigned int phase) {
-    unsigned int ok;
-    asm volatile(
-        "{ .reg .pred p; mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
-        : "=r"(ok)
-        : "r"(bar), "r"(phase)
-        : "memory");
-    return ok != 0;
-}
-// Shared-memory reads of U by byte address.
-__device__ __forceinline__ void ld_u(unsigned int a, double2& v) {
-    asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "r"(a) : "memory");
-}
-__device__ __forceinline__ void ld_u(unsigned int a, float2& v) {
-    asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a) : "memory");
-}
-__device__ __forceinline__ void cluster_arrive_release() {
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void cluster_wait() {
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-
-// Two words of (32 bits of data, sequence number).
-__device__ __forceinline__ uint4 ld_words(const uint4* p) {
-    uint4 v;
-    asm volatile("ld.volatile.global.v4.u32 {%0, %1, %2, %3}, [%4];"
-                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-                 : "l"(p)
-                 : "memory");
-    return v;
-}
-__device__ __forceinline__ void st_words(uint4* p, unsigned int lo, unsigned int hi, unsigned int seq) {
-    asm volatile("st.volatile.global.v4.u32 [%0], {%1, %2, %3, %4};" ::"l"(p), "r"(lo), "r"(seq), "r"(hi), "r"(seq)
-                 : "memory");
-}
-__device__ __forceinline__ void post(uint4* p, double v, unsigned int seq) {
-    st_words(p, __double2loint(v), __double2hiint(v), seq);
-}
-__device__ __forceinline__ void post(uint4* p, float2 v, unsigned int seq) {
-    st_words(p, __float_as_uint(v.x), __float_as_uint(v.y), seq);
-}
-__device__ __forceinline__ double word_value(const uint4& q) { return __hiloint2double(q.z, q.x); }
-
-// Polls N word pairs per lane until those of every lane of the warp carry seq;
-// false after `limit` rounds. The whole warp takes part, with valid addresses
-// in every lane: left to diverge, a warp of which some lanes polled and some
-// did not took 3700 cycles to come together again.
-template <int N>
-__device__ __forceinline__ bool poll(const uint4* p, size_t stride, unsigned int seq, unsigned int limit, uint4* c) {
-    for (unsigned int round = 0; round < limit; ++round) {
-        bool ok = true;
-#pragma unroll
-        for (int i = 0; i < N; ++i) c[i] = ld_words(p + i * stride);
-#pragma unroll
-        for (int i = 0; i < N; ++i) ok = ok && c[i].y == seq && c[i].w == seq;
-        if (__all_sync(0xffffffffu, ok)) return true;
-    }
-    return false;
-}
-
-// A record (u, M w, M kp): pair i at p[i * stride].
-template <typename T>
-struct Record;
-template <>
-struct Record<double> {
-    static constexpr int n = 6;
-    __device__ static void put(uint4* p, size_t stride, double2 u, double2 mw, double2 mk, unsigned int seq) {
-        post(p, u.x, seq);
-        post(p + stride, u.y, seq);
-        post(p + 2 * stride, mw.x, seq);
-        post(p + 3 * stride, mw.y, seq);
-        post(p + 4 * stride, mk.x, seq);
-        post(p + 5 * stride, mk.y, seq);
-    }
-    __device__ static void get(const uint4* c, double2* r) {
-#pragma unroll
-        for (int i = 0; i < 3; ++i) r[i] = make_double2(word_value(c[2 * i]), word_value(c[2 * i + 1]));
-    }
-};
-template <>
-struct Record<float> {
-    static constexpr int n = 3;
-    __device__ static void put(uint4* p, size_t stride, float2 u, float2 mw, float2 mk, unsigned int seq) {
-        post(p, u, seq);
-        post(p + stride, mw, seq);
-        post(p + 2 * stride, mk, seq);
-    }
-    __device__ static void get(const uint4* c, float2* r) {
-#pragma unroll
-        for (int i = 0; i < 3; ++i) r[i] = make_float2(__uint_as_float(c[i].x), __uint_as_float(c[i].z));
-    }
-};
-constexpr int kStepWords = 3;  // alpha, beta, go
-
-template <typename V2>
-__device__ __forceinline__ V2 make2(decltype(V2::x) x, decltype(V2::x) y) {
-    V2 v;
-    v.x = x;
-    v.y = y;
-    return v;
-}
-
-// Sums of the five values over the warp in 8 shuffles instead of 25 (the
-// shuffle unit takes one warp per cycle and SM): each step folds two values
-// into one register per half of the lanes. Lanes 0..3 end with v0, 4..7 with
-// v2, 8..15 with v1, 16..23 with v3, 24..31 with v4; every fourth lane stores
-// (slot lane / 4 of 8), and sum_slot(i) is a slot that holds value i. (A
-// store from the one lane of each value, picked by comparing the lane with
-// five constants, compiled to a branch table: 600 cycles more.)
-__device__ __forceinline__ double warp_sum5(const double* v, int lane) {
-    const unsigned int full = 0xffffffffu;
-    const bool h16 = lane & 16, h8 = lane & 8, h4 = lane & 4;
-    double a = h16 ? v[3] : v[0], b = h16 ? v[4] : v[1], c = h16 ? 0.0 : v[2];
-    a += __shfl_xor_sync(full, h16 ? v[0] : v[3], 16);
-    b += __shfl_xor_sync(full, h16 ? v[1] : v[4], 16);
-    {
-        const double t = __shfl_xor_sync(full, h16 ? v[2] : 0.0, 16);
-        c += h16 ? 0.0 : t;
-    }
-    double d = h8 ? b : a;
-    d += __shfl_xor_sync(full, h8 ? a : b, 8);
-    c += __shfl_xor_sync(full, c, 8);
-    // lanes 0..7: d = v0 sums, c = v2 sums: one of them per half of the lanes
-    const bool two = lane < 8;
-    double e = (two && h4) ? c : d;
-    e += __shfl_xor_sync(full, (two && !h4) ? c : d, 4);
-    e += __shfl_xor_sync(full, e, 2);
-    e += __shfl_xor_sync(full, e, 1);
-    return e;
-}
-__device__ __forceinline__ constexpr int sum_slot(int i) { return i == 0 ? 0 : i == 1 ? 2 : i == 2 ? 1 : 2 * i - 2; }
-
-// What the exchange decides: the next step's scalars, go = 0 at the end.
-struct Step {
-    double alpha, beta;
-    int go;
-};
-
 // ---------------------------------------------------------------- kernel --
 
-template <typename T, bool GRID>
+// NPT nodes per thread; of the second one (double) the whole row lies in
+// shared memory.
+template <typename T, bool GRID, int NPT>
 __global__ void __launch_bounds__(kChipWarps * 32, 1) k_chip(ChipArgs<T> a) {
     using V2 = typename Vec2<T>::type;
     using V4 = typename Vec4<T>::type;
-    constexpr int W = kRegBlocks, NR = Record<T>::n;
+    constexpr int RN = sizeof(T) == 4 ? NPT : 1;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ double wsum[16][8];  // per warp: its sums (unused warps stay zero)
-    __shared__ double gsum[kMaxPolls][8];  // grid, the adding CTA: the same of the CTAs' sums
-    __shared__ __align__(16) double part[2][kMaxCluster][6];  // cluster: every CTA's sums (0, 2, 1, -, 3, 4), by parity
-    __shared__ __align__(8) unsigned long long bar[2];  // cluster: they have arrived
-    __shared__ Step step;
+    __shared__ CommShared cs;
     const ChipPlan& P = a.plan;
-    const int tid = threadIdx.x, nthr = blockDim.x, lane = tid & 31, w = tid >> 5;
-    const int rank = blockIdx.x, ctas = P.ctas, own = P.spc * 32;
-    const size_t slots = (size_t)ctas * own;
-    const int slot = rank * own + tid, n = GRID && rank == ctas ? -1 : P.order[slot];
-    const bool act = n >= 0;
+    const int tid = threadIdx.x, nthr = blockDim.x, w = tid >> 5;
+    const int rank = blockIdx.x, ctas = P.ctas, own = nthr * NPT;
+    const bool adder = GRID && rank == ctas;  // the CTA without nodes
+    Comm<T, GRID> comm{cs,        tid,       nthr,      tid & 31,          w,           rank,        ctas,
+                       own,       0u,        a.ll_rec,  a.ll_part,         a.ll_step,   (size_t)ctas * own,
+                       a.poll_limit, a.seq_skew};
     // shared memory: U [own + halo], then (cluster) records [2][3][own], then
-    // the blocks beyond W: values, local indexes
+    // the blocks that are not in registers
     V2* U = reinterpret_cast<V2*>(smem_raw);
     V2* rec = U + own + P.halo_cap;
-    const int extra = P.wmax > W ? P.wmax - W : 0;
-    V4* kval = reinterpret_cast<V4*>(rec + (GRID ? 0 : 6 * own));
-    unsigned short* kidx = reinterpret_cast<unsigned short*>(kval + (size_t)own * extra);
-    const unsigned int u_base = smem_addr(U);
+    comm.rec_base = smem_addr(rec);
+    ChipRows<T, NPT, RN> rows;
+    rows.tid = tid;
+    rows.nthr = nthr;
+    rows.init(rec + (GRID ? 0 : 6 * own), smem_addr(U), P.wmax);
 
-    for (int i = tid; i < 128; i += nthr) (&wsum[0][0])[i] = 0.0;
-    for (int i = tid; i < kMaxPolls * 8; i += nthr) (&gsum[0][0])[i] = 0.0;
-    for (int i = tid; i < 2 * kMaxCluster * 6; i += nthr) (&part[0][0][0])[i] = 0.0;
     // ---- rows, r = m.(b - K x), M
-    V4 kr[W];
-    unsigned int li[W];  // byte addresses in U
-#pragma unroll
-    for (int k = 0; k < W; ++k) {
-        kr[k].x = kr[k].y = kr[k].z = kr[k].w = (T)0;
-        li[k] = u_base + tid * (unsigned int)sizeof(V2);
-    }
-    int wd = 0;
-    double2 x = make_double2(0.0, 0.0);
-    uchar2 m = make_uchar2(0, 0);
-    V2 r = make2<V2>(0, 0), p = r, kp = r, wv = r, u = r;
-    T mi0 = (T)0, mi1 = (T)0, mi2 = (T)0;  // M, symmetric as K is: m00, m01 = m10, m11
-    bool publish = false;
+    int n[NPT];
+    double2 x[NPT];
+    uchar2 m[NPT];
+    V2 r[NPT], p[NPT], kp[NPT], wv[NPT], u[NPT];
+    T mi0[NPT], mi1[NPT], mi2[NPT];  // M, symmetric as K is: m00, m01 = m10, m11
+    bool publish[NPT];
     double v[kSums] = {0.0, 0.0, 0.0, 0.0, 0.0};
-    if (act) {
-        const int base = a.slice_ptr[n >> 5] + (n & 31);
-        wd = (a.slice_ptr[(n >> 5) + 1] - base + 31) >> 5;
-        m = a.mask[n];
-        x = a.x[n];
-        publish = P.pub[slot] != 0;
-        const unsigned short* lx = P.lidx + (size_t)(slot >> 5) * P.wmax * 32 + lane;
+#pragma unroll
+    for (int j = 0; j < NPT; ++j) {
+        const int slot = rank * own + j * nthr + tid;
+        n[j] = adder ? -1 : P.order[slot];
+        x[j] = make_double2(0.0, 0.0);
+        m[j] = make_uchar2(0, 0);
+        r[j] = p[j] = kp[j] = wv[j] = u[j] = make2<V2>(0, 0);
+        mi0[j] = mi1[j] = mi2[j] = (T)0;
+        publish[j] = false;
+        if (n[j] < 0) continue;
+        const int nd = n[j], base = a.slice_ptr[nd >> 5] + (nd & 31);
+        m[j] = a.mask[nd];
+        x[j] = a.x[nd];
+        publish[j] = P.pub[slot] != 0;
         double k0 = 0.0, k1 = 0.0;
         double4 diag = make_double4(0.0, 0.0, 0.0, 0.0);
-        auto residual = [&](int k) {  // FP64, also in the mixed mode
-            const long long bi = base + 32LL * k;
-            const double2* vp = reinterpret_cast<const double2*>(a.val64 + 4 * bi);
-            const double2 lo = __ldg(vp), hi = __ldg(vp + 1);
-            const double2 xc = a.x[__ldg(a.scol + bi)];
-            k0 += lo.x * xc.x + lo.y * xc.y;
-            k1 += hi.x * xc.x + hi.y * xc.y;
-            if (k == 0) diag = make_double4(lo.x, lo.y, hi.x, hi.y);
-            V4 q;
-            q.x = (T)lo.x; q.y = (T)lo.y; q.z = (T)hi.x; q.w = (T)hi.y;
-            return q;
-        };
-#pragma unroll
-        for (int k = 0; k < W; ++k)
-            if (k < wd) {
-                kr[k] = residual(k);
-                li[k] = u_base + lx[32 * k] * (unsigned int)sizeof(V2);
-            }
-        for (int k = W; k < wd; ++k) {
-            const size_t q = (size_t)(k - W) * own + tid;
-            kval[q] = residual(k);
-            kidx[q] = lx[32 * k];
-        }
-        const double2 bb = a.b[n];
-        const double r0 = m.x ? bb.x - k0 : 0.0, r1 = m.y ? bb.y - k1 : 0.0;
-        r = make2<V2>((T)r0, (T)r1);
+        rows.load(j, (a.slice_ptr[(nd >> 5) + 1] - base + 31) >> 5,
+                  P.lidx + (size_t)(slot >> 5) * P.wmax * 32 + (tid & 31), [&](int k) {  // r in FP64, also for float
+                      const long long bi = base + 32LL * k;
+                      const double2* vp = reinterpret_cast<const double2*>(a.val64 + 4 * bi);
+                      const double2 lo = __ldg(vp), hi = __ldg(vp + 1);
+                      const double2 xc = a.x[__ldg(a.scol + bi)];
+                      k0 += lo.x * xc.x + lo.y * xc.y;
+                      k1 += hi.x * xc.x + hi.y * xc.y;
+                      if (k == 0) diag = make_double4(lo.x, lo.y, hi.x, hi.y);
+                      V4 q;
+                      q.x = (T)lo.x; q.y = (T)lo.y; q.z = (T)hi.x; q.w = (T)hi.y;
+                      return q;
+                  });
+        const double2 bb = a.b[nd];
+        const double r0 = m[j].x ? bb.x - k0 : 0.0, r1 = m[j].y ? bb.y - k1 : 0.0;
+        r[j] = make2<V2>((T)r0, (T)r1);
         if (a.precond) {  // inverse of the diagonal block on the free DOFs
-            if (m.x && m.y) {
+            if (m[j].x && m[j].y) {
                 const double det = diag.x * diag.w - diag.y * diag.z;
-                mi0 = (T)(diag.w / det);
-                mi1 = (T)(-diag.y / det);
-                mi2 = (T)(diag.x / det);
-            } else if (m.x) {
-                mi0 = (T)(1.0 / diag.x);
-            } else if (m.y) {
-                mi2 = (T)(1.0 / diag.w);
+                mi0[j] = (T)(diag.w / det);
+                mi1[j] = (T)(-diag.y / det);
+                mi2[j] = (T)(diag.x / det);
+            } else if (m[j].x) {
+                mi0[j] = (T)(1.0 / diag.x);
+            } else if (m[j].y) {
+                mi2[j] = (T)(1.0 / diag.w);
             }
         } else {
-            mi0 = (T)(m.x ? 1 : 0);
-            mi2 = (T)(m.y ? 1 : 0);
+            mi0[j] = (T)(m[j].x ? 1 : 0);
+            mi2[j] = (T)(m[j].y ? 1 : 0);
         }
-        u = make2<V2>(mi0 * r.x + mi1 * r.y, mi1 * r.x + mi2 * r.y);
-        v[0] = (double)r.x * (double)r.x + (double)r.y * (double)r.y;
-        v[1] = bb.x * bb.x + bb.y * bb.y;
-        v[2] = r0 * r0 + r1 * r1;
+        u[j] = make2<V2>(mi0[j] * r[j].x + mi1[j] * r[j].y, mi1[j] * r[j].x + mi2[j] * r[j].y);
+        v[0] += (double)r[j].x * (double)r[j].x + (double)r[j].y * (double)r[j].y;
+        v[1] += bb.x * bb.x + bb.y * bb.y;
+        v[2] += r0 * r0 + r1 * r1;
     }
-    wd -= W;  // blocks beyond the registers
     // ---- halo: thread nthr - 1 - tid takes the first halo nodes, so that the
-    // warps that wait for the sums have few of them
-    const int hc = GRID && rank == ctas ? 0 : P.halo_cnt[rank], h0 = nthr - 1 - tid;
+    // warps that wait for the sums have few of them; past the last halo node a
+    // thread reads the last one again, so that whole warps read
+    const int hc = adder ? 0 : P.halo_cnt[rank], h0 = nthr - 1 - tid, h_min = nthr - 32 * (w + 1);
     const int* hl = P.halo + (size_t)rank * kHaloMax;
-    const unsigned int rec_base = smem_addr(rec);
-    // where the record of halo slot s is read: cluster address, or the slot (grid)
-    auto halo_at = [&](int s) -> unsigned int {
-        if (GRID) return (unsigned int)s;
-        const int cr = s / own;
-        return mapa(rec_base + (unsigned int)((s - cr * own) * sizeof(V2)), cr);
-    };
-    // the first halo record of this thread (past the last one: the last one,
-    // so that whole warps read), and the smallest h0 of the warp
-    const unsigned int ha = hc > 0 ? halo_at(hl[min(h0, hc - 1)]) : 0u;
-    const int h_min = nthr - 32 * (w + 1);
-    unsigned int seq = GRID ? *a.seq : 0u;
-    const int np = (ctas + 31) >> 5;  // grid: warps of CTA 0 that poll the CTAs' sums
-    int par = 1;                      // parity of the last exchange
-    bool failed = false;
+    const unsigned int ha = hc > 0 ? comm.halo_at(hl[min(h0, hc - 1)]) : 0u;
     V2 hr[3];
-    // ---- the scalars of the solve: warp 0 (grid: of CTA 0)
+    comm.seq = GRID ? *a.seq : 0u;
+    // ---- the scalars of the solve: warp 0 (grid: of the adding CTA)
     double rr = 0.0, rho = 0.0, rho_inv = 0.0, bnorm2 = 0.0, res64 = 0.0, normB_inv = 0.0;
     int status = 0, converged = 0, lin_done = 0;
     int iter = 0;
     const int max_iter = (int)(a.max_iter < 0x7fffffffLL ? a.max_iter : 0x7fffffffLL);
-    unsigned int phase = 0;  // of the mbarriers' next wait
-    if (!GRID && tid == 0) {
-        bar_init(smem_addr(&bar[0]));
-        bar_init(smem_addr(&bar[1]));
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        bar_expect(smem_addr(&bar[0]), 48u * ctas);
-        bar_expect(smem_addr(&bar[1]), 48u * ctas);
-    }
-    if constexpr (!GRID) {
-        cluster_arrive_release();
-        cluster_wait();
-    } else {
-        __syncthreads();
-    }
+    comm.init();
 
-    auto apply_m = [&](V2 q) { return make2<V2>(mi0 * q.x + mi1 * q.y, mi1 * q.x + mi2 * q.y); };
-    auto read_halo = [&](unsigned int at, V2* q) {
-        if constexpr (GRID) {
-            uint4 c[NR];
-            if (!poll<NR>(a.ll_rec + (size_t)par * NR * slots + at, slots, seq, a.poll_limit, c)) failed = true;
-            Record<T>::get(c, q);
-        } else {
-            const unsigned int s = at + (unsigned int)(par * 3 * own * sizeof(V2));
-#pragma unroll
-            for (int i = 0; i < 3; ++i) ld_cluster(s + (unsigned int)(i * own * sizeof(V2)), q[i]);
-        }
-    };
+    auto apply_m = [&](int j, V2 q) { return make2<V2>(mi0[j] * q.x + mi1[j] * q.y, mi1[j] * q.x + mi2[j] * q.y); };
     // The next step from the sums of an iteration (see cg_fused.cu for the
     // recurrences). Straight-line: one warp runs it while all others wait, and
     // its branches cost more than its arithmetic; why the solve ended is
@@ -580,7 +357,7 @@ __global__ void __launch_bounds__(kChipWarps * 32, 1) k_chip(ChipArgs<T> a) {
     auto finish = [&]() {
         if (tid != 0) return;
         CgScalars* sc = a.sc;
-        if (failed) {
+        if (comm.failed) {
             atomicExch(&sc->chip_err, 1);
             return;
         }
@@ -604,168 +381,43 @@ __global__ void __launch_bounds__(kChipWarps * 32, 1) k_chip(ChipArgs<T> a) {
         sc->converged = converged;
         sc->status = status;
         sc->lin_done = lin_done;
-        sc->alpha = step.alpha;
-        sc->beta = step.beta;
+        sc->alpha = cs.step.alpha;
+        sc->beta = cs.step.beta;
         sc->rho = rho;
         sc->ticket = 0;
-        if (GRID) *a.seq = seq;  // every CTA has read the old value: all have taken part in an exchange
+        if (GRID) *a.seq = comm.seq;  // every CTA has read the old value: all have taken part in an exchange
     };
-    // Posts the own record and the sums v; receives the first halo record (hr)
-    // and the next step. Every thread returns with `step` readable.
     auto exchange = [&](auto decide_now) {
-        par ^= 1;
-        if constexpr (GRID) {
-            seq += 1;
-            if (publish)
-                Record<T>::put(a.ll_rec + (size_t)par * NR * slots + slot, slots, u, apply_m(wv), apply_m(kp),
-                               seq + a.seq_skew);
-        } else {
-            if (publish) {
-                V2* own_rec = rec + (size_t)par * 3 * own + tid;
-                own_rec[0] = u;
-                own_rec[own] = apply_m(wv);
-                own_rec[2 * own] = apply_m(kp);
-            }
-        }
-        {
-            const double s = warp_sum5(v, lane);
-            if ((lane & 3) == 0) wsum[w][lane >> 2] = s;
-        }
-        __syncthreads();
-        // lane (g, j): slot j of the warps g, g + 4, ..; then over g
-        const int j = lane & 7, g = lane >> 3;
-        double s = 0.0;
-        if (w == 0) {
-            s = (wsum[g][j] + wsum[g + 4][j]) + wsum[g + 8][j];
-            s += __shfl_xor_sync(0xffffffffu, s, 8);
-            s += __shfl_xor_sync(0xffffffffu, s, 16);
-        }
-        if constexpr (GRID) {
-            uint4* pp = a.ll_part + (size_t)par * 8 * ctas;
-            uint4* rp = a.ll_step + par * 4;
-            // slots 0, 1, 2, 4, 6 hold the values 0, 2, 1, 3, 4
-            const int val = lane == 1 ? 2 : lane == 2 ? 1 : lane > 2 ? lane / 2 + 1 : 0;
-            if (w == 0 && (lane < 3 || lane == 4 || lane == 6))
-                post(pp + (size_t)val * ctas + rank, s, seq + a.seq_skew);
-            if (w == 0) {
-                uint4 c[1];
-                if (!poll<1>(rp + min(lane, kStepWords - 1), 1, seq, a.poll_limit, c)) failed = true;
-                const double q = word_value(c[0]);
-                if (lane == 0) step.alpha = q;
-                if (lane == 1) step.beta = q;
-                if (lane == 2) step.go = q != 0.0;
-            }
-            if (h_min < hc) read_halo(ha, hr);
-            failed = __syncthreads_or(failed ? 1 : 0) != 0;
-        } else {
-            if (w == 0) {
-                // sums (0, 2), (1, 1), (3, 4) to every CTA, with the records of
-                // all warps written before the block barrier above
-                const double s2 = __shfl_sync(0xffffffffu, s, j == 4 ? 6 : j + 1);
-                if (!(j & 1) && j < 6) {
+        comm.begin();
 #pragma unroll
-                    for (int i = 0; i < 4; ++i)
-                        if (g + 4 * i < ctas)
-                            st_async(mapa(smem_addr(&part[par][rank][j]), g + 4 * i),
-                                     mapa(smem_addr(&bar[par]), g + 4 * i), s, s2);
-                }
-            }
-            {
-                const unsigned int ba = smem_addr(&bar[par]);
-                unsigned int round = 0;
-                while (!bar_try(ba, phase)) {
-                    if (++round > a.poll_limit) {
-                        failed = true;
-                        break;
-                    }
-                }
-            }
-            if (par) phase ^= 1u;
-            if (h_min < hc) read_halo(ha, hr);
-            if (w == 0) {
-                if (lane == 0) bar_expect(smem_addr(&bar[par]), 48u * ctas);  // its next use
-                // lane (g, j): value j of the CTAs g, g + 4, ..; then over g
-                const int e = j < 6 ? j : 0;
-                s = (part[par][g][e] + part[par][g + 4][e]) + (part[par][g + 8][e] + part[par][g + 12][e]);
-                s += __shfl_xor_sync(0xffffffffu, s, 8);
-                s += __shfl_xor_sync(0xffffffffu, s, 16);
-                double tot[kSums];
-#pragma unroll
-                for (int i = 0; i < kSums; ++i)
-                    tot[i] = __shfl_sync(0xffffffffu, s, i == 0 ? 0 : i == 1 ? 2 : i == 2 ? 1 : i + 1);
-                const Step st = decide_now(tot);
-                if (lane == 0) step = st;
-            }
-            failed = __syncthreads_or(failed ? 1 : 0) != 0;
-        }
+        for (int j = 0; j < NPT; ++j)
+            if (publish[j]) comm.put_record(rec, j * nthr + tid, u[j], apply_m(j, wv[j]), apply_m(j, kp[j]));
+        comm.finish(
+            v, [&] { if (h_min < hc) comm.read_halo(ha, hr); }, decide_now);
     };
-    // U of the own node and of the halo at step (al, bt).
+    // U of the own nodes and of the halo at step (al, bt).
     auto fill_u = [&](T al, T bt) {
-        U[tid] = u;
+#pragma unroll
+        for (int j = 0; j < NPT; ++j) U[j * nthr + tid] = u[j];
         if (h0 < hc)
             U[own + h0] = make2<V2>(hr[0].x - al * (hr[1].x + bt * hr[2].x), hr[0].y - al * (hr[1].y + bt * hr[2].y));
         if (hc > nthr) {
             for (int b = nthr; h_min + b < hc; b += nthr) {
                 const int h = h0 + b;
-                read_halo(halo_at(hl[min(h, hc - 1)]), hr);
+                comm.read_halo(comm.halo_at(hl[min(h, hc - 1)]), hr);
                 if (h < hc)
                     U[own + h] = make2<V2>(hr[0].x - al * (hr[1].x + bt * hr[2].x),
                                            hr[0].y - al * (hr[1].y + bt * hr[2].y));
             }
-            if (GRID) failed = __syncthreads_or(failed ? 1 : 0) != 0;
+            if (GRID) comm.failed = __syncthreads_or(comm.failed ? 1 : 0) != 0;
         }
         __syncthreads();
     };
-    auto gather = [&]() {
-        T k0 = (T)0, k1 = (T)0;
-#pragma unroll
-        for (int k = 0; k < W; ++k) {
-            V2 c;
-            ld_u(li[k], c);
-            k0 += kr[k].x * c.x + kr[k].y * c.y;
-            k1 += kr[k].z * c.x + kr[k].w * c.y;
-        }
-        for (int k = 0; k < wd; ++k) {
-            const size_t q = (size_t)k * own + tid;
-            const V4 kv = kval[q];
-            const V2 c = U[kidx[q]];
-            k0 += kv.x * c.x + kv.y * c.y;
-            k1 += kv.z * c.x + kv.w * c.y;
-        }
-        return make2<V2>(k0, k1);
-    };
-    if (GRID && rank == ctas) {
-        // the CTA without nodes: adds up all CTAs' sums and posts the steps
+
+    if (adder) {
         auto lead = [&](auto decide_now) {
-            par ^= 1;
-            seq += 1;
-            const uint4* pp = a.ll_part + (size_t)par * 8 * ctas;
-            for (int q = w; q < np; q += nthr >> 5) {
-                double t[kSums];
-                uint4 ch[kSums];
-                const int c = 32 * q + lane;
-                if (!poll<kSums>(pp + min(c, ctas - 1), ctas, seq, a.poll_limit, ch)) failed = true;
-#pragma unroll
-                for (int i = 0; i < kSums; ++i) t[i] = c < ctas ? word_value(ch[i]) : 0.0;
-                const double r5 = warp_sum5(t, lane);
-                if ((lane & 3) == 0) gsum[q][lane >> 2] = r5;
-            }
-            failed = __syncthreads_or(failed ? 1 : 0) != 0;
-            if (w == 0) {
-                double t = 0.0;
-#pragma unroll
-                for (int q = 0; q < kMaxPolls; ++q) t += gsum[q][lane & 7];
-                double tot[kSums];
-#pragma unroll
-                for (int i = 0; i < kSums; ++i) tot[i] = __shfl_sync(0xffffffffu, t, sum_slot(i));
-                const Step st = decide_now(tot);
-                if (lane < kStepWords)
-                    post(a.ll_step + par * 4 + lane, lane == 0 ? st.alpha : lane == 1 ? st.beta : (double)st.go,
-                         seq + a.seq_skew);
-                if (lane == 0) step = st;
-            }
-            __syncthreads();
-            return step.go != 0 && !failed;
+            comm.lead(decide_now);
+            return cs.step.go != 0 && !comm.failed;
         };
         if (lead(decide_init) && lead(decide_first)) {
             do {
@@ -778,59 +430,76 @@ __global__ void __launch_bounds__(kChipWarps * 32, 1) k_chip(ChipArgs<T> a) {
     // ---- (r, r), (b, b), and u to the neighbours
     exchange(decide_init);
     fill_u((T)0, (T)0);
-    bool go = step.go != 0 && !failed;
+    bool go = cs.step.go != 0 && !comm.failed;
     if (go) {
         // ---- first step: w = K u; gamma = (r, u), delta = (w, u)
-        wv = gather();
-        v[0] = (double)r.x * (double)u.x + (double)r.y * (double)u.y;
-        v[1] = (double)wv.x * (double)u.x + (double)wv.y * (double)u.y;
-        v[2] = 0.0;
+        v[0] = v[1] = v[2] = 0.0;
+#pragma unroll
+        for (int j = 0; j < NPT; ++j) {
+            wv[j] = rows.gather(j);
+            v[0] += (double)r[j].x * (double)u[j].x + (double)r[j].y * (double)u[j].y;
+            v[1] += (double)wv[j].x * (double)u[j].x + (double)wv[j].y * (double)u[j].y;
+        }
         exchange(decide_first);
-        go = step.go != 0 && !failed;
+        go = cs.step.go != 0 && !comm.failed;
     }
     // ---- iterations
     while (go) {
-        const double alpha = step.alpha;
+        const double alpha = cs.step.alpha;
         if (!GRID) rho_inv = __drcp_rn(rho);  // for the next decision, off its path
-        const T al = (T)alpha, bt = (T)step.beta;
-        const V2 u0 = u;
-        const V2 mw = apply_m(wv), mk = apply_m(kp);
-        u = make2<V2>(u0.x - al * (mw.x + bt * mk.x), u0.y - al * (mw.y + bt * mk.y));
+        const T al = (T)alpha, bt = (T)cs.step.beta;
+        V2 u0[NPT];
+#pragma unroll
+        for (int j = 0; j < NPT; ++j) {
+            u0[j] = u[j];
+            const V2 mw = apply_m(j, wv[j]), mk = apply_m(j, kp[j]);
+            u[j] = make2<V2>(u0[j].x - al * (mw.x + bt * mk.x), u0[j].y - al * (mw.y + bt * mk.y));
+        }
         fill_u(al, bt);
-        p = make2<V2>(u0.x + bt * p.x, u0.y + bt * p.y);
-        kp = make2<V2>(wv.x + bt * kp.x, wv.y + bt * kp.y);
-        x.x += alpha * (double)p.x;
-        x.y += alpha * (double)p.y;
-        if (m.x) r.x -= al * kp.x;
-        if (m.y) r.y -= al * kp.y;
-        wv = gather();
-        v[0] = (double)r.x * (double)u.x + (double)r.y * (double)u.y;
-        v[1] = (double)wv.x * (double)u.x + (double)wv.y * (double)u.y;
-        v[2] = (double)r.x * (double)r.x + (double)r.y * (double)r.y;
-        v[3] = ((double)wv.x * (double)p.x + (double)wv.y * (double)p.y) +
-               ((double)kp.x * (double)u.x + (double)kp.y * (double)u.y);
-        v[4] = (double)kp.x * (double)p.x + (double)kp.y * (double)p.y;
+#pragma unroll
+        for (int i = 0; i < kSums; ++i) v[i] = 0.0;
+#pragma unroll
+        for (int j = 0; j < NPT; ++j) {
+            p[j] = make2<V2>(u0[j].x + bt * p[j].x, u0[j].y + bt * p[j].y);
+            kp[j] = make2<V2>(wv[j].x + bt * kp[j].x, wv[j].y + bt * kp[j].y);
+            x[j].x += alpha * (double)p[j].x;
+            x[j].y += alpha * (double)p[j].y;
+            if (m[j].x) r[j].x -= al * kp[j].x;
+            if (m[j].y) r[j].y -= al * kp[j].y;
+            wv[j] = rows.gather(j);
+            const V2 wj = wv[j], uj = u[j], rj = r[j], pj = p[j], kj = kp[j];
+            v[0] += (double)rj.x * (double)uj.x + (double)rj.y * (double)uj.y;
+            v[1] += (double)wj.x * (double)uj.x + (double)wj.y * (double)uj.y;
+            v[2] += (double)rj.x * (double)rj.x + (double)rj.y * (double)rj.y;
+            v[3] += ((double)wj.x * (double)pj.x + (double)wj.y * (double)pj.y) +
+                    ((double)kj.x * (double)uj.x + (double)kj.y * (double)uj.y);
+            v[4] += (double)kj.x * (double)pj.x + (double)kj.y * (double)pj.y;
+        }
         exchange(decide);
-        go = step.go != 0 && !failed;
+        go = cs.step.go != 0 && !comm.failed;
     }
     if constexpr (!GRID) {  // the others have read this CTA's memory for the last time
         cluster_arrive_release();
         cluster_wait();
     }
-    if (failed) {
+    if (comm.failed) {
         if (tid == 0) atomicExch(&a.sc->chip_err, 1);
         return;
     }
-    if (act) a.x[n] = x;
+#pragma unroll
+    for (int j = 0; j < NPT; ++j)
+        if (n[j] >= 0) a.x[n[j]] = x[j];
     if (!GRID && rank == 0) finish();
 }
 
 // Dynamic shared memory per CTA.
-size_t chip_smem(bool grid, int spc, int wmax, int halo, size_t st) {
-    const size_t own = (size_t)spc * 32, extra = wmax > kRegBlocks ? wmax - kRegBlocks : 0;
-    size_t b = (own + halo) * 2 * st;
-    if (!grid) b += 6 * own * 2 * st;
-    b += own * extra * (4 * st + 2);
+template <typename T, bool GRID, int NPT>
+size_t chip_smem(const ChipPlan& p) {
+    const int nthr = 32 * p.spc / NPT;
+    const size_t own = (size_t)nthr * NPT;
+    size_t b = (own + p.halo_cap) * 2 * sizeof(T);
+    if (!GRID) b += 6 * own * 2 * sizeof(T);
+    b += ChipRows<T, NPT, sizeof(T) == 4 ? NPT : 1>::smem_blocks(nthr, p.wmax) * (4 * sizeof(T) + 2);
     return (b + 15) / 16 * 16;
 }
 
@@ -838,7 +507,7 @@ template <typename K>
 cudaLaunchConfig_t chip_config(K, const ChipPlan& p, size_t smem, cudaLaunchAttribute* attr, cudaStream_t s) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(p.ctas + (p.grid ? 1 : 0));  // the grid form's last CTA adds up the sums
-    cfg.blockDim = dim3(32 * p.spc);
+    cfg.blockDim = dim3(32 * p.spc / p.npt);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
     if (p.grid) {
@@ -864,28 +533,32 @@ bool chip_attributes(K k, bool grid) {
     return ok;
 }
 
-template <typename T>
-bool chip_schedulable(const ChipPlan& p, int sm_count) {
-    const size_t smem = chip_smem(p.grid, p.spc, p.wmax, p.halo_cap, sizeof(T));
-    if (smem > kSmemCap) return false;
-    if (p.grid) {
+template <typename T, bool GRID, int NPT>
+bool schedulable(const ChipPlan& p, int sm_count) {
+    const auto k = k_chip<T, GRID, NPT>;
+    const size_t smem = chip_smem<T, GRID, NPT>(p);
+    if (smem > kSmemCap || !chip_attributes(k, GRID)) return false;
+    if (GRID) {
         int per_sm = 0;
-        if (!chip_attributes(k_chip<T, true>, true) ||
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_chip<T, true>, 32 * p.spc, smem) != cudaSuccess) {
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, 32 * p.spc / NPT, smem) != cudaSuccess) {
             cudaGetLastError();
             return false;
         }
         return (long long)per_sm * sm_count >= p.ctas + 1;
     }
-    if (!chip_attributes(k_chip<T, false>, false)) return false;
     cudaLaunchAttribute attr[1];
-    cudaLaunchConfig_t cfg = chip_config(k_chip<T, false>, p, smem, attr, nullptr);
+    cudaLaunchConfig_t cfg = chip_config(k, p, smem, attr, nullptr);
     int clusters = 0;
-    if (cudaOccupancyMaxActiveClusters(&clusters, k_chip<T, false>, &cfg) != cudaSuccess || clusters < 1) {
+    if (cudaOccupancyMaxActiveClusters(&clusters, k, &cfg) != cudaSuccess || clusters < 1) {
         cudaGetLastError();
         return false;
     }
     return true;
+}
+template <typename T>
+bool chip_schedulable(const ChipPlan& p, int sm_count) {
+    if (!p.grid) return schedulable<T, false, 1>(p, sm_count);
+    return p.npt == 2 ? schedulable<T, true, 2>(p, sm_count) : schedulable<T, true, 1>(p, sm_count);
 }
 
 }  // namespace
@@ -893,13 +566,15 @@ bool chip_schedulable(const ChipPlan& p, int sm_count) {
 // The shape of the cluster (grid = false) or grid form for n nodes; ctas = 0
 // when it does not hold them.
 //   cluster: about 13 CTAs, of at least 4 slices. 1024 nodes: 8 CTAs of 4
-//     slices 1.70 us per iteration, 16 of 2 2.10, 3 of 12 1.92; 4160 nodes: 13
-//     of 10 1.93, 11 of 12 1.93 (the whole solve in one cluster with every
+//     slices 1.70 us per iteration, 16 of 2 2.10, 3 of 12 2.02; 4160 nodes: 13
+//     of 10 1.98, 11 of 12 2.10 (the whole solve in one cluster with every
 //     record read through distributed shared memory: 4.9 and 5.7).
 //   grid: about 128 CTAs, of at least 8 slices. 16104 nodes: 63 CTAs of 8
-//     slices 3.40 us, 126 of 4 3.82, 42 of 12 3.54 (one launch per iteration,
-//     cg_fused.cu: 10.2); 40200 nodes: 126 of 10 3.67, 105 of 12 3.83 (11.3).
-//     At sizes that both hold the cluster is the faster one (4160 nodes: 3.13
+//     slices 3.40 us, 126 of 4 3.80, 42 of 12 3.62 (one launch per iteration,
+//     cg_fused.cu: 10.2); 40200 nodes: 126 of 10 3.67, 105 of 12 3.98 (11.3).
+//     Above 147 CTAs of 12, two nodes per thread: 65536 nodes 86 CTAs of 24
+//     6.26 us, 128 of 16 6.70 (12.0); 99856 nodes 131 of 24 6.33 (16.3).
+//     At sizes that both hold the cluster is the faster one (4160 nodes: 3.16
 //     as a grid).
 ChipShape chip_shape(int n, int wmax, int sm_count, bool grid) {
     const int n_slices = (n + 31) / 32;
@@ -909,14 +584,20 @@ ChipShape chip_shape(int n, int wmax, int sm_count, bool grid) {
     s.spc = grid ? std::max((n_slices + 127) / 128, 8) : std::max((n_slices + 12) / 13, 4);
     if (const char* e = std::getenv("CUPLAST_CHIP_FORM")) {  // c<slices per CTA> or g<slices per CTA> (measurements)
         const int v = std::atoi(e + 1);
-        if ((e[0] == 'c' || e[0] == 'g') && v >= 1 && v <= kChipWarps) {
+        if ((e[0] == 'c' || e[0] == 'g') && v >= 1 && v <= (e[0] == 'g' ? 2 : 1) * kChipWarps) {
             if (grid != (e[0] == 'g')) return s;
             s.spc = v;
         }
     }
-    s.spc = std::min(s.spc, kChipWarps);
+    const int most = grid ? std::min(sm_count - 1, 32 * kMaxPolls) : kMaxCluster;
+    if (s.spc <= kChipWarps || !grid || (long long)most * kChipWarps >= n_slices) {
+        s.spc = std::min(s.spc, kChipWarps);
+    } else {  // two nodes per thread
+        s.npt = 2;
+        s.spc = 2 * kChipWarps;
+    }
     s.ctas = (n_slices + s.spc - 1) / s.spc;
-    if (s.ctas > (grid ? std::min(sm_count - 1, 32 * kMaxPolls) : kMaxCluster)) s.ctas = 0;
+    if (s.ctas > most) s.ctas = 0;
     return s;
 }
 
@@ -945,6 +626,7 @@ void chip_build_plan(ChipPlan& p, const ChipShape& s, void* mem, int n, const do
     const size_t slots = chip_slots(s);
     p.grid = s.grid;
     p.spc = s.spc;
+    p.npt = s.npt;
     p.wmax = s.wmax;
     p.ctas = 0;
     int* ints = static_cast<int*>(mem);
@@ -975,19 +657,23 @@ void chip_build_plan(ChipPlan& p, const ChipShape& s, void* mem, int n, const do
     if (!chip_schedulable<double>(p, sm_count) || !chip_schedulable<float>(p, sm_count)) p.ctas = 0;
 }
 
+namespace {
+template <typename T, bool GRID, int NPT>
+void launch_as(const ChipArgs<T>& a, cudaStream_t s) {
+    const auto k = k_chip<T, GRID, NPT>;
+    cudaLaunchAttribute attr[1];
+    cudaLaunchConfig_t cfg = chip_config(k, a.plan, chip_smem<T, GRID, NPT>(a.plan), attr, s);
+    CP_CUDA(cudaLaunchKernelEx(&cfg, k, a));
+}
+}  // namespace
+
 template <typename T>
 void chip_launch(const ChipArgs<T>& a, cudaStream_t s) {
     const ChipPlan& p = a.plan;
     CP_CHECK(p.ctas > 0, CP_ERR_INVALID, "on-chip CG: the instance does not fit");
-    const size_t smem = chip_smem(p.grid, p.spc, p.wmax, p.halo_cap, sizeof(T));
-    cudaLaunchAttribute attr[1];
-    if (p.grid) {
-        cudaLaunchConfig_t cfg = chip_config(k_chip<T, true>, p, smem, attr, s);
-        CP_CUDA(cudaLaunchKernelEx(&cfg, k_chip<T, true>, a));
-    } else {
-        cudaLaunchConfig_t cfg = chip_config(k_chip<T, false>, p, smem, attr, s);
-        CP_CUDA(cudaLaunchKernelEx(&cfg, k_chip<T, false>, a));
-    }
+    if (!p.grid) launch_as<T, false, 1>(a, s);
+    else if (p.npt == 2) launch_as<T, true, 2>(a, s);
+    else launch_as<T, true, 1>(a, s);
 }
 
 template void chip_launch<double>(const ChipArgs<double>&, cudaStream_t);

@@ -74,9 +74,11 @@ def check(problem, u, rep, csr, eps, unit=EPS64):
 
 
 # nodes: 4, 32 and around (a slice), 127..129 x 2 (a CTA), 1664, 1665 (13 CTAs of 4), 6144, 6145 (16 CTAs of 12: the cluster's
-# largest, then the grid), 32768, 32769 (128 CTAs of 8, then 9)
+# largest, then the grid), 32768, 32769 (128 CTAs of 8, then 9), 56448, 56560 (147 CTAs of 12, then two nodes per
+# thread), 112896, 113008 (the largest, then the graph loop)
 @pytest.mark.parametrize("nx, ny", [(2, 2), (31, 2), (16, 2), (11, 3), (127, 2), (43, 3), (64, 26),
-                                    (555, 3), (96, 64), (2048, 3), (5, 1229), (256, 128), (331, 99)])
+                                    (555, 3), (96, 64), (2048, 3), (1229, 5), (256, 128), (331, 99), (504, 112), (505, 112),
+                                    (1008, 112), (1009, 112)])
 def test_sizes(nx, ny, ctx):
     p = strip(nx, ny)
     for precond in (0, 1):
@@ -104,7 +106,7 @@ def test_wide_rows(n_c, n_r, form, ctx, monkeypatch):
     check(p, *solve(ctx, p), 1e-11)
 
 
-@pytest.mark.parametrize("nx, ny", [(2, 2), (16, 2), (127, 2), (64, 26), (96, 64), (1229, 5), (331, 99)])
+@pytest.mark.parametrize("nx, ny", [(2, 2), (16, 2), (127, 2), (64, 26), (96, 64), (1229, 5), (331, 99), (505, 112)])
 def test_mixed_precision(nx, ny, ctx):
     """FP32 recurrences inside FP64 defect correction: the solve ends on the FP64 residual itself."""
     p = strip(nx, ny)

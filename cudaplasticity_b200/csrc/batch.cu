@@ -23,6 +23,8 @@
 // every (instance, tile) pair. Three persistent kernels walk that list, each
 // acting only on the tiles whose instance is in one of its phases:
 //   k_batch_cg    RES (FP64 residual), W (w = K u), ITER (one CG iteration)
+//   k_batch_chip  the three together, as phase CHIP, for instances of up to
+//                 12,288 nodes: one cluster each (not by tiles)
 //   k_batch_asm   ASM (FP64 + FP32 values of K, node gather, no atomics)
 //   k_batch_elem  LEVEL, UPD (strain / stress / secant / exit norm),
 //                 RELAX (Aitken), PLASTIC
@@ -33,7 +35,7 @@
 // tiling, on the grid, or on the other instances in the batch.
 //
 // One CUDA graph drives a run: a WHILE node whose body is
-//   elem x E, asm, cg x C, condition
+//   elem x E, asm, cg x C beside chip x 3 (cluster sizes), condition
 // and every launch advances every instance in a matching phase by one step.
 #include <cuda_runtime.h>
 
@@ -44,6 +46,7 @@
 #include <new>
 #include <vector>
 
+#include "chip.cuh"
 #include "common.cuh"
 #include "elements.cuh"
 #include "instance.h"
@@ -55,6 +58,7 @@ namespace {
 constexpr int kThreads = 128;  // 4 warps; every kernel of the batch
 constexpr int kWarps = kThreads / 32;
 constexpr int kBuckets = 24;
+constexpr int kBChipClasses = 3;  // cluster sizes 4, 8, 16 of the on-chip linear solve
 
 enum : int {
     PH_FREE = 0,
@@ -67,6 +71,7 @@ enum : int {
     PH_RELAX,
     PH_PLASTIC,
     PH_DONE,
+    PH_CHIP,  // a linear solve on chip (k_batch_chip), in place of RES, W and ITER
     PH_COUNT
 };
 
@@ -100,6 +105,7 @@ struct BDesc {
     int predict;        // level predictor (cp_solve_opts.predict)
     double2* pred_u;    // the last level's u and psi (predict only)
     double* pred_psi;
+    ChipPlan chip;      // chip.ctas > 0: linear solves on chip
 };
 
 // Mutable state of one instance.
@@ -112,6 +118,7 @@ struct BState {
     double rr, gamma, alpha, beta, rr_ref, eps2_inner, bb, res64, res_last;
     double eps, rel_err, w_prev, omega, cg_rel_res;
     unsigned long long t_first, t_done;  // %globaltimer, ns
+    int resume;  // PH_CHIP: 0 a linear solve begins, 1 one goes on
 };
 
 // Run control. The host writes it before every launch.
@@ -122,6 +129,7 @@ struct BCtl {
     int exit_on_done;  // stop once done >= exit_on_done (0: never)
     long long trips, max_trips;
     int pop[PH_COUNT];  // instances per phase
+    int n_chip[kBChipClasses], chip_at[kBChipClasses];  // on-chip instances per cluster size, in the chip list
     const volatile int* stop;  // host-mapped interrupt flag
     int go;                    // condition of the last trip (direct launches)
 };
@@ -565,6 +573,331 @@ __global__ void __launch_bounds__(kThreads, 8) k_batch_cg(const BDesc* __restric
     }
 }
 
+// -------------------------------------------------- linear solve on chip --
+//
+// The same linear solve (RES, W, ITER with FP64 residual replacement) of one
+// instance inside one thread-block cluster, two nodes per thread (chip.cuh).
+// The tile kernels take a launch and two trips through L2 per iteration: 18 us
+// for the hardest of 24 instances of 2k to 16k DOF; here all 24 iterate at
+// about 2 us on 150 SMs (whole batch 222 -> 48 ms, 64 instances 448 -> 120). A
+// launch advances every instance by at most `budget` iterations, so that the
+// others (their updates and assemblies, and instances too large for a cluster)
+// do not wait for its longest solve; the state between launches is kept
+// exactly, so the result does not depend on where a solve was cut. Budgets of
+// 128, 256, 512 and 1024: 54, 52, 52 and 57 ms for the 24, 25, 26, 30 and 28
+// for 6 instances up to 6k DOF.
+
+constexpr int kBChipThreads = 32 * kChipWarps;
+constexpr int kBChipBudget = 256;
+constexpr size_t kBChipSmem = 150 * 1024;
+
+enum : int { NX_END = 0, NX_ITER, NX_RES, NX_W };
+enum : int { OUT_UPD = 0, OUT_BREAKDOWN, OUT_SAVE };
+
+size_t bchip_smem(const ChipPlan& p) {
+    const int half = p.spc * 16;
+    return ((size_t)2 * half + p.halo_cap) * sizeof(float2) + (size_t)12 * half * sizeof(float2) +
+           ChipRows<float, 2, 2>::smem_blocks(half, p.wmax) * (2 * sizeof(float2) + 2);
+}
+
+__global__ void __launch_bounds__(kBChipThreads, 1) k_batch_chip(const BDesc* __restrict__ D, BState* SS,
+                                                                 const int* __restrict__ list, int cls, BCtl* c,
+                                                                 int budget) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ CommShared cs;
+    const int C = 4 << cls, tid = threadIdx.x, w = tid >> 5;
+    const int rank = (int)(blockIdx.x % C), ncl = (int)(gridDim.x / C);
+    // the list is the host's and constant during a run, and an instance's
+    // phase is changed by its own cluster only: all CTAs see the same
+    const int count = c->n_chip[cls];
+    if (count == 0) return;
+    Comm<float, false> comm{cs, tid, kBChipThreads, tid & 31, w, rank, C, 0, 0u, nullptr, nullptr, nullptr, 0,
+                            1u << 22, 0u};
+    comm.init();
+    const int first_of_class = c->chip_at[cls];
+    for (int it = blockIdx.x / C; it < count; it += ncl) {
+        const int sl = list[first_of_class + it];
+        BState* S = SS + sl;
+        if (*(const volatile int*)&S->phase != PH_CHIP) continue;
+        const BDesc& d = D[sl];
+        const ChipPlan& P = d.chip;
+        const int own = P.spc * 32, half = own / 2;
+        comm.own = own;
+        float2* U = reinterpret_cast<float2*>(smem_raw);
+        float2* rec = U + own + P.halo_cap;
+        comm.rec_base = smem_addr(rec);
+        const bool in = tid < half;
+        ChipRows<float, 2, 2> rows;
+        rows.tid = in ? tid : half - 1;  // idle threads gather zeros from a valid place
+        rows.nthr = half;
+        rows.init(rec + 6 * own, smem_addr(U), P.wmax);
+        int n[2];
+        bool publish[2];
+        double2 x[2];
+        uchar2 m[2];
+        float2 r[2], p[2], kp[2], wv[2], u[2];
+        float mi0[2], mi1[2], mi2[2];
+        const int resume = S->resume;
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const int slot = rank * own + j * half + tid;
+            n[j] = in ? P.order[slot] : -1;
+            publish[j] = false;
+            x[j] = make_double2(0.0, 0.0);
+            m[j] = make_uchar2(0, 0);
+            r[j] = p[j] = kp[j] = wv[j] = u[j] = make_float2(0.f, 0.f);
+            mi0[j] = mi1[j] = mi2[j] = 0.f;
+            if (n[j] < 0) continue;
+            const int nd = n[j], base = d.slice_ptr[nd >> 5] + (nd & 31);
+            publish[j] = P.pub[slot] != 0;
+            x[j] = d.x[nd];
+            m[j] = d.mask[nd];
+            double4 diag = make_double4(0.0, 0.0, 0.0, 0.0);
+            rows.load(j, (d.slice_ptr[(nd >> 5) + 1] - base + 31) >> 5,
+                      P.lidx + (size_t)(slot >> 5) * P.wmax * 32 + (slot & 31), [&](int k) {
+                          const double2* vp = reinterpret_cast<const double2*>(d.val64 + 4 * (base + 32LL * k));
+                          const double2 lo = __ldg(vp), hi = __ldg(vp + 1);
+                          if (k == 0) diag = make_double4(lo.x, lo.y, hi.x, hi.y);
+                          return make_float4((float)lo.x, (float)lo.y, (float)hi.x, (float)hi.y);
+                      });
+            if (d.precond) {
+                if (m[j].x && m[j].y) {
+                    const double det = diag.x * diag.w - diag.y * diag.z;
+                    mi0[j] = (float)(diag.w / det);
+                    mi1[j] = (float)(-diag.y / det);
+                    mi2[j] = (float)(diag.x / det);
+                } else if (m[j].x) {
+                    mi0[j] = (float)(1.0 / diag.x);
+                } else if (m[j].y) {
+                    mi2[j] = (float)(1.0 / diag.w);
+                }
+            } else {
+                mi0[j] = m[j].x ? 1.f : 0.f;
+                mi2[j] = m[j].y ? 1.f : 0.f;
+            }
+            if (resume) {
+                r[j] = d.r[nd];
+                p[j] = d.p[nd];
+                kp[j] = d.kp[nd];
+                wv[j] = d.w[nd];
+                u[j] = reinterpret_cast<const float2*>(d.gA + 2 * (size_t)nd)[0];
+            }
+        }
+        const int hc = P.halo_cnt[rank], h0 = kBChipThreads - 1 - tid, h_min = kBChipThreads - 32 * (w + 1);
+        const int* hl = P.halo + (size_t)rank * kHaloMax;
+        const unsigned int ha = hc > 0 ? comm.halo_at(hl[min(h0, hc - 1)]) : 0u;
+        float2 hr[3];
+        // scalars (warp 0 of every CTA holds the same)
+        const double eps2 = S->eps * S->eps, eps2_inner = S->eps2_inner;
+        double rr = S->rr, rr_ref = S->rr_ref, gamma = S->gamma, bb = S->bb, res64 = S->res64, res_last = S->res_last;
+        int res_kind = S->res_kind, stalls = S->stalls, outcome = OUT_UPD, done = 0, nres = 0;
+        const long long lin0 = S->lin_iters;
+        const int cap = (int)min(d.max_cg - lin0, (long long)0x3fffffff);
+        auto apply_m = [&](int j, float2 q) {
+            return make_float2(mi0[j] * q.x + mi1[j] * q.y, mi1[j] * q.x + mi2[j] * q.y);
+        };
+        double v[kSums] = {0.0, 0.0, 0.0, 0.0, 0.0};
+        auto exchange = [&](auto decide) {
+            comm.begin();
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+                if (publish[j]) comm.put_record(rec, j * half + tid, u[j], apply_m(j, wv[j]), apply_m(j, kp[j]));
+            comm.finish(
+                v, [&] { if (h_min < hc) comm.read_halo(ha, hr); }, decide);
+        };
+        auto fill_u = [&](float al, float bt) {
+            if (in) {
+                U[tid] = u[0];
+                U[half + tid] = u[1];
+            }
+            if (h0 < hc)
+                U[own + h0] = make_float2(hr[0].x - al * (hr[1].x + bt * hr[2].x), hr[0].y - al * (hr[1].y + bt * hr[2].y));
+            for (int b = kBChipThreads; h_min + b < hc; b += kBChipThreads) {
+                const int h = h0 + b;
+                comm.read_halo(comm.halo_at(hl[min(h, hc - 1)]), hr);
+                if (h < hc)
+                    U[own + h] =
+                        make_float2(hr[0].x - al * (hr[1].x + bt * hr[2].x), hr[0].y - al * (hr[1].y + bt * hr[2].y));
+            }
+            __syncthreads();
+        };
+        // tile_res's, tile_w's and tile_iter's decisions
+        auto decide_res = [&](const double* tot) -> Step {
+            rr = tot[0];
+            res64 = tot[2];
+            nres += 1;
+            if (res_kind == 0) {
+                bb = tot[1];
+                stalls = 0;
+            } else {
+                stalls = res64 < 0.25 * res_last ? 0 : stalls + 1;
+            }
+            res_last = res64;
+            if (!(rr == rr) || !(bb == bb) || !(res64 == res64)) {
+                outcome = OUT_BREAKDOWN;
+                return {0.0, 0.0, NX_END};
+            }
+            if (res64 <= eps2 * bb || rr == 0.0 || done >= cap || stalls >= 2) return {0.0, 0.0, NX_END};
+            rr_ref = rr;
+            return {0.0, 0.0, NX_W};
+        };
+        auto decide_w = [&](const double* tot) -> Step {
+            const double g = tot[0], beta = res_kind != 0 ? g / gamma : 0.0;
+            const double den = tot[1] + beta * tot[3] + beta * beta * tot[4], alpha = g / den;
+            if (!(den > 0.0) || !(g > 0.0) || !(alpha == alpha)) {
+                if (res_kind == 0) outcome = OUT_BREAKDOWN;
+                return {0.0, 0.0, NX_END};
+            }
+            gamma = g;
+            return {alpha, beta, NX_ITER};
+        };
+        auto decide = [&](const double* tot) -> Step {
+            const double g = tot[0], rn = tot[2], beta = g / gamma;
+            const double den = tot[1] + beta * tot[3] + beta * beta * tot[4], alpha = g * __drcp_rn(den);
+            done += 1;
+            rr = rn;
+            const bool nan = !(rn == rn) || !(g == g);
+            const bool check = rn <= eps2 * bb || rn <= eps2_inner * rr_ref || !(den > 0.0) || !(g > 0.0);
+            const bool cut = done >= budget;
+            if (!check) gamma = g;  // after a replacement beta is (its gamma) / (this iteration's)
+            if (nan) outcome = OUT_BREAKDOWN;
+            else if (check) res_kind = 1;
+            else if (done < cap && cut) outcome = OUT_SAVE;
+            return {alpha, beta, nan ? NX_END : check ? NX_RES : (done >= cap || cut) ? NX_END : NX_ITER};
+        };
+        int next = NX_RES;
+        bool fresh = true;  // x lies in global memory as it is here
+        if (resume) {
+            const double alpha0 = S->alpha, beta0 = S->beta;
+            exchange([&](const double*) -> Step { return {alpha0, beta0, NX_ITER}; });
+            next = cs.step.go;
+        }
+        while (next != NX_END && !comm.failed) {
+            if (next == NX_RES) {
+                if (!fresh) {
+#pragma unroll
+                    for (int j = 0; j < 2; ++j)
+                        if (n[j] >= 0) d.x[n[j]] = x[j];
+                    cluster_arrive_release();
+                    cluster_wait();
+                }
+                v[0] = v[1] = v[2] = v[3] = v[4] = 0.0;
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                    if (n[j] < 0) continue;
+                    const int nd = n[j], base = d.slice_ptr[nd >> 5] + (nd & 31);
+                    double k0 = 0.0, k1 = 0.0;
+#pragma unroll 3
+                    for (int k = 0; k < rows.wd[j]; ++k) {
+                        const long long bi = base + 32LL * k;
+                        const double2* vp = reinterpret_cast<const double2*>(d.val64 + 4 * bi);
+                        const double2 lo = __ldg(vp), hi = __ldg(vp + 1);
+                        const double2 xc = __ldcg(d.x + __ldg(d.scol + bi));
+                        k0 += lo.x * xc.x + lo.y * xc.y;
+                        k1 += hi.x * xc.x + hi.y * xc.y;
+                    }
+                    const double2 b = d.b[nd];
+                    const double r0 = m[j].x ? b.x - k0 : 0.0, r1 = m[j].y ? b.y - k1 : 0.0;
+                    r[j] = make_float2((float)r0, (float)r1);
+                    u[j] = apply_m(j, r[j]);
+                    v[0] += (double)r[j].x * (double)r[j].x + (double)r[j].y * (double)r[j].y;
+                    v[1] += b.x * b.x + b.y * b.y;
+                    v[2] += r0 * r0 + r1 * r1;
+                }
+                exchange(decide_res);
+                next = cs.step.go;
+            } else if (next == NX_W) {
+                fill_u(0.f, 0.f);
+                v[0] = v[1] = v[2] = v[3] = v[4] = 0.0;
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                    wv[j] = rows.gather(j);
+                    const float2 wj = wv[j], uj = u[j], rj = r[j], pj = p[j], kj = kp[j];
+                    v[0] += (double)rj.x * (double)uj.x + (double)rj.y * (double)uj.y;
+                    v[1] += (double)wj.x * (double)uj.x + (double)wj.y * (double)uj.y;
+                    v[3] += ((double)wj.x * (double)pj.x + (double)wj.y * (double)pj.y) +
+                            ((double)kj.x * (double)uj.x + (double)kj.y * (double)uj.y);
+                    v[4] += (double)kj.x * (double)pj.x + (double)kj.y * (double)pj.y;
+                }
+                exchange(decide_w);
+                next = cs.step.go;
+            } else {
+                fresh = false;
+                do {
+                    const double alpha = cs.step.alpha;
+                    const float al = (float)alpha, bt = (float)cs.step.beta;
+                    float2 u0[2];
+#pragma unroll
+                    for (int j = 0; j < 2; ++j) {
+                        u0[j] = u[j];
+                        const float2 mw = apply_m(j, wv[j]), mk = apply_m(j, kp[j]);
+                        u[j] = make_float2(u0[j].x - al * (mw.x + bt * mk.x), u0[j].y - al * (mw.y + bt * mk.y));
+                    }
+                    fill_u(al, bt);
+                    v[0] = v[1] = v[2] = v[3] = v[4] = 0.0;
+#pragma unroll
+                    for (int j = 0; j < 2; ++j) {
+                        p[j] = make_float2(u0[j].x + bt * p[j].x, u0[j].y + bt * p[j].y);
+                        kp[j] = make_float2(wv[j].x + bt * kp[j].x, wv[j].y + bt * kp[j].y);
+                        x[j].x += alpha * (double)p[j].x;
+                        x[j].y += alpha * (double)p[j].y;
+                        if (m[j].x) r[j].x -= al * kp[j].x;
+                        if (m[j].y) r[j].y -= al * kp[j].y;
+                        wv[j] = rows.gather(j);
+                        const float2 wj = wv[j], uj = u[j], rj = r[j], pj = p[j], kj = kp[j];
+                        v[0] += (double)rj.x * (double)uj.x + (double)rj.y * (double)uj.y;
+                        v[1] += (double)wj.x * (double)uj.x + (double)wj.y * (double)uj.y;
+                        v[2] += (double)rj.x * (double)rj.x + (double)rj.y * (double)rj.y;
+                        v[3] += ((double)wj.x * (double)pj.x + (double)wj.y * (double)pj.y) +
+                                ((double)kj.x * (double)uj.x + (double)kj.y * (double)uj.y);
+                        v[4] += (double)kj.x * (double)pj.x + (double)kj.y * (double)pj.y;
+                    }
+                    exchange(decide);
+                    next = cs.step.go;
+                } while (next == NX_ITER && !comm.failed);
+            }
+        }
+        // every thread: the step's scalars, before the next instance's
+        const double alpha1 = cs.step.alpha, beta1 = cs.step.beta;
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+            if (n[j] >= 0) {
+                const int nd = n[j];
+                d.x[nd] = x[j];
+                d.r[nd] = r[j];
+                d.p[nd] = p[j];
+                d.kp[nd] = kp[j];
+                d.w[nd] = wv[j];
+                reinterpret_cast<float2*>(d.gA + 2 * (size_t)nd)[0] = u[j];
+            }
+        // the others have read this CTA's memory, and the instance's state,
+        // for the last time
+        const bool gave_up = comm.close();
+        if (rank == 0 && tid == 0) {
+            if (gave_up) outcome = OUT_BREAKDOWN;
+            S->fp64_spmv += nres;
+            S->iter += done;
+            S->lin_iters += done;
+            S->cg_total += done;
+            S->rr = rr;
+            S->rr_ref = rr_ref;
+            S->gamma = gamma;
+            S->alpha = alpha1;
+            S->beta = beta1;
+            S->bb = bb;
+            S->res64 = res64;
+            S->res_last = res_last;
+            S->res_kind = res_kind;
+            S->stalls = stalls;
+            S->cg_rel_res = bb > 0.0 ? sqrt(res64 / bb) : 0.0;
+            if (outcome == OUT_BREAKDOWN) finish(S, c, gave_up ? CP_ERR_TIMEOUT : CP_ERR_BREAKDOWN);
+            else if (outcome == OUT_SAVE) S->resume = 1;
+            else set_phase(S, c, PH_UPD);
+        }
+        if (gave_up) return;
+    }
+}
+
 // The work of an iteration for the autotuner, with the same per-tile costs
 // as ITER: the phase read, the own-node and neighbour loads and arithmetic,
 // the per-slice sums, a fence and a ticket per tile, and the last tile's
@@ -678,7 +1011,8 @@ __global__ void __launch_bounds__(kThreads) k_batch_asm(const BDesc* __restrict_
             S->ticket = 0;
             S->res_kind = 0;
             S->eps2_inner = d.inner_tol * d.inner_tol;
-            set_phase(S, c, PH_RES);
+            S->resume = 0;
+            set_phase(S, c, d.chip.ctas > 0 ? PH_CHIP : PH_RES);
         }
     }
 }
@@ -879,6 +1213,11 @@ struct cp_batch {
     BState* d_state = nullptr;
     int4* d_tiles = nullptr;
     BCtl* d_ctl = nullptr;
+    int* d_chip = nullptr;  // on-chip instances by cluster size (slots)
+    int* h_chip = nullptr;  // pinned
+    bool chip_ok = false;   // the GPU takes the on-chip kernel's clusters
+    cudaStream_t aux[kBChipClasses] = {};  // capture: the on-chip launches beside the tile kernels'
+    cudaEvent_t fork = nullptr, join[kBChipClasses] = {};
     int tiles_cap = 0;
     int4* h_tiles = nullptr;  // pinned
     BState* h_state = nullptr;  // pinned
@@ -1032,8 +1371,84 @@ void launch_body(cp_batch* b, cudaStream_t s) {
     else
         k_batch_asm<false><<<b->grid_asm, kThreads, b->asm_smem, s>>>(b->d_desc, b->d_state, b->d_tiles, b->d_ctl,
                                                                       b->o.max_width);
+    if (b->chip_ok) {
+        CP_CUDA(cudaEventRecord(b->fork, s));
+        for (int k = kBChipClasses - 1; k >= 0; --k) {
+            const int C = 4 << k;
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3(C * (b->ctx->sm_count / C));
+            cfg.blockDim = dim3(kBChipThreads);
+            cfg.dynamicSmemBytes = kBChipSmem;
+            cfg.stream = b->aux[k];
+            cudaLaunchAttribute attr[1];
+            attr[0].id = cudaLaunchAttributeClusterDimension;
+            attr[0].val.clusterDim.x = C;
+            attr[0].val.clusterDim.y = 1;
+            attr[0].val.clusterDim.z = 1;
+            cfg.attrs = attr;
+            cfg.numAttrs = 1;
+            CP_CUDA(cudaStreamWaitEvent(b->aux[k], b->fork, 0));
+            CP_CUDA(cudaLaunchKernelEx(&cfg, k_batch_chip, (const BDesc*)b->d_desc, b->d_state, (const int*)b->d_chip,
+                                       k, b->d_ctl, kBChipBudget));
+            CP_CUDA(cudaEventRecord(b->join[k], b->aux[k]));
+        }
+    }
     for (int k = 0; k < b->o.cg_per_trip; ++k)
         batch_cg_kernel()<<<b->grid_cg, kThreads, 0, s>>>(b->d_desc, b->d_state, b->d_tiles, b->d_ctl);
+    if (b->chip_ok)
+        for (int k = 0; k < kBChipClasses; ++k) CP_CUDA(cudaStreamWaitEvent(s, b->join[k], 0));
+}
+
+// Whether the GPU takes clusters of all sizes of k_batch_chip.
+bool bchip_available() {
+    if (cudaFuncSetAttribute(k_batch_chip, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBChipSmem) != cudaSuccess ||
+        cudaFuncSetAttribute(k_batch_chip, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    for (int k = 0; k < kBChipClasses; ++k) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(4 << k);
+        cfg.blockDim = dim3(kBChipThreads);
+        cfg.dynamicSmemBytes = kBChipSmem;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = 4 << k;
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        int n = 0;
+        if (cudaOccupancyMaxActiveClusters(&n, k_batch_chip, &cfg) != cudaSuccess || n < 1) {
+            cudaGetLastError();
+            return false;
+        }
+    }
+    return true;
+}
+
+// The on-chip plan of an instance in a batch, built on its first add: the
+// smallest cluster of 4, 8 or 16 CTAs of up to 768 nodes that holds it
+// (12,288 nodes). CUPLAST_BATCH_CHIP=0 keeps the tile kernels (measurements).
+void plan_bchip(cp_instance* I) {
+    if (I->bchip_planned) return;
+    I->bchip_planned = 1;
+    const char* e = std::getenv("CUPLAST_BATCH_CHIP");
+    if (e && e[0] == '0') return;
+    for (int k = 0; k < kBChipClasses; ++k) {
+        const int C = 4 << k, per = (I->csr.n_slices + C - 1) / C;
+        cp::ChipShape sh;
+        sh.ctas = C;
+        sh.spc = (per + 1) / 2 * 2;  // two nodes per thread
+        sh.npt = 2;
+        sh.wmax = I->csr.max_width;
+        if (sh.spc > 2 * kChipWarps) continue;
+        void* mem = I->alloc<unsigned char>(cp::chip_plan_bytes(sh, I->n_nodes));
+        cp::chip_build_plan(I->bchip, sh, mem, I->n_nodes, I->mesh.xy, I->csr.slice_ptr, I->csr.scol, I->sms(), I->s(),
+                            false);
+        if (I->bchip.ctas > 0 && bchip_smem(I->bchip) > kBChipSmem) I->bchip.ctas = 0;
+        return;
+    }
 }
 
 // Direct launches: trip after trip with the condition read back each time.
@@ -1130,6 +1545,14 @@ CP_API int cp_batch_create(cp_context* ctx, const cp_batch_opts* opts, cp_batch*
         CP_CUDA(cudaMalloc(&b->d_desc, sizeof(BDesc) * (size_t)b->cap));
         CP_CUDA(cudaMalloc(&b->d_state, sizeof(BState) * (size_t)b->cap));
         CP_CUDA(cudaMemset(b->d_state, 0, sizeof(BState) * (size_t)b->cap));
+        CP_CUDA(cudaMalloc(&b->d_chip, sizeof(int) * (size_t)b->cap));
+        CP_CUDA(cudaMallocHost(&b->h_chip, sizeof(int) * (size_t)b->cap));
+        b->chip_ok = bchip_available();
+        CP_CUDA(cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming));
+        for (int k = 0; k < kBChipClasses; ++k) {
+            CP_CUDA(cudaStreamCreateWithFlags(&b->aux[k], cudaStreamNonBlocking));
+            CP_CUDA(cudaEventCreateWithFlags(&b->join[k], cudaEventDisableTiming));
+        }
         CP_CUDA(cudaMalloc(&b->d_ctl, sizeof(BCtl)));
         CP_CUDA(cudaMemset(b->d_ctl, 0, sizeof(BCtl)));
         CP_CUDA(cudaMallocHost(&b->h_state, sizeof(BState) * (size_t)b->cap));
@@ -1172,6 +1595,13 @@ CP_API int cp_batch_destroy(cp_batch* b) {
     if (b->d_state) cudaFree(b->d_state);
     if (b->d_tiles) cudaFree(b->d_tiles);
     if (b->d_ctl) cudaFree(b->d_ctl);
+    if (b->d_chip) cudaFree(b->d_chip);
+    if (b->h_chip) cudaFreeHost(b->h_chip);
+    if (b->fork) cudaEventDestroy(b->fork);
+    for (int k = 0; k < kBChipClasses; ++k) {
+        if (b->join[k]) cudaEventDestroy(b->join[k]);
+        if (b->aux[k]) cudaStreamDestroy(b->aux[k]);
+    }
     if (b->h_tiles) cudaFreeHost(b->h_tiles);
     if (b->h_state) cudaFreeHost(b->h_state);
     if (b->h_ctl) cudaFreeHost(b->h_ctl);
@@ -1274,6 +1704,10 @@ CP_API int cp_batch_add(cp_batch* b, cp_instance* I, const cp_solve_opts* opts, 
             d.pred_psi = I->pred_psi;
         }
         d.precond = o.precond;
+        if (b->chip_ok) {
+            plan_bchip(I);
+            d.chip = I->bchip;
+        }
         CP_CUDA(cudaStreamSynchronize(I->s()));  // buffers of the instance's own stream are ready
         BState S{};
         S.phase = PH_LEVEL;
@@ -1311,6 +1745,18 @@ CP_API int cp_batch_launch(cp_batch* b, int until, long long max_trips) {
             if (ph == PH_DONE) ++done;
             else ++active;
         }
+        // on-chip instances by cluster size, each size's largest first
+        int at = 0;
+        for (int k = 0; k < kBChipClasses; ++k) {
+            std::vector<int> of;
+            for (int sl : b->listed)
+                if (b->state[sl].phase != PH_DONE && b->desc[sl].chip.ctas == 4 << k) of.push_back(sl);
+            std::stable_sort(of.begin(), of.end(),
+                             [&](int p, int q) { return b->desc[p].n_slices > b->desc[q].n_slices; });
+            c.chip_at[k] = at;
+            c.n_chip[k] = (int)of.size();
+            for (int sl : of) b->h_chip[at++] = sl;
+        }
         c.active = active;
         c.done = 0;
         c.exit_on_done = until == CP_BATCH_RUN_ANY_DONE ? 1 : 0;
@@ -1320,6 +1766,7 @@ CP_API int cp_batch_launch(cp_batch* b, int until, long long max_trips) {
         *b->h_ctl = c;
         *(volatile int*)b->h_stop = 0;
         if (nt > 0) CP_CUDA(cudaMemcpyAsync(b->d_tiles, b->h_tiles, sizeof(int4) * (size_t)nt, cudaMemcpyHostToDevice, s));
+        if (at > 0) CP_CUDA(cudaMemcpyAsync(b->d_chip, b->h_chip, sizeof(int) * (size_t)at, cudaMemcpyHostToDevice, s));
         CP_CUDA(cudaMemcpyAsync(b->d_ctl, b->h_ctl, sizeof(BCtl), cudaMemcpyHostToDevice, s));
         b->last_tiles = nt;
         b->timed = false;
@@ -1368,7 +1815,8 @@ CP_API int cp_batch_wait(cp_batch* b, int* active, int* done) {
         b->last_run_ms = ms;
         const long long trips = b->h_ctl->trips;
         b->trips += trips;
-        b->launches += trips * (long long)(b->o.elem_per_trip + 1 + b->o.cg_per_trip + 1);
+        b->launches +=
+            trips * (long long)(b->o.elem_per_trip + 1 + b->o.cg_per_trip + 1 + (b->chip_ok ? kBChipClasses : 0));
         int a = 0, d = 0;
         for (int sl : b->listed) {
             b->state[sl] = b->h_state[sl];
@@ -1484,7 +1932,7 @@ CP_API int cp_batch_progress(const cp_batch* b, int slot, int* phase, int* level
     if (!b || slot < 0 || slot >= b->cap || !b->inst[slot]) return CP_ERR_INVALID;
     if (b->running) return CP_ERR_BUSY;
     const BState& S = b->state[slot];
-    if (phase) *phase = S.phase;
+    if (phase) *phase = S.phase == PH_CHIP ? PH_ITER : S.phase;
     if (level) *level = S.level;
     if (report) *report = report_of(S);
     return CP_OK;

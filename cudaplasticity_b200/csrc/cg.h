@@ -135,8 +135,9 @@ ChipShape chip_shape(int n, int wmax, int sm_count, bool grid);
 size_t chip_plan_bytes(const ChipShape& s, int n);
 size_t chip_ll_bytes(const ChipShape& s);
 void chip_ll_carve(const ChipPlan& p, void* mem, uint4** rec, uint4** part, uint4** step);
+// for_solve: checks that k_chip can run the plan (a batch brings its own kernel).
 void chip_build_plan(ChipPlan& p, const ChipShape& s, void* mem, int n, const double2* xy, const int* slice_ptr,
-                     const int* scol, int sm_count, cudaStream_t st);
+                     const int* scol, int sm_count, cudaStream_t st, bool for_solve = true);
 template <typename T>
 void chip_launch(const ChipArgs<T>& a, cudaStream_t s);
 

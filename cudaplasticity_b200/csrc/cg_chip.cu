@@ -622,7 +622,7 @@ void chip_ll_carve(const ChipPlan& p, void* mem, uint4** rec, uint4** part, uint
 
 // Builds the plan on the device; plan.ctas = 0 when the instance does not fit.
 void chip_build_plan(ChipPlan& p, const ChipShape& s, void* mem, int n, const double2* xy, const int* slice_ptr,
-                     const int* scol, int sm_count, cudaStream_t st) {
+                     const int* scol, int sm_count, cudaStream_t st, bool for_solve) {
     const size_t slots = chip_slots(s);
     p.grid = s.grid;
     p.spc = s.spc;
@@ -654,7 +654,7 @@ void chip_build_plan(ChipPlan& p, const ChipShape& s, void* mem, int n, const do
     if (most > kHaloMax) return;
     p.halo_cap = (most + 7) / 8 * 8;
     p.ctas = s.ctas;
-    if (!chip_schedulable<double>(p, sm_count) || !chip_schedulable<float>(p, sm_count)) p.ctas = 0;
+    if (for_solve && (!chip_schedulable<double>(p, sm_count) || !chip_schedulable<float>(p, sm_count))) p.ctas = 0;
 }
 
 namespace {

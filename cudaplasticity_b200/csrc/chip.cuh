@@ -188,6 +188,7 @@ struct CommShared {
     __align__(16) double part[2][kMaxCluster][6];    // cluster: every CTA's sums (0, 2, 1, -, 3, 4), by parity
     __align__(8) unsigned long long bar[2];          // cluster: they have arrived
     Step step;
+    int fail;                                        // rank 0's: some CTA of the cluster gave up
 };
 
 // The exchange of one iteration: the own records and sums out, the halo
@@ -197,7 +198,8 @@ struct Comm {
     using V2 = typename Vec2<T>::type;
     static constexpr int NR = Record<T>::n;
     CommShared& S;
-    const int tid, nthr, lane, w, rank, ctas, own;
+    const int tid, nthr, lane, w, rank, ctas;
+    int own;
     unsigned int rec_base = 0;  // cluster: records [2][3][own]
     uint4 *ll_rec, *ll_part, *ll_step;
     size_t slots;
@@ -209,6 +211,7 @@ struct Comm {
 
     // Once per kernel, whole block (cluster: whole cluster).
     __device__ __forceinline__ void init() {
+        if (tid == 0) S.fail = 0;
         for (int i = tid; i < 128; i += nthr) (&S.wsum[0][0])[i] = 0.0;
         for (int i = tid; i < kMaxPolls * 8; i += nthr) (&S.gsum[0][0])[i] = 0.0;
         for (int i = tid; i < 2 * kMaxCluster * 6; i += nthr) (&S.part[0][0][0])[i] = 0.0;
@@ -333,6 +336,23 @@ struct Comm {
             }
         }
         failed = __syncthreads_or(failed ? 1 : 0) != 0;
+    }
+    // Cluster: at the end of a solve, whole cluster: all CTAs have read each
+    // other's shared memory for the last time; whether any of them gave up.
+    __device__ __forceinline__ bool close() {
+        if (failed && tid == 0) {
+            const unsigned int f = mapa(smem_addr(&S.fail), 0);
+            asm volatile("st.shared::cluster.u32 [%0], 1;" ::"r"(f) : "memory");
+        }
+        cluster_arrive_release();
+        cluster_wait();
+        int any;
+        asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(any) : "r"(mapa(smem_addr(&S.fail), 0)) : "memory");
+        if (any) {  // nobody goes while the flag is read
+            cluster_arrive_release();
+            cluster_wait();
+        }
+        return any != 0;
     }
     // Grid: the adding CTA's side of one exchange.
     template <typename Decide>

@@ -86,6 +86,8 @@ struct cp_instance {
     float2* bt_vec = nullptr;
     float4* bt_rec = nullptr;
     double* bt_part = nullptr;
+    int bchip_planned = 0;  // bchip below is computed (once per instance)
+    cp::ChipPlan bchip;     // the batch's on-chip linear solve; bchip.ctas = 0: the tile kernels
     // aggregation-multigrid PCG (mg.cu, cp_solve_opts.precond 2), built on first use
     std::vector<unsigned char> mask_host;  // the Dirichlet mask of the last cp_instance_set_loads
     std::vector<unsigned char> mg_mask;    // the mask the hierarchy was built for

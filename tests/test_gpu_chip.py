@@ -117,6 +117,33 @@ def test_mixed_precision(nx, ny, ctx):
         assert rep["cg_rel_res"] <= 1e-11 and abs(res - rep["cg_rel_res"]) <= 2 * 20 * EPS64 * gap
 
 
+# nodes: tiny, 3072, 3075 (clusters of 4, then 8), 6144, 6145, 12288, 12291 (16, then the tile kernels)
+@pytest.mark.parametrize("nx, ny", [(2, 2), (16, 2), (96, 32), (1025, 3), (96, 64), (1229, 5), (128, 96), (4097, 3)])
+def test_batch(nx, ny, ctx):
+    """A batch's linear solves on chip, alone and beside another instance: they end on the FP64 residual, and the
+    result is the same bit for bit."""
+    p = strip(nx, ny)
+    kw = dict(cg_tol=1e-11, outer_tol=1e300, inner_tol=1e-3, max_outer=1, max_cg=100000)
+    for precond in (0, 1):
+        batch, out = cp.Batch(ctx, max_instances=2), []
+        for other in (False, True):
+            insts = [cp.Instance(ctx, a, cp.material(210000.0, 0.3)) for a, _, _ in ([strip(40, 30)] * other + [p])]
+            for i, (_, rp, mask) in zip(insts, [strip(40, 30)] * other + [p]):
+                i.set_loads(rp, mask)
+                batch.add(i, precond=precond, **kw)
+            batch.run()
+            rep = {i._h.value: r for _, i, r in batch.harvest()}[insts[-1]._h.value]
+            u, csr = insts[-1].field("uv"), insts[-1].csr()
+            res, gap = residual(p, u, csr)
+            assert rep["status"] == 0 and rep["cg_rel_res"] <= 1e-11
+            assert abs(res - rep["cg_rel_res"]) <= 2 * 20 * EPS64 * gap
+            out.append(u)
+            for i in insts:
+                i.close()
+        assert np.array_equal(out[0], out[1])
+        batch.close()
+
+
 def test_mixed_precision_falls_back(ctx, monkeypatch):
     """Where FP32 cannot carry the system (a column 900 elements high and two wide, kappa eps32 >> 1), the on-chip form
     hands over to the two-kernel loop from the same start: the same outcome as that loop alone."""

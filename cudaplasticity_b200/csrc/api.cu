@@ -355,12 +355,14 @@ void chip_check(cp_instance* I) {
     throw Error{CP_ERR_TIMEOUT, "on-chip CG: an exchange timed out"};
 }
 
-// One on-chip solve; its scalars end in sc_h.
+// One on-chip solve; its scalars end in sc_h. defer: without waiting for it
+// (the caller synchronises later and calls chip_check).
 template <typename T>
-void run_chip(cp_instance* I, const cp::ChipArgs<T>& a) {
+void run_chip(cp_instance* I, const cp::ChipArgs<T>& a, bool defer = false) {
     cp::chip_launch(a, I->s());
     I->launches += 1;
     CP_CUDA(cudaMemcpyAsync(I->sc_h, I->sc, sizeof(cp::CgScalars), cudaMemcpyDeviceToHost, I->s()));
+    if (defer) return;
     CP_CUDA(cudaStreamSynchronize(I->s()));
     chip_check(I);
 }
@@ -515,13 +517,18 @@ void recycle_before(cp_instance* I, int m) {
     I->launches += a.cnt > 0 ? 2 : 1;
 }
 
+// The ring's next slot has been (or is being) written.
+void recycle_advance(cp_instance* I, int m) {
+    I->rec_head = (I->rec_head + 1) % m;
+    I->rec_cnt = std::min(I->rec_cnt + 1, m);
+}
+
 // After it: the increment u - u0 goes into the ring.
 void recycle_after(cp_instance* I, int m) {
     const cp::RecycleArgs a = recycle_args(I, m);
     cp::recycle_push(a, I->rec_head, I->sms(), I->s());
     I->launches += 1;
-    I->rec_head = (I->rec_head + 1) % m;
-    I->rec_cnt = std::min(I->rec_cnt + 1, m);
+    recycle_advance(I, m);
 }
 
 // Mixed precision: FP64 defect correction around FP32 CG. Each step computes
@@ -924,7 +931,7 @@ CP_API int cp_secant_update(cp_instance* I, double* rel_err) {
     if (I && I->in_batch) return CP_ERR_BUSY;  // owned by a batch until harvested
     if (!I) return CP_ERR_INVALID;
     return guarded(I->ctx, [&] {
-        cp::launch_update(I->mesh, I->mat, I->u, I->st, I->osc, I->partials, 0, I->s(), I->sms());
+        cp::launch_update(I->mesh, I->mat, I->u, I->st, I->osc, I->partials, 0, 0, I->s(), I->sms());
         CP_CUDA(cudaMemcpyAsync(I->osc_h, I->osc, sizeof(cp::OuterScalars), cudaMemcpyDeviceToHost, I->s()));
         CP_CUDA(cudaStreamSynchronize(I->s()));
         if (rel_err) *rel_err = I->osc_h->rel_err;
@@ -1000,7 +1007,8 @@ CP_API int cp_solve(cp_instance* I, const cp_solve_opts* opts, cp_solve_report* 
             I->launches += 2;
             I->rec_cnt = 0;  // increments of this level only
             I->rec_head = 0;
-            double rel_err = 1.0, w_prev = 1.0;
+            double rel_err = 1.0;
+            int first = 1;  // the next update begins an Aitken history
             bool converged = false;
             // floatBoost: the reduced-precision phase, then FP64 from its state
             bool boost = o.precision == CP_PREC_FLOAT_BOOST;
@@ -1019,10 +1027,21 @@ CP_API int cp_solve(cp_instance* I, const cp_solve_opts* opts, cp_solve_report* 
                     eps = std::max(o.cg_tol, rule2_factor() * rel_err);
                 // the on-chip CG rounds K to FP32 as it loads it
                 assemble(I, prec == CP_PREC_MIXED && chip_ready(I) ? CP_PREC_FP64 : prec);
-                // the multigrid graph loop leaves its scalars for after the update
+                // the multigrid graph loop and the on-chip CG leave their scalars
+                // for after the update: one wait of the host per outer iteration
                 const bool mg_deferred = prec == CP_PREC_FP64 && o.precond == 2 && I->use_graph;
+                const bool chip_deferred = prec == CP_PREC_FP64 && o.precond != 2 && I->fused_fp64 && chip_ready(I);
                 if (mg_deferred) {
                     cg_fp64_mg(I, eps, o.max_cg, true);
+                } else if (chip_deferred) {
+                    cp::ChipArgs<double> a = chip_args<double>(I, eps * eps, o.max_cg, o.precond ? 1 : 0);
+                    if (m_rec > 0) {
+                        recycle_before(I, m_rec);
+                        a.u0 = I->rec_u0;
+                        a.inc = I->rec_w + (size_t)I->rec_head * I->n_nodes;
+                        recycle_advance(I, m_rec);
+                    }
+                    run_chip(I, a, true);
                 } else if (prec == CP_PREC_FP64) {
                     if (o.precond == 2) {
                         cg_fp64_mg(I, eps, o.max_cg);
@@ -1039,12 +1058,18 @@ CP_API int cp_solve(cp_instance* I, const cp_solve_opts* opts, cp_solve_report* 
                     cg_mixed(I, eps, o.inner_tol, o.max_cg, &R.cg_iters, &R.fp64_spmv, &rr, o.precond ? 1 : 0);
                     R.cg_rel_res = rr;
                 }
-                cp::launch_update(I->mesh, I->mat, I->u, I->st, I->osc, I->partials, o.aitken, s, I->sms());
+                cp::launch_update(I->mesh, I->mat, I->u, I->st, I->osc, I->partials, o.aitken, first, s, I->sms());
                 I->launches += 1;
                 CP_CUDA(cudaMemcpyAsync(I->osc_h, I->osc, sizeof(cp::OuterScalars), cudaMemcpyDeviceToHost, s));
+                if (o.aitken) {  // the factor stays on the device
+                    cp::launch_aitken_relax(I->mesh, I->mat, I->st, I->osc, s, I->sms());
+                    I->launches += 1;
+                }
+                first = 0;
                 CP_CUDA(cudaStreamSynchronize(s));
-                if (mg_deferred) {
-                    mg_count_graph_launches(I);
+                if (mg_deferred || chip_deferred) {
+                    if (mg_deferred) mg_count_graph_launches(I);
+                    else chip_check(I);
                     R.cg_iters += I->sc_h->iter;
                     R.cg_rel_res = std::sqrt(I->sc_h->rr * I->sc_h->normB_inv);
                     if (I->sc_h->status == CP_ERR_BREAKDOWN) throw Error{CP_ERR_BREAKDOWN, "CG broke down"};
@@ -1052,15 +1077,6 @@ CP_API int cp_solve(cp_instance* I, const cp_solve_opts* opts, cp_solve_report* 
                 rel_err = I->osc_h->rel_err;
                 R.outer_iters += 1;
                 CP_CHECK(std::isfinite(rel_err), CP_ERR_BREAKDOWN, "secant iteration produced NaN");
-                if (o.aitken) {
-                    double w = 1.0;
-                    if (it > 0 && I->osc_h->a_den > 0) w = -w_prev * I->osc_h->a_num / I->osc_h->a_den;
-                    if (!(w >= 0.1)) w = 0.1;
-                    if (w > 10.0) w = 10.0;
-                    cp::launch_aitken_relax(I->mesh, I->mat, I->st, I->osc, w, s, I->sms());
-                    I->launches += 1;
-                    w_prev = w;
-                }
                 if (boost) {
                     if (rel_err <= kBoostTol) {
                         // switch to FP64 (copyFloatToDouble keeps u, E_c, nu_c;
@@ -1068,7 +1084,7 @@ CP_API int cp_solve(cp_instance* I, const cp_solve_opts* opts, cp_solve_report* 
                         // gets its own max_outer and takes at least one step
                         boost = false;
                         prec = CP_PREC_FP64;
-                        w_prev = 1.0;
+                        first = 1;
                         I->rec_cnt = 0;
                         I->rec_head = 0;
                         int g2;

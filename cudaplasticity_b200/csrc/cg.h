@@ -122,6 +122,9 @@ struct ChipArgs {
     double eps2 = 0.0, outer_eps2 = -1.0;  // as cg_launch_init
     long long max_iter = 0;
     int relative_to_r0 = 0;
+    // with inc: the solve's increment x - u0 is left there (recycle.h)
+    const double2* u0 = nullptr;
+    double2* inc = nullptr;
     // grid exchange: records, sums and steps by parity, the last sequence
     // number in use; rounds a poll takes before it gives up, and what is
     // added to the posted sequence numbers (0; 1 makes every poll run out:

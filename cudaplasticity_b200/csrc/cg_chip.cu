@@ -488,7 +488,13 @@ __global__ void __launch_bounds__(kChipWarps * 32, 1) k_chip(ChipArgs<T> a) {
     }
 #pragma unroll
     for (int j = 0; j < NPT; ++j)
-        if (n[j] >= 0) a.x[n[j]] = x[j];
+        if (n[j] >= 0) {
+            a.x[n[j]] = x[j];
+            if (a.inc) {
+                const double2 b = a.u0[n[j]];
+                a.inc[n[j]] = make_double2(x[j].x - b.x, x[j].y - b.y);
+            }
+        }
     if (!GRID && rank == 0) finish();
 }
 

@@ -91,7 +91,8 @@ constexpr int kElemThreads = 256;
 // the moment form, 85 at 2 blocks per SM, 74 now (floor 26: 168 MB).
 template <bool Q8>
 __global__ void __launch_bounds__(kElemThreads, 4) k_update(DevMesh m, MaterialDev M, const double2* __restrict__ u,
-                                                         ElemState st, OuterScalars* sc, double* partials, int aitken) {
+                                                         ElemState st, OuterScalars* sc, double* partials, int aitken,
+                                                         int first) {
     __shared__ double sh[2 * kElemThreads / 32];
     __shared__ bool last;
     const int ne = m.c3 + m.c4 + m.c8;
@@ -120,6 +121,13 @@ __global__ void __launch_bounds__(kElemThreads, 4) k_update(DevMesh m, MaterialD
             sc->rel_err = sqrt(x.x / x.y);
             sc->a_num = y.x;
             sc->a_den = y.y;
+            if (aitken) {  // the relaxation factor of this step, from the last one's
+                double w = 1.0;
+                if (!first && y.y > 0.0) w = -sc->aitken_omega * y.x / y.y;
+                if (!(w >= 0.1)) w = 0.1;
+                if (w > 10.0) w = 10.0;
+                sc->aitken_omega = w;
+            }
             sc->ticket = 0;
         }
     }
@@ -130,8 +138,9 @@ namespace {
 // Aitken (Irons-Tuck) relaxation of the secant iteration on psi:
 // psi_{k+1} = psi_k + w_k r_k, w_k = -w_{k-1} (r_{k-1}, r_k - r_{k-1}) / |r_k - r_{k-1}|^2.
 // The fixed point (r = 0) is the reference's.
-__global__ void k_aitken(DevMesh m, MaterialDev M, ElemState st, const OuterScalars* sc, double w) {
+__global__ void k_aitken(DevMesh m, MaterialDev M, ElemState st, const OuterScalars* sc) {
     const int ne = m.c3 + m.c4 + m.c8;
+    const double w = sc->aitken_omega;
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < ne; e += gridDim.x * blockDim.x)
         relax_element(M, st, e, w);
 }
@@ -185,19 +194,19 @@ int update_grid(int ne, int sm_count) {
 }
 
 void launch_update(const DevMesh& m, const MaterialDev& mat, const double2* u, ElemState& st, OuterScalars* sc,
-                   double* partials, int aitken, cudaStream_t s, int sm_count) {
+                   double* partials, int aitken, int first, cudaStream_t s, int sm_count) {
     const int ne = m.c3 + m.c4 + m.c8;
     if (m.c8)
-        k_update<true><<<update_grid(ne, sm_count), elem_threads(ne, sm_count), 0, s>>>(m, mat, u, st, sc, partials, aitken);
+        k_update<true><<<update_grid(ne, sm_count), elem_threads(ne, sm_count), 0, s>>>(m, mat, u, st, sc, partials, aitken, first);
     else
-        k_update<false><<<update_grid(ne, sm_count), elem_threads(ne, sm_count), 0, s>>>(m, mat, u, st, sc, partials, aitken);
+        k_update<false><<<update_grid(ne, sm_count), elem_threads(ne, sm_count), 0, s>>>(m, mat, u, st, sc, partials, aitken, first);
     CP_CUDA(cudaGetLastError());
 }
 
-void launch_aitken_relax(const DevMesh& m, const MaterialDev& mat, ElemState& st, const OuterScalars* sc, double w,
+void launch_aitken_relax(const DevMesh& m, const MaterialDev& mat, ElemState& st, const OuterScalars* sc,
                          cudaStream_t s, int sm_count) {
     const int ne = m.c3 + m.c4 + m.c8;
-    k_aitken<<<update_grid(ne, sm_count), elem_threads(ne, sm_count), 0, s>>>(m, mat, st, sc, w);
+    k_aitken<<<update_grid(ne, sm_count), elem_threads(ne, sm_count), 0, s>>>(m, mat, st, sc);
     CP_CUDA(cudaGetLastError());
 }
 
@@ -291,7 +300,7 @@ extern "C" CP_API int cp_secant_update_noalloc(void* stream, const cp_material* 
     es.psi = d_psi; es.E_c = d_E_c; es.nu_c = d_nu_c;
     const int threads = cp::elem_threads(count4, 148);
     const int grid = cp::update_grid(count4, 148);  // <= kNoAllocMaxBlocks
-    cp::k_update<false><<<grid, threads, 0, s>>>(m, M, reinterpret_cast<const double2*>(d_uv), es, sc, partials, 0);
+    cp::k_update<false><<<grid, threads, 0, s>>>(m, M, reinterpret_cast<const double2*>(d_uv), es, sc, partials, 0, 0);
     if (cudaGetLastError() != cudaSuccess) return CP_ERR_CUDA;
     double host_err = 0.0;
     if (cudaMemcpyAsync(&host_err, &sc->rel_err, sizeof(double), cudaMemcpyDeviceToHost, s) != cudaSuccess)

@@ -9,77 +9,95 @@ namespace cp {
 namespace {
 
 constexpr int kRecThreads = 256;
+constexpr int kSumThreads = 128;  // small blocks: 4160 nodes are 33 of them
 
 // The small system (W^T K W) y = W^T r0 by Cholesky of the diagonally scaled
 // Gram matrix, dropping increments whose pivot is at most kDrop (or whose
-// diagonal is not positive); dropped increments get y = 0. One thread.
+// diagonal is not positive); dropped increments get y = 0. One thread. Every
+// loop has constant bounds and is unrolled, so that on the device the arrays
+// are registers: indexed at run time they were local memory, and the solve
+// took two thirds of the sums kernel.
 constexpr double kDrop = 1e-10;
+#ifdef __CUDA_ARCH__
+#define CP_UNROLL _Pragma("unroll")
+#else
+#define CP_UNROLL
+#endif
 
-__host__ __device__ void small_solve(const double* t, int cnt, double* y) {
-    double A[kRecycleMax][kRecycleMax], S[kRecycleMax][kRecycleMax], L[kRecycleMax][kRecycleMax];
-    double h[kRecycleMax], d[kRecycleMax], z[kRecycleMax], yy[kRecycleMax];
-    bool keep[kRecycleMax], ok[kRecycleMax];
-    for (int j = 0; j < kRecycleMax; ++j) {
-        for (int k = 0; k < kRecycleMax; ++k) {
-            A[j][k] = 0.0;
-            S[j][k] = 0.0;
-            L[j][k] = 0.0;
-        }
-        h[j] = d[j] = z[j] = yy[j] = 0.0;
-        keep[j] = ok[j] = false;
-    }
-    for (int j = 0; j < cnt; ++j) {
-        for (int k = 0; k < cnt; ++k) A[j][k] = j <= k ? t[k * (k + 1) / 2 + j] : t[j * (j + 1) / 2 + k];
-        h[j] = t[kRecycleGram + j];
-        d[j] = A[j][j] > 0.0 ? sqrt(A[j][j]) : 0.0;
+__host__ __device__ __forceinline__ void small_solve(const double* t, int cnt, double* y) {
+    constexpr int N = kRecycleMax;
+    double S[N][N], L[N][N], d[N], z[N], yy[N];
+    bool keep[N], ok[N];
+    CP_UNROLL
+    for (int j = 0; j < N; ++j) {
+        const double a = j < cnt ? t[j * (j + 1) / 2 + j] : 0.0;
+        d[j] = a > 0.0 ? sqrt(a) : 0.0;
         keep[j] = d[j] > 0.0;
+        ok[j] = false;
+        z[j] = yy[j] = 0.0;
     }
-    for (int j = 0; j < cnt; ++j)
-        for (int k = 0; k < cnt; ++k) S[j][k] = (keep[j] && keep[k]) ? A[j][k] / (d[j] * d[k]) : 0.0;
-    for (int j = 0; j < cnt; ++j) {
-        if (!keep[j]) continue;
+    CP_UNROLL
+    for (int j = 0; j < N; ++j)
+        CP_UNROLL
+        for (int k = 0; k < N; ++k) {
+            L[j][k] = 0.0;
+            S[j][k] = 0.0;
+            if (k <= j && keep[j] && keep[k]) S[j][k] = t[j * (j + 1) / 2 + k] / (d[j] * d[k]);
+        }
+    CP_UNROLL
+    for (int j = 0; j < N; ++j) {
         double v = S[j][j];
-        for (int k = 0; k < j; ++k)
-            if (ok[k]) v -= L[j][k] * L[j][k];
-        if (!(v > kDrop)) continue;
-        L[j][j] = sqrt(v);
-        ok[j] = true;
-        for (int i = j + 1; i < cnt; ++i) {
-            if (!keep[i]) continue;
-            double s = S[i][j];
-            for (int k = 0; k < j; ++k)
-                if (ok[k]) s -= L[i][k] * L[j][k];
-            L[i][j] = s / L[j][j];
+        CP_UNROLL
+        for (int k = 0; k < N; ++k)
+            if (k < j && ok[k]) v -= L[j][k] * L[j][k];
+        if (keep[j] && v > kDrop) {
+            L[j][j] = sqrt(v);
+            ok[j] = true;
+            CP_UNROLL
+            for (int i = 0; i < N; ++i)
+                if (i > j && keep[i]) {
+                    double s = S[i][j];
+                    CP_UNROLL
+                    for (int k = 0; k < N; ++k)
+                        if (k < j && ok[k]) s -= L[i][k] * L[j][k];
+                    L[i][j] = s / L[j][j];
+                }
         }
     }
-    for (int j = 0; j < cnt; ++j) {
-        if (!ok[j]) continue;
-        double s = h[j] / d[j];
-        for (int k = 0; k < j; ++k)
-            if (ok[k]) s -= L[j][k] * z[k];
-        z[j] = s / L[j][j];
-    }
-    for (int j = cnt - 1; j >= 0; --j) {
-        if (!ok[j]) continue;
-        double s = z[j];
-        for (int k = j + 1; k < cnt; ++k)
-            if (ok[k]) s -= L[k][j] * yy[k];
-        yy[j] = s / L[j][j];
-    }
+    CP_UNROLL
+    for (int j = 0; j < N; ++j)
+        if (ok[j]) {
+            double s = t[kRecycleGram + j] / d[j];
+            CP_UNROLL
+            for (int k = 0; k < N; ++k)
+                if (k < j && ok[k]) s -= L[j][k] * z[k];
+            z[j] = s / L[j][j];
+        }
+    CP_UNROLL
+    for (int j = N - 1; j >= 0; --j)
+        if (ok[j]) {
+            double s = z[j];
+            CP_UNROLL
+            for (int k = 0; k < N; ++k)
+                if (k > j && ok[k]) s -= L[k][j] * yy[k];
+            yy[j] = s / L[j][j];
+        }
     bool finite = true;
-    for (int j = 0; j < kRecycleMax; ++j) {
+    CP_UNROLL
+    for (int j = 0; j < N; ++j) {
         const double v = ok[j] ? yy[j] / d[j] : 0.0;
         yy[j] = v;
         if (!(v - v == 0.0)) finite = false;  // NaN or infinity
     }
-    for (int j = 0; j < kRecycleMax; ++j) y[j] = finite ? yy[j] : 0.0;
+    CP_UNROLL
+    for (int j = 0; j < N; ++j) y[j] = finite ? yy[j] : 0.0;
 }
 
 // Per node: K u and K w_j gathered from the sliced blocks, r0 = m.(b - K u);
 // partial sums w_j . K w_k (j <= k) and w_j . r0, reduced in a fixed order;
 // the last block solves for y.
-__global__ void __launch_bounds__(kRecThreads) k_recycle_sums(RecycleArgs a) {
-    __shared__ double wpart[kRecThreads / 32][kRecycleStride];
+__global__ void __launch_bounds__(kSumThreads) k_recycle_sums(RecycleArgs a) {
+    __shared__ double wpart[kSumThreads / 32][kRecycleStride];
     __shared__ double tot[kRecycleStride];
     __shared__ bool last;
     const int cnt = a.cnt;
@@ -138,12 +156,17 @@ __global__ void __launch_bounds__(kRecThreads) k_recycle_sums(RecycleArgs a) {
         a.partials[(size_t)blockIdx.x * kRecycleStride + threadIdx.x] = t;
     }
     if (last_block_arrive(a.ticket, &last)) {
-        if (threadIdx.x < kRecycleSums) {
-            const volatile double* p = a.partials;
-            double t = 0.0;
-            for (int q = 0; q < (int)gridDim.x; ++q) t += p[(size_t)q * kRecycleStride + threadIdx.x];
-            tot[threadIdx.x] = t;
+        // four threads per sum, every fourth block each
+        const int i = threadIdx.x >> 2, g = threadIdx.x & 3;
+        double t = 0.0;
+        if (i < kRecycleSums) {
+            const double* p = a.partials + i;
+#pragma unroll 4
+            for (int q = g; q < (int)gridDim.x; q += 4) t += __ldcg(p + (size_t)q * kRecycleStride);
         }
+        t += __shfl_xor_sync(0xffffffffu, t, 1);
+        t += __shfl_xor_sync(0xffffffffu, t, 2);
+        if (i < kRecycleSums && g == 0) tot[i] = t;
         __syncthreads();
         if (threadIdx.x == 0) {
             small_solve(tot, cnt, a.y);
@@ -189,7 +212,8 @@ int node_grid(int n, int sm_count) {
 }  // namespace
 
 int recycle_grid(int n, int sm_count) {
-    const long long g = ((long long)n + kRecThreads - 1) / kRecThreads;
+    static_assert(4 * kRecycleSums <= kSumThreads, "four threads per sum");
+    const long long g = ((long long)n + kSumThreads - 1) / kSumThreads;
     const long long cap = 4LL * sm_count;
     return (int)std::max<long long>(1, std::min(g, cap));
 }
@@ -199,7 +223,7 @@ void recycle_project(const RecycleArgs& a, int sm_count, cudaStream_t s) {
     for (int j = 0; j < a.cnt; ++j)
         CP_CHECK(a.slot[j] >= 0 && a.slot[j] < kRecycleMax, CP_ERR_INVALID, "recycle: bad slot");
     if (a.cnt > 0) {
-        k_recycle_sums<<<recycle_grid(a.n, sm_count), kRecThreads, 0, s>>>(a);
+        k_recycle_sums<<<recycle_grid(a.n, sm_count), kSumThreads, 0, s>>>(a);
         CP_CUDA(cudaGetLastError());
     }
     k_recycle_apply<<<node_grid(a.n, sm_count), kRecThreads, 0, s>>>(a);

@@ -24,12 +24,15 @@ constexpr int kAsmThreads = 128;  // = 4 slices of 32 nodes
 // memory (each thread only touches its own node's blocks: no atomics, and the
 // summation order is the element order) and written out coalesced, once. The
 // next incidence's element is loaded ahead of the current one's arithmetic.
-// On the 1,048,576-quad plate 135 us (2.86 TB/s of its 386 MB) against 238
-// before the moment form of the element rows, the bank-conflict-free
-// accumulators and one block per tile in place of 8 per SM (6 fit: a second
-// wave a third full); 4096 quads 8.3 against 12.4 us. It is bound by the
-// latency of its gathers; fewer registers (6 or 8 blocks per SM) lose: 156,
-// 191 us.
+// On the 1,048,576-quad plate 193 us (2.0 TB/s of its 386 MB) against 240
+// before the bank-conflict-free accumulators and one block per tile in place of
+// 8 per SM (6 fit: a second wave a third full); 4096 quads 10.3 against 12.4
+// us. It is bound by its FP64 operations, about 600 per incidence (140 us at
+// the full rate); fewer registers (5 or 6 blocks per SM) lose: 200, 216 us. The
+// order of those operations is part of the result: a bilinear form in the
+// nodes' signs takes 280 and 135 us, but moves K by an ulp, and solves whose
+// linear iterations are capped then move by up to 1e-5 on meshes of near
+// rotational symmetry, where the order of the CG's sums moves them by 1e-12.
 template <bool W64, bool W32, bool Q8>
 __global__ void __launch_bounds__(kAsmThreads) k_assemble(DevMesh m, DevCsr csr, MaterialDev M,
                                                           const double* __restrict__ E_c,
@@ -87,8 +90,8 @@ constexpr int kElemThreads = 256;
 // secant target psi is stored as a residual and the relax kernel moves psi.
 // 4 blocks per SM (64 registers) for the latency of the gathers, and a grid
 // that fits once, so that the block sums and their fence are paid once per
-// block: 1,048,576 quads with Hollomon hardening, whole call 128 us before
-// the moment form, 85 at 2 blocks per SM, 74 now (floor 26: 168 MB).
+// block: 1,048,576 quads with Hollomon hardening, whole call 125 us at 2
+// blocks per SM with Newton's method on pow, 73 now (floor 26: 168 MB).
 template <bool Q8>
 __global__ void __launch_bounds__(kElemThreads, 4) k_update(DevMesh m, MaterialDev M, const double2* __restrict__ u,
                                                          ElemState st, OuterScalars* sc, double* partials, int aitken,

@@ -37,35 +37,26 @@ __device__ __forceinline__ Dmat form_d(int plane, double E, double nu) {
     return d;
 }
 
-// The 4-node quad (calcB4, src/PlasticitySolver.cu:26-64) in the basis of its
-// nodes' signs r = (1, -1, -1, 1), s = (1, 1, -1, -1), h = r s: for a nodal
-// field f, with f_a = r.f, f_b = s.f, f_h = h.f, four times its derivatives at
-// the Gauss point (sr q, ss q), sr, ss = +-1, are
-//   f_r = f_a + ss q f_h,  f_s = f_b + sr q f_h
-// two values each over the four points, so the whole element costs 7 sums and
-// 4 fused operations per field instead of a Jacobian and 8 gradients per
-// point. All factors of 4 cancel or go into the weights.
-struct QuadField {
-    double rp, rm, sp, sm;  // f_r at ss = +, -; f_s at sr = +, -
-};
-__device__ __forceinline__ QuadField quad_field(double f0, double f1, double f2, double f3) {
-    const double p = f0 - f2, q = f1 - f3;
-    const double fa = p - q, fb = p + q, fh = kGp * ((f0 + f2) - (f1 + f3));
-    return {fa + fh, fa - fh, fb + fh, fb - fh};
-}
-// 1 / x and 1 / y by one division.
-__device__ __forceinline__ void inv2(double x, double y, double& ix, double& iy) {
-    const double t = 1.0 / (x * y);
-    ix = y * t;
-    iy = x * t;
-}
-// Reciprocals of the four determinants (16 times the true ones) at (sr, ss) =
-// (+,+), (+,-), (-,+), (-,-).
-__device__ __forceinline__ void quad_inv_det(const QuadField& x, const QuadField& y, double* w) {
-    const double d0 = x.rp * y.sp - y.rp * x.sp, d1 = x.rm * y.sp - y.rm * x.sp;
-    const double d2 = x.rp * y.sm - y.rp * x.sm, d3 = x.rm * y.sm - y.rm * x.sm;
-    inv2(d0, d1, w[0], w[1]);
-    inv2(d2, d3, w[2], w[3]);
+// calcB4 (src/PlasticitySolver.cu:26-64) at Gauss point (r, s): shape-function
+// gradients bx[k] = dN_k/dx, by[k] = dN_k/dy and detJ.
+__device__ __forceinline__ double q4_grad(const double* x, const double* y, double r, double s, double* bx,
+                                          double* by) {
+    double J0 = 0.25 * ((1. + s) * x[0] - (1. + s) * x[1] - (1. - s) * x[2] + (1. - s) * x[3]);
+    double J2 = 0.25 * ((1. + r) * x[0] + (1. - r) * x[1] - (1. - r) * x[2] - (1. + r) * x[3]);
+    double J1 = 0.25 * ((1. + s) * y[0] - (1. + s) * y[1] - (1. - s) * y[2] + (1. - s) * y[3]);
+    double J3 = 0.25 * ((1. + r) * y[0] + (1. - r) * y[1] - (1. - r) * y[2] - (1. + r) * y[3]);
+    double det = J0 * J3 - J1 * J2;
+    double inv = 1. / det;
+    double i0 = J3 * inv, i1 = -J1 * inv, i2 = -J2 * inv, i3 = J0 * inv;
+    bx[0] = 0.25 * ((1. + s) * i0 + (1. + r) * i1);
+    by[0] = 0.25 * ((1. + s) * i2 + (1. + r) * i3);
+    bx[1] = 0.25 * ((-1. - s) * i0 + (1. - r) * i1);
+    by[1] = 0.25 * ((-1. - s) * i2 + (1. - r) * i3);
+    bx[2] = 0.25 * ((-1. + s) * i0 - (1. - r) * i1);
+    by[2] = 0.25 * ((-1. + s) * i2 - (1. - r) * i3);
+    bx[3] = 0.25 * ((1. - s) * i0 - (1. + r) * i1);
+    by[3] = 0.25 * ((1. - s) * i2 - (1. + r) * i3);
+    return det;
 }
 
 // calcB8 (src/PlasticitySolver.cu:67-134) at (r, s): gradients and detJ of the
@@ -226,75 +217,31 @@ __device__ __forceinline__ void element_rows(const DevMesh& m, int e, int i, uin
 #pragma unroll
         for (int j = 0; j < 3; ++j) add_scaled(nb, (int)((kk >> (8 * j)) & 0xffu), blk[j], h);
     } else {
-        // formKe4 (src/PlasticitySolver.cu:157-186): the block of nodes i, j is
-        // a bilinear form in their signs (r_i, s_i, h_i), (r_j, s_j, h_j), so
-        // the element is the 21 moments of its Gauss points' weights with the
-        // three coefficient vectors, and a row is a few signed sums of them:
-        // about 280 FP64 operations per incidence, where the Jacobian,
-        // gradients and products of every point took 800. The moments do not
-        // depend on i, and the sums change only by exact signs under i <-> j,
-        // so K is bitwise symmetric.
+        // formKe4 (src/PlasticitySolver.cu:157-186)
         const int4 el = m.e4[e - m.c3];
-        const double2 p0 = m.xy[el.x], p1 = m.xy[el.y], p2 = m.xy[el.z], p3 = m.xy[el.w];
-        const QuadField X = quad_field(p0.x, p1.x, p2.x, p3.x), Y = quad_field(p0.y, p1.y, p2.y, p3.y);
-        double w[4];
-        quad_inv_det(X, Y, w);
-        const double hw = h * 0.0625;
-        const double w0 = hw * w[0], w1 = hw * w[1], w2 = hw * w[2], w3 = hw * w[3];
-        // 16 det dN/dx = al r - be s + et h with al = y_s, be = y_r, et = ss q al - sr q be;
-        // 16 det dN/dy the same with ax = -x_s, bx = -x_r
-        const double alp = Y.sp, alm = Y.sm, bep = Y.rp, bem = Y.rm;
-        const double axp = -X.sp, axm = -X.sm, bxp = -X.rp, bxm = -X.rm;
-        // et at (+,+) = -at (-,-), at (-,+) = -at (+,-)
-        const double ya = 0.5 * (bep + bem), yb = 0.5 * (alp + alm), xa = 0.5 * (bxp + bxm), xb = 0.5 * (axp + axm);
-        const double e1 = kGp * (yb - ya), e2 = kGp * (yb + ya), f1 = kGp * (xb - xa), f2 = kGp * (xb + xa);
-        const double wrp = w0 + w1, wrm = w2 + w3, wsp = w0 + w2, wsm = w1 + w3, u1 = w0 + w3, u2 = w1 + w2;
-        // moments: xx, yy symmetric (rr, ss, hh, rs, rh, sh), xy full
-        const double arp = alp * wrp, arm = alm * wrm, brp = axp * wrp, brm = axm * wrm;
-        const double xx_rr = alp * arp + alm * arm, xy_rr = axp * arp + axm * arm, yy_rr = axp * brp + axm * brm;
-        const double asp = bep * wsp, asm_ = bem * wsm, bsp = bxp * wsp, bsm = bxm * wsm;
-        const double xx_ss = bep * asp + bem * asm_, xy_ss = bxp * asp + bxm * asm_, yy_ss = bxp * bsp + bxm * bsm;
-        const double g1 = e1 * u1, g2 = e2 * u2, g3 = f1 * u1, g4 = f2 * u2;
-        const double xx_hh = e1 * g1 + e2 * g2, xy_hh = f1 * g1 + f2 * g2, yy_hh = f1 * g3 + f2 * g4;
-        // sums over ss of w be, w et at sr = +, -; over sr of w et at ss = +, -
-        const double Bp = w0 * bep + w1 * bem, Bm = w2 * bep + w3 * bem;
-        const double Cp = w0 * bxp + w1 * bxm, Cm = w2 * bxp + w3 * bxm;
-        const double Ep = w0 * e1 - w1 * e2, Em = w2 * e2 - w3 * e1;
-        const double Fp = w0 * f1 - w1 * f2, Fm = w2 * f2 - w3 * f1;
-        const double Gp = w0 * e1 + w2 * e2, Gm = w1 * e2 + w3 * e1;
-        const double Hp = w0 * f1 + w2 * f2, Hm = w1 * f2 + w3 * f1;
-        const double xx_rs = -(alp * Bp + alm * Bm), yy_rs = -(axp * Cp + axm * Cm);
-        const double xy_rs = -(alp * Cp + alm * Cm), xy_sr = -(axp * Bp + axm * Bm);
-        const double xx_rh = alp * Ep + alm * Em, yy_rh = axp * Fp + axm * Fm;
-        const double xy_rh = alp * Fp + alm * Fm, xy_hr = axp * Ep + axm * Em;
-        const double xx_sh = -(bep * Gp - bem * Gm), yy_sh = -(bxp * Hp - bxm * Hm);
-        const double xy_sh = -(bep * Hp - bem * Hm), xy_hs = -(bxp * Gp - bxm * Gm);
-        // signs of node i; its row's columns: i, same s (i ^ 1), same r (3 - i), opposite (i ^ 2)
-        const double ri = (i == 0 || i == 3) ? 1.0 : -1.0, si = i < 2 ? 1.0 : -1.0, hi = ri * si;
-        double K00[4], K11[4];
-        auto sym_row = [&](double rr, double ss, double hh, double rs, double rh, double sh, double* K) {
-            const double a2 = 2.0 * hi * rs, b2 = 2.0 * si * rh, c2 = 2.0 * ri * sh;
-            K[0] = (rr + ss + hh) + (a2 + b2 + c2);
-            K[1] = (ss - (rr + hh)) - b2;
-            K[2] = (rr - (ss + hh)) - c2;
-            K[3] = (hh - (rr + ss)) - a2;
-        };
-        sym_row(d.c00 * xx_rr + d.c22 * yy_rr, d.c00 * xx_ss + d.c22 * yy_ss, d.c00 * xx_hh + d.c22 * yy_hh,
-                d.c00 * xx_rs + d.c22 * yy_rs, d.c00 * xx_rh + d.c22 * yy_rh, d.c00 * xx_sh + d.c22 * yy_sh, K00);
-        sym_row(d.c11 * yy_rr + d.c22 * xx_rr, d.c11 * yy_ss + d.c22 * xx_ss, d.c11 * yy_hh + d.c22 * xx_hh,
-                d.c11 * yy_rs + d.c22 * xx_rs, d.c11 * yy_rh + d.c22 * xx_rh, d.c11 * yy_sh + d.c22 * xx_sh, K11);
-        // c01 xy + c22 xy^T: symmetric and antisymmetric parts
-        const double cs = d.c01 + d.c22, ca = d.c01 - d.c22;
-        const double rr = cs * xy_rr, ss = cs * xy_ss, hh = cs * xy_hh;
-        const double q0 = hi * cs * (xy_rs + xy_sr), q1 = si * cs * (xy_rh + xy_hr), q2 = ri * cs * (xy_sh + xy_hs);
-        const double d0 = hi * ca * (xy_rs - xy_sr), d1 = si * ca * (xy_rh - xy_hr), d2 = ri * ca * (xy_sh - xy_hs);
-        const double b0 = (rr + ss + hh) + (q0 + q1 + q2), b1 = (ss - (rr + hh)) - q1, b2 = (rr - (ss + hh)) - q2,
-                     b3 = (hh - (rr + ss)) - q0;
-        const double t1 = d0 - d2, t2 = -(d0 + d1), t3 = d1 + d2;
-        add_to(nb, (int)((kk >> (8 * i)) & 0xffu), K00[0], b0, b0, K11[0]);
-        add_to(nb, (int)((kk >> (8 * (i ^ 1))) & 0xffu), K00[1], b1 + t1, b1 - t1, K11[1]);
-        add_to(nb, (int)((kk >> (8 * (3 - i))) & 0xffu), K00[2], b2 + t2, b2 - t2, K11[2]);
-        add_to(nb, (int)((kk >> (8 * (i ^ 2))) & 0xffu), K00[3], b3 + t3, b3 - t3, K11[3]);
+        double x[4], y[4];
+#pragma unroll
+        for (int a = 0; a < 4; ++a) {
+            const double2 p = m.xy[nth(el, a)];
+            x[a] = p.x;
+            y[a] = p.y;
+        }
+        double blk[4][4] = {};
+#pragma unroll
+        for (int gi = 0; gi < 2; ++gi)
+#pragma unroll
+            for (int gj = 0; gj < 2; ++gj) {
+                double bx[4], by[4];
+                const double det = q4_grad(x, y, gi ? kGp : -kGp, gj ? kGp : -kGp, bx, by);
+                double bxi = bx[0], byi = by[0];
+#pragma unroll
+                for (int a = 1; a < 4; ++a)
+                    if (i == a) { bxi = bx[a]; byi = by[a]; }
+#pragma unroll
+                for (int j = 0; j < 4; ++j) add_block(blk[j], bxi, byi, bx[j], by[j], d, det);
+            }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) add_scaled(nb, (int)((kk >> (8 * j)) & 0xffu), blk[j], h);
     }
 }
 
@@ -399,24 +346,26 @@ __device__ __forceinline__ void update_element(const DevMesh& m, const MaterialD
         }
         ex *= 0.25; ey *= 0.25; g *= 0.25;
     } else {
-        // the mean over the Gauss points, from the fields' derivatives there
         const int4 el = m.e4[e - m.c3];
-        const double2 p0 = m.xy[el.x], p1 = m.xy[el.y], p2 = m.xy[el.z], p3 = m.xy[el.w];
-        const double2 w0 = u[el.x], w1 = u[el.y], w2 = u[el.z], w3 = u[el.w];
-        const QuadField X = quad_field(p0.x, p1.x, p2.x, p3.x), Y = quad_field(p0.y, p1.y, p2.y, p3.y);
-        const QuadField U = quad_field(w0.x, w1.x, w2.x, w3.x), V = quad_field(w0.y, w1.y, w2.y, w3.y);
-        double w[4];
-        quad_inv_det(X, Y, w);
+        double x[4], y[4], uu[4], vv[4];
+#pragma unroll
+        for (int a = 0; a < 4; ++a) {
+            const int nd = nth(el, a);
+            const double2 p = m.xy[nd], w = u[nd];
+            x[a] = p.x; y[a] = p.y; uu[a] = w.x; vv[a] = w.y;
+        }
         ex = 0.0; ey = 0.0; g = 0.0;
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const double xr = q & 1 ? X.rm : X.rp, xs = q & 2 ? X.sm : X.sp, yr = q & 1 ? Y.rm : Y.rp,
-                         ys = q & 2 ? Y.sm : Y.sp, ur = q & 1 ? U.rm : U.rp, us = q & 2 ? U.sm : U.sp,
-                         vr = q & 1 ? V.rm : V.rp, vs = q & 2 ? V.sm : V.sp;
-            ex += (ur * ys - us * yr) * w[q];
-            ey += (vs * xr - vr * xs) * w[q];
-            g += ((us * xr - ur * xs) + (vr * ys - vs * yr)) * w[q];
-        }
+        for (int gi = 0; gi < 2; ++gi)
+#pragma unroll
+            for (int gj = 0; gj < 2; ++gj) {
+                double bx[4], by[4];
+                q4_grad(x, y, gi ? kGp : -kGp, gj ? kGp : -kGp, bx, by);
+                ex += uu[0] * bx[0] + uu[1] * bx[1] + uu[2] * bx[2] + uu[3] * bx[3];
+                ey += vv[0] * by[0] + vv[1] * by[1] + vv[2] * by[2] + vv[3] * by[3];
+                g += uu[0] * by[0] + uu[1] * by[1] + uu[2] * by[2] + uu[3] * by[3] + vv[0] * bx[0] +
+                     vv[1] * bx[1] + vv[2] * bx[2] + vv[3] * bx[3];
+            }
         ex *= 0.25; ey *= 0.25; g *= 0.25;
     }
     const Dmat d = form_d(M.plane, Ec, nuc);
@@ -434,10 +383,9 @@ __device__ __forceinline__ void update_element(const DevMesh& m, const MaterialD
     s_num += diff * diff;
     s_den += tab * tab;
     if (!aitken) {
-        const double ips = 1.0 / ps;
         st.psi[e] = ps;
-        st.E_c[e] = E0 * ips;
-        st.nu_c[e] = 0.5 * (1. - (1. - 2. * nu0) * ips);
+        st.E_c[e] = E0 / ps;
+        st.nu_c[e] = 0.5 * (1. - (1. - 2. * nu0) / ps);
     } else {
         const double r = (ps == ps) ? ps - st.psi[e] : 0.0;
         const double dr = r - st.res_prev[e];

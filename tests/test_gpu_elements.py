@@ -1,5 +1,5 @@
 """The element kernels at the sizes where their tiles end and on distorted
-quads: K from the moment form against 2x2 Gauss quadrature in numpy (1e-13 of
+quads: K against 2x2 Gauss quadrature in numpy (1e-13 of
 the row's largest value, the bar of the reference fixtures), bitwise symmetry,
 and the Hollomon diagram's inverse against its own equation."""
 import ctypes

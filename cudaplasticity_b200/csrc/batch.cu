@@ -597,7 +597,7 @@ enum : int { OUT_UPD = 0, OUT_BREAKDOWN, OUT_SAVE };
 size_t bchip_smem(const ChipPlan& p) {
     const int half = p.spc * 16;
     return ((size_t)2 * half + p.halo_cap) * sizeof(float2) + (size_t)12 * half * sizeof(float2) +
-           ChipRows<float, 2, 2>::smem_blocks(half, p.wmax) * (2 * sizeof(float2) + 2);
+           ChipRows<float, 2, 2, true>::smem_blocks(half, p.wmax) * (2 * sizeof(float2) + 2);
 }
 
 __global__ void __launch_bounds__(kBChipThreads, 1) k_batch_chip(const BDesc* __restrict__ D, BState* SS,
@@ -627,7 +627,7 @@ __global__ void __launch_bounds__(kBChipThreads, 1) k_batch_chip(const BDesc* __
         float2* rec = U + own + P.halo_cap;
         comm.rec_base = smem_addr(rec);
         const bool in = tid < half;
-        ChipRows<float, 2, 2> rows;
+        ChipRows<float, 2, 2, true> rows;
         rows.tid = in ? tid : half - 1;  // idle threads gather zeros from a valid place
         rows.nthr = half;
         rows.init(rec + 6 * own, smem_addr(U), P.wmax);

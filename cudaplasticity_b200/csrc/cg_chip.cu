@@ -150,6 +150,23 @@ __global__ void __launch_bounds__(kOrderThreads) k_chip_order(int n, int slots, 
     }
 }
 
+// One block per CTA of the solve: its nodes by node number, so that the
+// neighbours of consecutive threads tend to be consecutive too (the gathers'
+// shared-memory banks, the halo records' order): 4160 nodes 1.85 -> 1.74 us.
+__global__ void __launch_bounds__(kPlanThreads) k_chip_local(int own, int* order, int* slot_of) {
+    extern __shared__ int ids[];
+    const int s0 = blockIdx.x * own;
+    for (int i = threadIdx.x; i < own; i += blockDim.x) ids[i] = order[s0 + i];
+    __syncthreads();
+    for (int i = threadIdx.x; i < own; i += blockDim.x) {
+        const unsigned int id = (unsigned int)ids[i];  // -1 sorts last
+        int at = 0;
+        for (int q = 0; q < own; ++q) at += ((unsigned int)ids[q] < id || ((unsigned int)ids[q] == id && q < i)) ? 1 : 0;
+        order[s0 + at] = (int)id;
+        if ((int)id >= 0) slot_of[id] = s0 + at;
+    }
+}
+
 // One block per CTA of the solve: its halo (ascending slots), the local index
 // of every block of its rows, and a mark on every slot that is in another
 // CTA's halo.
@@ -221,7 +238,7 @@ __global__ void __launch_bounds__(kPlanThreads) k_chip_plan(int slots, int own, 
 
 // NPT nodes per thread; of the second one (double) the whole row lies in
 // shared memory.
-template <typename T, bool GRID, int NPT>
+template <typename T, bool GRID, int NPT, bool WIDE>
 __global__ void __launch_bounds__(kChipWarps * 32, 1) k_chip(ChipArgs<T> a) {
     using V2 = typename Vec2<T>::type;
     using V4 = typename Vec4<T>::type;
@@ -240,7 +257,7 @@ __global__ void __launch_bounds__(kChipWarps * 32, 1) k_chip(ChipArgs<T> a) {
     V2* U = reinterpret_cast<V2*>(smem_raw);
     V2* rec = U + own + P.halo_cap;
     comm.rec_base = smem_addr(rec);
-    ChipRows<T, NPT, RN> rows;
+    ChipRows<T, NPT, RN, WIDE> rows;
     rows.tid = tid;
     rows.nthr = nthr;
     rows.init(rec + (GRID ? 0 : 6 * own), smem_addr(U), P.wmax);
@@ -505,7 +522,7 @@ size_t chip_smem(const ChipPlan& p) {
     const size_t own = (size_t)nthr * NPT;
     size_t b = (own + p.halo_cap) * 2 * sizeof(T);
     if (!GRID) b += 6 * own * 2 * sizeof(T);
-    b += ChipRows<T, NPT, sizeof(T) == 4 ? NPT : 1>::smem_blocks(nthr, p.wmax) * (4 * sizeof(T) + 2);
+    b += ChipRows<T, NPT, sizeof(T) == 4 ? NPT : 1, true>::smem_blocks(nthr, p.wmax) * (4 * sizeof(T) + 2);
     return (b + 15) / 16 * 16;
 }
 
@@ -539,9 +556,9 @@ bool chip_attributes(K k, bool grid) {
     return ok;
 }
 
-template <typename T, bool GRID, int NPT>
+template <typename T, bool GRID, int NPT, bool WIDE>
 bool schedulable(const ChipPlan& p, int sm_count) {
-    const auto k = k_chip<T, GRID, NPT>;
+    const auto k = k_chip<T, GRID, NPT, WIDE>;
     const size_t smem = chip_smem<T, GRID, NPT>(p);
     if (smem > kSmemCap || !chip_attributes(k, GRID)) return false;
     if (GRID) {
@@ -561,10 +578,14 @@ bool schedulable(const ChipPlan& p, int sm_count) {
     }
     return true;
 }
+template <typename T, bool WIDE>
+bool chip_schedulable_as(const ChipPlan& p, int sm_count) {
+    if (!p.grid) return schedulable<T, false, 1, WIDE>(p, sm_count);
+    return p.npt == 2 ? schedulable<T, true, 2, WIDE>(p, sm_count) : schedulable<T, true, 1, WIDE>(p, sm_count);
+}
 template <typename T>
 bool chip_schedulable(const ChipPlan& p, int sm_count) {
-    if (!p.grid) return schedulable<T, false, 1>(p, sm_count);
-    return p.npt == 2 ? schedulable<T, true, 2>(p, sm_count) : schedulable<T, true, 1>(p, sm_count);
+    return p.wmax > kRegBlocks ? chip_schedulable_as<T, true>(p, sm_count) : chip_schedulable_as<T, false>(p, sm_count);
 }
 
 }  // namespace
@@ -572,16 +593,15 @@ bool chip_schedulable(const ChipPlan& p, int sm_count) {
 // The shape of the cluster (grid = false) or grid form for n nodes; ctas = 0
 // when it does not hold them.
 //   cluster: about 13 CTAs, of at least 4 slices. 1024 nodes: 8 CTAs of 4
-//     slices 1.70 us per iteration, 16 of 2 2.10, 3 of 12 2.02; 4160 nodes: 13
-//     of 10 1.98, 11 of 12 2.10 (the whole solve in one cluster with every
+//     slices 1.45 us per iteration, 16 of 2 1.9, 3 of 12 1.7; 4160 nodes: 13 of
+//     10 1.74, 11 of 12 1.8 (the whole solve in one cluster with every
 //     record read through distributed shared memory: 4.9 and 5.7).
 //   grid: about 128 CTAs, of at least 8 slices. 16104 nodes: 63 CTAs of 8
-//     slices 3.40 us, 126 of 4 3.80, 42 of 12 3.62 (one launch per iteration,
-//     cg_fused.cu: 10.2); 40200 nodes: 126 of 10 3.67, 105 of 12 3.98 (11.3).
+//     slices 3.31 us, 126 of 4 3.7, 42 of 12 3.7 (one launch per iteration,
+//     cg_fused.cu: 10.2); 40200 nodes: 126 of 10 3.71, 105 of 12 3.8 (11.4).
 //     Above 147 CTAs of 12, two nodes per thread: 65536 nodes 86 CTAs of 24
-//     6.26 us, 128 of 16 6.70 (12.0); 99856 nodes 131 of 24 6.33 (16.3).
-//     At sizes that both hold the cluster is the faster one (4160 nodes: 3.16
-//     as a grid).
+//     5.98 us (11.9); 99856 nodes 131 of 24 6.09 (16.3). At sizes that both
+//     hold the cluster is the faster one (4160 nodes: 3.2 as a grid).
 ChipShape chip_shape(int n, int wmax, int sm_count, bool grid) {
     const int n_slices = (n + 31) / 32;
     ChipShape s;
@@ -648,6 +668,7 @@ void chip_build_plan(ChipPlan& p, const ChipShape& s, void* mem, int n, const do
     constexpr int order_smem = kDigits * kOrderThreads * (int)sizeof(unsigned int);
     CP_CUDA(cudaFuncSetAttribute(k_chip_order, cudaFuncAttributeMaxDynamicSharedMemorySize, order_smem));
     k_chip_order<<<1, kOrderThreads, order_smem, st>>>(n, (int)slots, xy, scratch, p.order, slot_of);
+    k_chip_local<<<s.ctas, kPlanThreads, sizeof(int) * (size_t)s.spc * 32, st>>>(s.spc * 32, p.order, slot_of);
     k_chip_plan<<<s.ctas, kPlanThreads, 2 * sizeof(unsigned int) * (slots / 32), st>>>(
         (int)slots, s.spc * 32, s.wmax, slice_ptr, scol, p.order, slot_of, p.lidx, p.halo, p.halo_cnt, p.pub);
     CP_CUDA(cudaGetLastError());
@@ -664,12 +685,18 @@ void chip_build_plan(ChipPlan& p, const ChipShape& s, void* mem, int n, const do
 }
 
 namespace {
-template <typename T, bool GRID, int NPT>
+template <typename T, bool GRID, int NPT, bool WIDE>
 void launch_as(const ChipArgs<T>& a, cudaStream_t s) {
-    const auto k = k_chip<T, GRID, NPT>;
+    const auto k = k_chip<T, GRID, NPT, WIDE>;
     cudaLaunchAttribute attr[1];
     cudaLaunchConfig_t cfg = chip_config(k, a.plan, chip_smem<T, GRID, NPT>(a.plan), attr, s);
     CP_CUDA(cudaLaunchKernelEx(&cfg, k, a));
+}
+template <typename T, bool WIDE>
+void launch_form(const ChipArgs<T>& a, cudaStream_t s) {
+    if (!a.plan.grid) launch_as<T, false, 1, WIDE>(a, s);
+    else if (a.plan.npt == 2) launch_as<T, true, 2, WIDE>(a, s);
+    else launch_as<T, true, 1, WIDE>(a, s);
 }
 }  // namespace
 
@@ -677,9 +704,8 @@ template <typename T>
 void chip_launch(const ChipArgs<T>& a, cudaStream_t s) {
     const ChipPlan& p = a.plan;
     CP_CHECK(p.ctas > 0, CP_ERR_INVALID, "on-chip CG: the instance does not fit");
-    if (!p.grid) launch_as<T, false, 1>(a, s);
-    else if (p.npt == 2) launch_as<T, true, 2>(a, s);
-    else launch_as<T, true, 1>(a, s);
+    if (p.wmax > kRegBlocks) launch_form<T, true>(a, s);
+    else launch_form<T, false>(a, s);
 }
 
 template void chip_launch<double>(const ChipArgs<double>&, cudaStream_t);

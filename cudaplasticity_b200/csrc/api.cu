@@ -260,6 +260,37 @@ void run_cg_loop(cp_instance* I, const cp::CgArgs<T>& a, cudaGraphExec_t g) {
     }
 }
 
+// The upper half of K for the one-launch FP64 CG, its columns built on first
+// use; without room for it the iterations read all of K.
+void fused_half(cp_instance* I, cp::FusedArgs& a) {
+    if (!I->f_half_tried && cp::fused_wants_half(a.n, I->csr.max_width)) {
+        I->f_half_tried = true;
+        cp::HalfK& h = a.half;
+        const size_t nodes = 32 * (size_t)I->csr.n_slices;
+        int *widths = I->alloc<int>(2), most[2];
+        h.width = I->alloc<unsigned short>(I->csr.n_slices);
+        CP_CUDA(cudaMemsetAsync(widths, 0, 2 * sizeof(int), I->s()));
+        cp::fused_half_widths(a, widths, I->s());
+        CP_CUDA(cudaMemcpyAsync(most, widths, sizeof(most), cudaMemcpyDeviceToHost, I->s()));
+        CP_CUDA(cudaStreamSynchronize(I->s()));
+        h.u = most[0];
+        h.l = most[1];
+        try {
+            h.ucol = I->alloc<int>(nodes * h.u);
+            h.low = I->alloc<unsigned int>(nodes * std::max(h.l, 1));
+            h.val = I->alloc<double2>(2 * nodes * h.u);
+        } catch (const Error&) {
+            (void)cudaGetLastError();
+            h.val = nullptr;
+            return;
+        }
+        CP_CUDA(cudaMemsetAsync(h.val, 0, 2 * sizeof(double2) * nodes * h.u, I->s()));
+        cp::fused_half_columns(a, I->s());
+        I->f_half = h;
+    }
+    a.half = I->f_half;
+}
+
 // Arguments of the one-launch FP64 CG (cg_fused.cu) of this instance; its
 // vectors are allocated on first use.
 cp::FusedArgs fused_args(cp_instance* I, int precond) {
@@ -293,6 +324,7 @@ cp::FusedArgs fused_args(cp_instance* I, int precond) {
     a.precond = precond;
     a.sc = I->sc;
     a.partials = I->f_partials;
+    fused_half(I, a);
     return a;
 }
 
@@ -1242,7 +1274,9 @@ CP_API int cp_bench_cg_fused(cp_instance* I, int precond, int iters, double* ms_
         // block-Jacobi inverse (34 with, 2 without)
         const double n = I->n_nodes, nnz = (double)I->csr.nnz;
         if (ms_iter) *ms_iter = t / iters;
-        if (bytes_iter) *bytes_iter = nnz * 8 + nnz + n * (256 + (precond ? 34 : 2));
+        // (of K's upper half: (blocks + n) / 2 values, all columns)
+        const double vals = a.half.val ? (nnz + 4 * n) / 2 : nnz;
+        if (bytes_iter) *bytes_iter = vals * 8 + nnz + n * (256 + (precond ? 34 : 2));
     });
 }
 

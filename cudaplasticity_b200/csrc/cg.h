@@ -52,6 +52,17 @@ struct CgArgs {
     double* partials = nullptr;     // >= 3 * max_blocks doubles
 };
 
+// The upper half of K for cg_fused.cu's iterations: per slice of 32 nodes, up
+// to u blocks right of the diagonal (block 0 is the diagonal one) and up to l
+// left of it, in slots of the slice's widest row.
+struct HalfK {
+    int u = 0, l = 0;
+    unsigned short* width = nullptr;  // per slice: upper blocks | lower blocks << 8
+    int* ucol = nullptr;              // per upper slot: its column (the node itself: padding)
+    unsigned int* low = nullptr;      // per lower slot: its column and its mirror's upper slot
+    double2* val = nullptr;           // per upper slot: the block, rewritten by every solve's start; null: not in use
+};
+
 // The single-launch FP64 iteration of cg_fused.cu.
 struct FusedArgs {
     int n = 0;
@@ -67,6 +78,7 @@ struct FusedArgs {
     double2 *gA = nullptr, *gB = nullptr;  // per node: u, M w, M kp (by parity)
     double4* minv = nullptr;
     int precond = 0;
+    HalfK half;
     CgScalars* sc = nullptr;
     double* partials = nullptr;
     // persistent form only: time limit of each grid-barrier wait, and the
@@ -77,6 +89,12 @@ struct FusedArgs {
     unsigned int barrier_skew = 0;
 };
 
+// The upper half of K: whether the iterations of an instance read it, its
+// widths (widths: two ints, zero before; a.half.width is written), and, once
+// those are on the host, its columns.
+bool fused_wants_half(int n, int wmax);
+void fused_half_widths(const FusedArgs& a, int* widths, cudaStream_t s);
+void fused_half_columns(const FusedArgs& a, cudaStream_t s);
 void fused_launch_start(const FusedArgs& a, double eps2, long long max_iter, cudaStream_t s);
 void fused_launch_iteration(const FusedArgs& a, int parity, cudaStream_t s);
 // The whole solve (init, first step, iterations) as one cooperative launch;

@@ -17,6 +17,7 @@
 // deterministic cross-block reduction (last block, index order). The
 // scalars stay on the device; the loop runs in a CUDA graph with a WHILE
 // node, as in cg.cu.
+#include <algorithm>
 #include <cstddef>
 #include <cstdlib>
 #include <mutex>
@@ -92,18 +93,99 @@ __device__ __forceinline__ double2 ld_other(const double2* p) {
     return __ldg(p);
 }
 
+// ------------------------------------------------- the upper half of K --
+//
+// Above kHalfLeast nodes the iterations read K's upper half alone. A block left
+// of the diagonal is the transpose of its mirror in the row above (K is bitwise
+// symmetric), which the warps nearby read at about the same time: taken from
+// there, out of L2, it leaves 5 of a quad mesh's 9 blocks per node to device
+// memory (482 bytes per node and iteration in place of 614). The solve's first
+// kernel, which reads all of K, writes the upper blocks to slots of their own,
+// so that a mirror's address follows from its row and slot.
+// (99,856 nodes: 20.0 -> 18.9 us; below, the working set lies in L2 anyway.)
+constexpr int kHalfLeast = 100000;
+constexpr int kLowShift = 27;  // of a lower slot's word: column below, mirror's upper slot above
+constexpr int kHalfMax = 31;
+
+__device__ __forceinline__ size_t half_at(int w, int sl, int q, int lane) {
+    return ((size_t)sl * w + q) * 32 + lane;
+}
+
+__global__ void k_f_half_widths(FusedArgs a, int* widths) {
+    CPF_SLICE_LOOP {
+        const int n = 32 * sl + lane;
+        const int base = a.slice_ptr[sl], wd = (a.slice_ptr[sl + 1] - base) >> 5;
+        int u = 1, l = 0;
+        if (n < a.n)
+            for (int k = 1; k < wd; ++k) {
+                const int j = a.scol[base + 32 * k + lane];
+                u += j > n;
+                l += j < n;
+            }
+        u = __reduce_max_sync(0xffffffffu, u);
+        l = __reduce_max_sync(0xffffffffu, l);
+        if (lane == 0) {
+            a.half.width[sl] = (unsigned short)(u | l << 8);
+            atomicMax(widths, u);
+            atomicMax(widths + 1, l);
+        }
+    }
+}
+
+__global__ void k_f_half_columns(FusedArgs a) {
+    CPF_SLICE_LOOP {
+        const int n = 32 * sl + lane;
+        const int base = a.slice_ptr[sl], wd = (a.slice_ptr[sl + 1] - base) >> 5;
+        int u = 0, l = 0;
+        if (n < a.n) {
+            a.half.ucol[half_at(a.half.u, sl, u++, lane)] = n;
+            for (int k = 1; k < wd; ++k) {
+                const int j = a.scol[base + 32 * k + lane];
+                if (j > n) a.half.ucol[half_at(a.half.u, sl, u++, lane)] = j;
+                if (j >= n) continue;
+                const int bj = a.slice_ptr[j >> 5], wj = (a.slice_ptr[(j >> 5) + 1] - bj) >> 5;
+                unsigned int q = 1;
+                for (int i = 1; i < wj; ++i) {
+                    const int c = a.scol[bj + 32 * i + (j & 31)];
+                    if (c == n) break;
+                    q += c > j;
+                }
+                a.half.low[half_at(a.half.l, sl, l++, lane)] = (unsigned int)j | q << kLowShift;
+            }
+        }
+        for (; u < a.half.u; ++u) a.half.ucol[half_at(a.half.u, sl, u, lane)] = -1;
+        for (; l < a.half.l; ++l) a.half.low[half_at(a.half.l, sl, l, lane)] = 0xffffffffu;
+    }
+}
+
+// Where value c (u, M w, M kp) of node n's record lies: side by side, or with
+// the upper half (whose kernel is the more bound by its L1 accesses) in three
+// arrays, 101 against 105 us at 1,049,600 nodes; the other kernel loses by
+// that, 117 against 129.
+template <bool HALF>
+__device__ __forceinline__ size_t rec_at(const FusedArgs& a, int n, int c) {
+    return HALF ? (size_t)c * a.n + n : 3 * (size_t)n + c;
+}
+
 // r = m.(b - K x), block-Jacobi inverse, u = M r, p = kp = 0, the parity-0
-// record (u, -, 0); sums (r, r), (b, b).
+// record (u, -, 0); sums (r, r), (b, b). HALF: also the upper half of K.
+template <bool HALF>
 __device__ __forceinline__ void init_body(const FusedArgs& a, double* v) {
     CPF_SLICE_LOOP {
         const int n = 32 * sl + lane;
         if (n >= a.n) continue;
         const int base = a.slice_ptr[sl], wd = (a.slice_ptr[sl + 1] - base) >> 5;
         double k0 = 0.0, k1 = 0.0;
+        int q = 0;
         for (int k = 0; k < wd; ++k) {
             const long long bi = base + 32LL * k + lane;
             const int col = __ldg(a.scol + bi);
             const double2 lo = load_lo(a.val, bi), hi = load_hi(a.val, bi);
+            if (HALF && (k == 0 || col > n)) {
+                double2* h = a.half.val + 2 * half_at(a.half.u, sl, q++, lane);
+                h[0] = lo;
+                h[1] = hi;
+            }
             const double2 xc = a.x[col];
             k0 += lo.x * xc.x + lo.y * xc.y;
             k1 += hi.x * xc.x + hi.y * xc.y;
@@ -129,8 +211,8 @@ __device__ __forceinline__ void init_body(const FusedArgs& a, double* v) {
         const double2 z = make_double2(0.0, 0.0);
         a.p[n] = z;
         a.kp[n] = z;
-        a.gA[3 * (size_t)n] = u;
-        a.gA[3 * (size_t)n + 2] = z;
+        a.gA[rec_at<HALF>(a, n, 0)] = u;
+        a.gA[rec_at<HALF>(a, n, 2)] = z;
         v[0] += r.x * r.x + r.y * r.y;
         v[1] += bb.x * bb.x + bb.y * bb.y;
     }
@@ -155,7 +237,7 @@ __device__ __forceinline__ void init_scalars(CgScalars* sc, const double* t, dou
 
 // w = K u (u from the parity-0 records), M w into the record; gamma = (r, u),
 // delta = (w, u): the first step.
-template <bool P>
+template <bool P, bool HALF>
 __device__ __forceinline__ void w_body(const FusedArgs& a, double* v) {
     CPF_SLICE_LOOP {
         const int n = 32 * sl + lane;
@@ -166,14 +248,15 @@ __device__ __forceinline__ void w_body(const FusedArgs& a, double* v) {
             const long long bi = base + 32LL * k + lane;
             const int col = __ldg(a.scol + bi);
             const double2 lo = load_lo(a.val, bi), hi = load_hi(a.val, bi);
-            const double2 uc = P ? __ldcg(a.gA + 3 * (size_t)col) : a.gA[3 * (size_t)col];
+            const double2* up = a.gA + rec_at<HALF>(a, col, 0);
+            const double2 uc = P ? __ldcg(up) : *up;
             k0 += lo.x * uc.x + lo.y * uc.y;
             k1 += hi.x * uc.x + hi.y * uc.y;
         }
         const double2 w = make_double2(k0, k1);
         a.w[n] = w;
-        a.gA[3 * (size_t)n + 1] = apply_m(a, n, w);
-        const double2 u = a.gA[3 * (size_t)n], r = a.r[n];
+        a.gA[rec_at<HALF>(a, n, 1)] = apply_m(a, n, w);
+        const double2 u = a.gA[rec_at<HALF>(a, n, 0)], r = a.r[n];
         v[0] += r.x * u.x + r.y * u.y;
         v[1] += w.x * u.x + w.y * u.y;
     }
@@ -268,6 +351,125 @@ __device__ __forceinline__ void iter_body(const FusedArgs& a, int parity, double
     }
 }
 
+// The same from the upper half of K: the diagonal block, the first kChunk ones
+// left and right of it in straight-line code (all of a quad's or triangle's
+// row away from the seams of the numbering), the rest in loops. The words of
+// the left ones are loaded a slice ahead, since the address of a block and its
+// record hang on them. It is bound by the loads that 16 warps of 128 registers
+// keep in flight: 0.76 of the copy rate. Per iteration: 230,400 nodes 36.4 ->
+// 27.1 us, 1,049,600 118 -> 101, 1,961,400 210 -> 177, triangles (1,049,600)
+// 110 -> 94, 8-node quads (461,824) 97 -> 95; 99,856 20.0 -> 18.9. (Mirrors
+// found through the slices' offsets instead of in slots of their own take 150
+// us at 1,049,600 nodes; chunks of 3, 3 blocks per SM, 1: 117, 117, 119.)
+constexpr int kChunk = 4;
+constexpr unsigned int kNoLow = 0xffffffffu;
+
+
+// A neighbour's block and record on their way.
+struct Term {
+    double2 lo, hi, uc, mw, mk;
+};
+__device__ __forceinline__ Term low_term(const FusedArgs& a, const double2* __restrict__ go, size_t N, int n,
+                                         unsigned int word) {
+    const bool in = word != kNoLow;
+    const int col = in ? (int)(word & ((1u << kLowShift) - 1)) : n;
+    const double2* vp = a.half.val + 2 * half_at(a.half.u, col >> 5, in ? word >> kLowShift : 0, col & 31);
+    Term t = {__ldg(vp), __ldg(vp + 1), __ldg(go + col), __ldg(go + N + col), __ldg(go + 2 * N + col)};
+    const double y = t.lo.y;  // the mirror's transpose
+    t.lo.y = in ? t.hi.x : 0.0;
+    t.hi.x = in ? y : 0.0;
+    if (!in) t.lo.x = t.hi.y = 0.0;
+    return t;
+}
+__device__ __forceinline__ Term up_term(const double2* __restrict__ go, size_t N, int n, const double2* vp, int c) {
+    const int col = c < 0 ? n : c;  // (padding blocks are zero)
+    return {__ldg(vp), __ldg(vp + 1), __ldg(go + col), __ldg(go + N + col), __ldg(go + 2 * N + col)};
+}
+__device__ __forceinline__ void add_term(const Term& t, double al, double bt, double& k0, double& k1) {
+    const double ux = t.uc.x - al * (t.mw.x + bt * t.mk.x), uy = t.uc.y - al * (t.mw.y + bt * t.mk.y);
+    k0 += t.lo.x * ux + t.lo.y * uy;
+    k1 += t.hi.x * ux + t.hi.y * uy;
+}
+
+__device__ __forceinline__ void iter_body_half(const FusedArgs& a, int parity, double al, double bt, double* v) {
+    const double2* __restrict__ go = parity ? a.gB : a.gA;
+    double2* __restrict__ gn = parity ? a.gA : a.gB;
+    const size_t N = a.n;
+    const int lane = threadIdx.x & 31;
+    const int nwarps = (gridDim.x * blockDim.x) >> 5, n_slices = (a.n + 31) / 32;
+    int sl = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    unsigned int ahead[kChunk], wide = 0;
+    if (sl < n_slices) {
+#pragma unroll
+        for (int j = 0; j < kChunk; ++j) ahead[j] = j < a.half.l ? __ldcs(a.half.low + half_at(a.half.l, sl, j, lane)) : kNoLow;
+        wide = a.half.width[sl];
+    }
+    for (; sl < n_slices; sl += nwarps) {
+        const int n = 32 * sl + lane;
+        const unsigned int wd = wide;
+        unsigned int low[kChunk];
+        int up[kChunk];
+#pragma unroll
+        for (int j = 0; j < kChunk; ++j) low[j] = ahead[j];
+        if (sl + nwarps < n_slices) {
+#pragma unroll
+            for (int j = 0; j < kChunk; ++j)
+                ahead[j] = j < a.half.l ? __ldcs(a.half.low + half_at(a.half.l, sl + nwarps, j, lane)) : kNoLow;
+            wide = a.half.width[sl + nwarps];
+        }
+#pragma unroll
+        for (int j = 0; j < kChunk; ++j) up[j] = 1 + j < a.half.u ? __ldcs(a.half.ucol + half_at(a.half.u, sl, 1 + j, lane)) : -1;
+        if (n >= a.n) continue;
+        const double2* own = a.half.val + 2 * half_at(a.half.u, sl, 0, lane);
+        const double2 dlo = __ldg(own), dhi = __ldg(own + 1);
+        const double2 u0 = go[n], mw0 = go[N + n], mk0 = go[2 * N + n];
+        const double2 pn = __ldcs(a.p + n), wn = __ldcs(a.w + n), kn = __ldcs(a.kp + n);
+        const uchar2 m = a.mask[n];
+        double2 x = __ldcs(a.x + n), r = __ldcs(a.r + n);
+        Term tl[kChunk], tu[kChunk];
+#pragma unroll
+        for (int j = 0; j < kChunk; ++j) tl[j] = low_term(a, go, N, n, low[j]);
+        const double2 p = make_double2(u0.x + bt * pn.x, u0.y + bt * pn.y);
+        const double2 kp = make_double2(wn.x + bt * kn.x, wn.y + bt * kn.y);
+        const double2 u = make_double2(u0.x - al * (mw0.x + bt * mk0.x), u0.y - al * (mw0.y + bt * mk0.y));
+        x.x += al * p.x;
+        x.y += al * p.y;
+        if (m.x) r.x -= al * kp.x;
+        if (m.y) r.y -= al * kp.y;
+        double k0 = dlo.x * u.x + dlo.y * u.y, k1 = dhi.x * u.x + dhi.y * u.y;
+#pragma unroll
+        for (int j = 0; j < kChunk; ++j) add_term(tl[j], al, bt, k0, k1);
+#pragma unroll
+        for (int j = 0; j < kChunk; ++j)  // (beyond the widest row: the diagonal block's place, not used)
+            tu[j] = up_term(go, N, n, own + (1 + j < a.half.u ? 64 * (1 + j) : 0), up[j]);
+#pragma unroll
+        for (int j = 0; j < kChunk; ++j)
+            if (up[j] >= 0) add_term(tu[j], al, bt, k0, k1);
+        const int wu = wd & 0xff, wl = wd >> 8;
+        for (int q = kChunk; q < wl; ++q)
+            add_term(low_term(a, go, N, n, __ldcs(a.half.low + half_at(a.half.l, sl, q, lane))), al, bt, k0, k1);
+        for (int q = 1 + kChunk; q < wu; ++q) {
+            const int c = __ldcs(a.half.ucol + half_at(a.half.u, sl, q, lane));
+            const Term t = up_term(go, N, n, own + 64 * q, c);
+            if (c >= 0) add_term(t, al, bt, k0, k1);
+        }
+        const double2 w = make_double2(k0, k1);
+        __stcs(a.p + n, p);
+        __stcs(a.kp + n, kp);
+        __stcs(a.x + n, x);
+        __stcs(a.r + n, r);
+        __stcs(a.w + n, w);
+        gn[n] = u;
+        gn[N + n] = apply_m(a, n, w);
+        gn[2 * N + n] = apply_m(a, n, kp);
+        v[0] += r.x * u.x + r.y * u.y;
+        v[1] += w.x * u.x + w.y * u.y;
+        v[2] += r.x * r.x + r.y * r.y;
+        v[3] += (w.x * p.x + w.y * p.y) + (kp.x * u.x + kp.y * u.y);
+        v[4] += kp.x * p.x + kp.y * p.y;
+    }
+}
+
 __device__ __forceinline__ void iter_scalars(CgScalars* sc, const double* t) {
     const double g = t[0], rn = t[2];
     const double beta = g / sc->rho;
@@ -284,23 +486,25 @@ __device__ __forceinline__ void iter_scalars(CgScalars* sc, const double* t) {
     sc->ticket = 0;
 }
 
+template <bool HALF>
 __global__ void __launch_bounds__(kThreads) k_f_init(FusedArgs a, double eps2, long long max_iter) {
     __shared__ double sh[2 * kThreads / 32];
     __shared__ bool last;
     double v[2] = {0.0, 0.0};
-    init_body(a, v);
+    init_body<HALF>(a, v);
     double t[kSums];
     if (!reduce_sums(a, v, 2, t, sh, &last)) return;
     if (threadIdx.x == 0) init_scalars(a.sc, t, eps2, max_iter);
 }
 
+template <bool HALF>
 __global__ void __launch_bounds__(kThreads) k_f_w(FusedArgs a) {
     __shared__ double sh[2 * kThreads / 32];
     __shared__ bool last;
     CgScalars* sc = a.sc;
     if (sc->converged || sc->status) return;
     double v[2] = {0.0, 0.0};
-    w_body<false>(a, v);
+    w_body<false, HALF>(a, v);
     double t[kSums];
     if (!reduce_sums(a, v, 2, t, sh, &last)) return;
     if (threadIdx.x == 0) w_scalars(sc, t);
@@ -329,6 +533,19 @@ __global__ void __launch_bounds__(kThreads) k_f_iter(FusedArgs a, int parity) {
 template <int C>
 __global__ void __launch_bounds__(kThreads, 4) k_f_iter4(FusedArgs a, int parity) {
     iter_kernel_body<C>(a, parity);
+}
+
+__global__ void __launch_bounds__(kThreads, 2) k_f_iter_half(FusedArgs a, int parity) {
+    __shared__ double sh[2 * kThreads / 32];
+    __shared__ bool last;
+    pdl_enter();
+    CgScalars* sc = a.sc;
+    if (sc->converged || sc->status) return;
+    double v[kSums] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+    iter_body_half(a, parity, sc->alpha, sc->beta, v);
+    double t[kSums];
+    if (!reduce_sums(a, v, 5, t, sh, &last)) return;
+    if (threadIdx.x == 0) iter_scalars(sc, t);
 }
 
 // ---------------------------------------------------- persistent form --
@@ -403,7 +620,7 @@ __global__ void __launch_bounds__(kThreads) k_f_persistent(FusedArgs a, double e
     double t[kSums];
     {
         double v[2] = {0.0, 0.0};
-        init_body(a, v);
+        init_body<false>(a, v);
         if (reduce_sums(a, v, 2, t, sh, &last) && threadIdx.x == 0) {
             init_scalars(sc, t, eps2, max_iter);
             grid_release(sc);
@@ -412,7 +629,7 @@ __global__ void __launch_bounds__(kThreads) k_f_persistent(FusedArgs a, double e
     }
     {
         double v[2] = {0.0, 0.0};
-        w_body<true>(a, v);
+        w_body<true, false>(a, v);
         if (reduce_sums(a, v, 2, t, sh, &last) && threadIdx.x == 0) {
             w_scalars(sc, t);
             grid_release(sc);
@@ -501,11 +718,29 @@ IterKernel iter_kernel() {
 
 }  // namespace
 
+// CUPLAST_HALF_K = 0 or 1: never or wherever it can be (tests, measurements).
+bool fused_wants_half(int n, int wmax) {
+    const char* e = std::getenv("CUPLAST_HALF_K");
+    return (e ? e[0] == '1' : n >= kHalfLeast) && n < (1 << kLowShift) && wmax <= kHalfMax && form() == kDefaultForm;
+}
+
+void fused_half_widths(const FusedArgs& a, int* widths, cudaStream_t s) {
+    k_f_half_widths<<<std::min((a.n + kThreads - 1) / kThreads, a.sm_count * 8), kThreads, 0, s>>>(a, widths);
+    CP_CUDA(cudaGetLastError());
+}
+
+void fused_half_columns(const FusedArgs& a, cudaStream_t s) {
+    k_f_half_columns<<<std::min((a.n + kThreads - 1) / kThreads, a.sm_count * 8), kThreads, 0, s>>>(a);
+    CP_CUDA(cudaGetLastError());
+}
+
 void fused_launch_start(const FusedArgs& a, double eps2, long long max_iter, cudaStream_t s) {
-    const int g1 = fused_grid(k_f_init, a.n, a.sm_count), g2 = fused_grid(k_f_w, a.n, a.sm_count);
+    const auto init = a.half.val ? k_f_init<true> : k_f_init<false>;
+    const auto first = a.half.val ? k_f_w<true> : k_f_w<false>;
+    const int g1 = fused_grid(init, a.n, a.sm_count), g2 = fused_grid(first, a.n, a.sm_count);
     CP_CHECK(g1 <= a.max_blocks && g2 <= a.max_blocks, CP_ERR_INVALID, "partials buffer too small");
-    k_f_init<<<g1, kThreads, 0, s>>>(a, eps2, max_iter);
-    k_f_w<<<g2, kThreads, 0, s>>>(a);
+    init<<<g1, kThreads, 0, s>>>(a, eps2, max_iter);
+    first<<<g2, kThreads, 0, s>>>(a);
     CP_CUDA(cudaGetLastError());
 }
 
@@ -535,7 +770,7 @@ bool pdl_enabled() {
 }
 
 void fused_launch_iteration(const FusedArgs& a, int parity, cudaStream_t s) {
-    const IterKernel k = iter_kernel();
+    const IterKernel k = a.half.val ? (IterKernel)k_f_iter_half : iter_kernel();
     const int g = fused_grid(k, a.n, a.sm_count);
     CP_CHECK(g <= a.max_blocks, CP_ERR_INVALID, "partials buffer too small");
     cudaLaunchConfig_t cfg = {};

@@ -81,6 +81,8 @@ struct cp_instance {
     double2* mix_u0 = nullptr;         // mixed mode on chip: u before the linear solve
     double2 *f_r = nullptr, *f_w = nullptr, *f_p = nullptr, *f_kp = nullptr, *f_g = nullptr;
     double* f_partials = nullptr;
+    bool f_half_tried = false;
+    cp::HalfK f_half;
     cudaGraphExec_t gf[2] = {nullptr, nullptr};  // [precond]
     // batched engine (batch.cu): FP32 CG vectors, neighbour records, partial sums
     float2* bt_vec = nullptr;

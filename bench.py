@@ -898,9 +898,9 @@ def run_product_arm(args):
         return {k: {"ms": ms[i], "bytes": by[i], "gbs": by[i] / (ms[i] * 1e-3) / 1e9,
                     "frac": by[i] / (ms[i] * 1e-3) / 1e9 / peak} for i, k in enumerate(names)}
 
-    # this workload's own CG: each linear solve is one k_c_solve launch (the
-    # whole CG inside one thread-block cluster, matrix and records in shared
-    # memory). Time per CG iteration from one elastic PCG solve from zero
+    # this workload's own CG: each linear solve is one k_chip launch (the
+    # whole CG inside one thread-block cluster, matrix and vectors in registers
+    # and shared memory). Time per CG iteration from one elastic PCG solve from zero
     # (CUDA events of cp_solve around assembly + solve + update; the solve
     # dominates), against the algorithmic bytes of one CG iteration
     # nnz (8 + 4) + 4 (N + 1) + 2 N 8 + 9 N 8 (N = DOF).
@@ -923,9 +923,9 @@ def run_product_arm(args):
         b_iter, t_iter = None, None
         small_error = str(exc)
     if t_iter is None:
-        roof_small = {"kernel": "k_c_solve", "error": small_error}
+        roof_small = {"kernel": "k_chip", "error": small_error}
     else:
-        roof_small = {"bound": "hbm", "kernel": "k_c_solve (FP64 PCG in one thread-block cluster, per CG iteration)",
+        roof_small = {"bound": "hbm", "kernel": "k_chip (FP64 PCG in one thread-block cluster, per CG iteration)",
                       "achieved": b_iter / t_iter / 1e9, "peak": peak, "unit": "GB/s",
                       "frac": b_iter / t_iter / 1e9 / peak, "traffic": None, "bytes_per_launch": b_iter,
                       "ms_per_launch": t_iter * 1e3, "peak_kind": peak_kind,
@@ -941,8 +941,8 @@ def run_product_arm(args):
     for prec, name in ((cp.CP_PREC_FP64, "fp64"), (cp.CP_PREC_MIXED, "fp32")):
         binst.set_field("uv", np.zeros_like(brp))
         rows[name] = bench_cg(binst, prec, 0, 100)
-    # the FP64 CG iteration that instances too large for one cluster run
-    # (configuration 2): one k_f_iter launch per block-Jacobi PCG iteration
+    # the FP64 CG iteration that instances too large for the chip run
+    # (configuration 2): one k_f_iter_half launch per block-Jacobi PCG iteration
     binst.set_field("uv", np.zeros_like(brp))
     fms, fby = ctypes.c_double(), ctypes.c_double()
     binst.ctx.check(cp._capi.lib().cp_bench_cg_fused(binst._h, 1, 200, ctypes.byref(fms), ctypes.byref(fby)))
@@ -971,18 +971,18 @@ def run_product_arm(args):
     throughput["dof_iterations_per_s_2M"] = 2 * big_nodes / ((mp + mu) * 1e-3)
     cg_large = {k: {"spmv_gbs": b / (m * 1e-3) / 1e9, "update_gbs": c / (n * 1e-3) / 1e9, "ms_spmv": m,
                     "ms_update": n, "us_per_cg_iter": 1e3 * (m + n)} for k, (m, n, b, c) in rows.items()}
-    # "CG GB/s": the FP64 CG iteration of the 2.1M-DOF plate (k_f_iter, the
+    # "CG GB/s": the FP64 CG iteration of the 2.1M-DOF plate (k_f_iter_half, the
     # kernel that takes 90 % of a configuration-2 solve), live CUDA events
-    roofline = {"bound": "hbm", "kernel": "k_f_iter (FP64 block-Jacobi PCG iteration, one launch) on the 2.1M-DOF "
+    roofline = {"bound": "hbm", "kernel": "k_f_iter_half (FP64 block-Jacobi PCG iteration, one launch) on the 2.1M-DOF "
                                           "1024x1024 O-grid plate",
                 "achieved": fby.value / (fms.value * 1e-3) / 1e9, "peak": peak, "unit": "GB/s",
-                "frac": fby.value / (fms.value * 1e-3) / 1e9 / peak, "traffic": 622.5e6,
-                "traffic_note": "dram__bytes_read.sum + dram__bytes_write.sum of one k_f_iter launch on this mesh "
+                "frac": fby.value / (fms.value * 1e-3) / 1e9 / peak, "traffic": 475.4e6,
+                "traffic_note": "dram__bytes_read.sum + dram__bytes_write.sum of one k_f_iter_half launch on this mesh "
                                 "(ncu capture, profiles/k_f_iter_2M.md)",
                 "bytes_per_launch": fby.value, "ms_per_launch": fms.value, "peak_kind": peak_kind,
                 "why_this_kernel": "the metric's CG GB/s: the dominant kernel of the configuration-2 solve "
-                                   "(k_f_iter, 114 us x 924k iterations of its 105 s); the headline step's own "
-                                   "kernel, k_c_solve, keeps the instance on chip and is latency-bound, so its "
+                                   "(k_f_iter_half, 101 us per iteration); the headline step's own "
+                                   "kernel, k_chip, keeps the instance on chip and is latency-bound, so its "
                                    "HBM fraction is reported apart as roofline_headline"}
     mp32, mu32, bp32, bu32 = rows["fp32"]
     roof_fp32 = {"bound": "hbm", "kernel": "k_cg_p<float> (mixed precision SpMV + direction) on the 2.1M-DOF plate",
@@ -1041,7 +1041,7 @@ def run_product_arm(args):
             "cg_form": ("graph loop: P, U, then the V-cycle (restrict per level, dense coarsest "
                         "inverse, prolongation fused into post-smoothing), one kernel each"
                         if SOLVE_KW["precond"] == 2 else os.environ.get("CUPLAST_FP64_CG") or
-                        "one thread-block cluster per linear solve (on chip) where the instance fits"),
+                        "one launch per linear solve (on chip) where the instance fits"),
             "e2e": {"value": e2e_value, "unit": "solves/s", "h2d_bytes_per_step": int(h2d),
                     "d2h_bytes_per_step": int(d2h)},
             "gpu_launches": int(launches), "roofline": roofline, "roofline_headline": roof_small,

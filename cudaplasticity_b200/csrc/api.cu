@@ -267,23 +267,24 @@ void fused_half(cp_instance* I, cp::FusedArgs& a) {
         I->f_half_tried = true;
         cp::HalfK& h = a.half;
         const size_t nodes = 32 * (size_t)I->csr.n_slices;
-        int *widths = I->alloc<int>(2), most[2];
-        h.width = I->alloc<unsigned short>(I->csr.n_slices);
+        const auto room = [I](auto*& p, size_t count) {
+            try {
+                p = I->alloc<std::remove_reference_t<decltype(*p)>>(count);
+            } catch (const Error&) {
+                (void)cudaGetLastError();
+                return false;
+            }
+            return true;
+        };
+        int *widths = nullptr, most[2];
+        if (!room(widths, 2) || !room(h.width, I->csr.n_slices)) return;
         CP_CUDA(cudaMemsetAsync(widths, 0, 2 * sizeof(int), I->s()));
         cp::fused_half_widths(a, widths, I->s());
         CP_CUDA(cudaMemcpyAsync(most, widths, sizeof(most), cudaMemcpyDeviceToHost, I->s()));
         CP_CUDA(cudaStreamSynchronize(I->s()));
         h.u = most[0];
         h.l = most[1];
-        try {
-            h.ucol = I->alloc<int>(nodes * h.u);
-            h.low = I->alloc<unsigned int>(nodes * std::max(h.l, 1));
-            h.val = I->alloc<double2>(2 * nodes * h.u);
-        } catch (const Error&) {
-            (void)cudaGetLastError();
-            h.val = nullptr;
-            return;
-        }
+        if (!room(h.ucol, nodes * h.u) || !room(h.low, nodes * std::max(h.l, 1)) || !room(h.val, 2 * nodes * h.u)) return;
         CP_CUDA(cudaMemsetAsync(h.val, 0, 2 * sizeof(double2) * nodes * h.u, I->s()));
         cp::fused_half_columns(a, I->s());
         I->f_half = h;

@@ -20,8 +20,9 @@
 //     are read through distributed shared memory; each CTA stores its sums
 //     into the other CTAs' shared memory, where they complete an mbarrier
 //     phase (one trip, where a cluster barrier and a read of the sums make
-//     two); every CTA adds up all CTAs' sums in the same
-//     order, so all hold the same scalars and take the same branches.
+//     two) together with one arrival of each CTA, which releases its records;
+//     every CTA adds up all CTAs' sums in the same order, so all hold the same
+//     scalars and take the same branches.
 //   grid (up to one CTA per SM, a cooperative launch): records and sums go
 //     through global memory (L2) in 8-byte words of 32 bits of data and their
 //     sequence number, so that a reader polls the data itself: one trip
@@ -595,7 +596,9 @@ bool chip_schedulable(const ChipPlan& p, int sm_count) {
 //   cluster: about 13 CTAs, of at least 4 slices. 1024 nodes: 8 CTAs of 4
 //     slices 1.45 us per iteration, 16 of 2 1.9, 3 of 12 1.7; 4160 nodes: 13 of
 //     10 1.74, 11 of 12 1.8 (the whole solve in one cluster with every
-//     record read through distributed shared memory: 4.9 and 5.7).
+//     record read through distributed shared memory: 4.9 and 5.7). These are
+//     without the records' release, with which the forms taken have 1.47 and
+//     1.80.
 //   grid: about 128 CTAs, of at least 8 slices. 16104 nodes: 63 CTAs of 8
 //     slices 3.31 us, 126 of 4 3.7, 42 of 12 3.7 (one launch per iteration,
 //     cg_fused.cu: 10.2); 40200 nodes: 126 of 10 3.71, 105 of 12 3.8 (11.4).

@@ -36,8 +36,13 @@ __device__ __forceinline__ void st_async(unsigned int a, unsigned int bar, doubl
                  "l"(__double_as_longlong(x)), "l"(__double_as_longlong(y)), "r"(bar)
                  : "memory");
 }
-__device__ __forceinline__ void bar_init(unsigned int bar) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
+__device__ __forceinline__ void bar_init(unsigned int bar, unsigned int arrivals) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(arrivals) : "memory");
+}
+// One arrival at another CTA's mbarrier, after all that the thread (and, past
+// a block barrier, its block) has read and written.
+__device__ __forceinline__ void bar_arrive_remote(unsigned int bar) {
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 __device__ __forceinline__ void bar_expect(unsigned int bar, unsigned int bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
@@ -186,7 +191,7 @@ struct CommShared {
     double wsum[16][8];                              // per warp: its sums (unused warps stay zero)
     double gsum[kMaxPolls][8];                       // grid, the adding CTA: the same of the CTAs' sums
     __align__(16) double part[2][kMaxCluster][6];    // cluster: every CTA's sums (0, 2, 1, -, 3, 4), by parity
-    __align__(8) unsigned long long bar[2];          // cluster: they have arrived
+    __align__(8) unsigned long long bar[2];          // cluster: they have arrived, and the records are written
     Step step;
     int fail;                                        // rank 0's: some CTA of the cluster gave up
 };
@@ -219,8 +224,8 @@ struct Comm {
             __syncthreads();
         } else {
             if (tid == 0) {
-                bar_init(smem_addr(&S.bar[0]));
-                bar_init(smem_addr(&S.bar[1]));
+                bar_init(smem_addr(&S.bar[0]), ctas + 1);  // every CTA's arrival and the own bar_expect
+                bar_init(smem_addr(&S.bar[1]), ctas + 1);
                 asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
                 bar_expect(smem_addr(&S.bar[0]), 48u * ctas);
                 bar_expect(smem_addr(&S.bar[1]), 48u * ctas);
@@ -273,6 +278,12 @@ struct Comm {
             if ((lane & 3) == 0) S.wsum[w][lane >> 2] = s;
         }
         __syncthreads();
+        // The records are plain stores of all warps, which st.async does not
+        // publish: every CTA releases its own by an arrival at every CTA's
+        // mbarrier (whose waits acquire), from the warp farthest from the sums:
+        // 0.06 us of an iteration at 4160 nodes, 0.02 at 1024.
+        if constexpr (!GRID)
+            if (w == (nthr >> 5) - 1 && lane < ctas) bar_arrive_remote(mapa(smem_addr(&S.bar[par]), lane));
         // lane (g, j): slot j of the warps g, g + 4, ..; then over g
         const int j = lane & 7, g = lane >> 3;
         double s = 0.0;
@@ -297,8 +308,7 @@ struct Comm {
             halo();
         } else {
             if (w == 0) {
-                // sums (0, 2), (1, 1), (3, 4) to every CTA, with the records of
-                // all warps written before the block barrier above
+                // sums (0, 2), (1, 1), (3, 4) to every CTA
                 const double s2 = __shfl_sync(0xffffffffu, s, j == 4 ? 6 : j + 1);
                 if (!(j & 1) && j < 6) {
 #pragma unroll

@@ -370,7 +370,7 @@ cp::ChipArgs<T> chip_args(cp_instance* I, double eps2, long long max_iter, int p
     if (I->chip.grid) cp::chip_ll_carve(I->chip, I->chip_ll, &a.ll_rec, &a.ll_part, &a.ll_step);
     a.seq = I->chip_seq;
     if (I->test_barrier_ns) {
-        a.poll_limit = 1000;
+        a.wait_ns = I->test_barrier_ns;
         a.seq_skew = 1;
     }
     return a;

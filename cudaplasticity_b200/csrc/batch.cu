@@ -134,12 +134,6 @@ struct BCtl {
     int go;                    // condition of the last trip (direct launches)
 };
 
-__device__ __forceinline__ unsigned long long global_ns() {
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-
 __device__ __forceinline__ void set_phase(BState* S, BCtl* c, int ph) {
     atomicSub(&c->pop[S->phase], 1);
     atomicAdd(&c->pop[ph], 1);
@@ -612,7 +606,7 @@ __global__ void __launch_bounds__(kBChipThreads, 1) k_batch_chip(const BDesc* __
     const int count = c->n_chip[cls];
     if (count == 0) return;
     Comm<float, false> comm{cs, tid, kBChipThreads, tid & 31, w, rank, C, 0, 0u, nullptr, nullptr, nullptr, 0,
-                            1u << 22, 0u};
+                            kWaitNs, 0u};
     comm.init();
     const int first_of_class = c->chip_at[cls];
     for (int it = blockIdx.x / C; it < count; it += ncl) {

@@ -52,6 +52,9 @@ struct CgArgs {
     double* partials = nullptr;     // >= 3 * max_blocks doubles
 };
 
+// Time limit of every wait between CTAs (an exchange takes microseconds).
+constexpr unsigned long long kWaitNs = 2000000000ull;
+
 // The upper half of K for cg_fused.cu's iterations: per slice of 32 nodes, up
 // to u blocks right of the diagonal (block 0 is the diagonal one) and up to l
 // left of it, in slots of the slice's widest row.
@@ -85,7 +88,7 @@ struct FusedArgs {
     // number of extra steps every wait asks for (0; 1 makes each wait ask for
     // a step that is never released, so that every wait runs out: the
     // time-out path's test)
-    unsigned long long barrier_ns = 2000000000ull;
+    unsigned long long barrier_ns = kWaitNs;
     unsigned int barrier_skew = 0;
 };
 
@@ -144,12 +147,12 @@ struct ChipArgs {
     const double2* u0 = nullptr;
     double2* inc = nullptr;
     // grid exchange: records, sums and steps by parity, the last sequence
-    // number in use; rounds a poll takes before it gives up, and what is
-    // added to the posted sequence numbers (0; 1 makes every poll run out:
-    // the time-out path's test)
+    // number in use; both exchanges: the time limit of a wait, and what is
+    // added to the posted sequence numbers (0; with 1 every wait runs out, in
+    // the cluster because nothing is sent: the time-out path's test)
     uint4 *ll_rec = nullptr, *ll_part = nullptr, *ll_step = nullptr;
     unsigned int* seq = nullptr;
-    unsigned int poll_limit = 1u << 22;
+    unsigned long long wait_ns = kWaitNs;
     unsigned int seq_skew = 0;
 };
 ChipShape chip_shape(int n, int wmax, int sm_count, bool grid);

@@ -29,8 +29,9 @@
 //     through L2 and no fence. One more CTA, without nodes, adds up the sums
 //     and posts the next step's scalars (all CTAs reading all CTAs' sums takes
 //     twice as long at 63 CTAs and more beyond: every poll then meets every
-//     other on the same lines). Every poll is bounded; a CTA that gives up sets sc->chip_err and
-//     returns, and so do the others at their next poll.
+//     other on the same lines).
+// Every wait of both is limited in time (kWaitNs); a CTA that gives up sets
+// sc->chip_err and returns, and so do the others at their next wait.
 // T is the type of K's values and of the recurrences (double, or float in the
 // mixed mode); x is FP64 and every sum is accumulated and reduced in FP64.
 #include <cstdlib>
@@ -252,7 +253,7 @@ __global__ void __launch_bounds__(kChipWarps * 32, 1) k_chip(ChipArgs<T> a) {
     const bool adder = GRID && rank == ctas;  // the CTA without nodes
     Comm<T, GRID> comm{cs,        tid,       nthr,      tid & 31,          w,           rank,        ctas,
                        own,       0u,        a.ll_rec,  a.ll_part,         a.ll_step,   (size_t)ctas * own,
-                       a.poll_limit, a.seq_skew};
+                       a.wait_ns, a.seq_skew};
     // shared memory: U [own + halo], then (cluster) records [2][3][own], then
     // the blocks that are not in registers
     V2* U = reinterpret_cast<V2*>(smem_raw);

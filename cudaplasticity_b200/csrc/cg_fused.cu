@@ -559,12 +559,6 @@ __global__ void __launch_bounds__(kThreads, 2) k_f_iter_half(FusedArgs a, int pa
 // the cooperative launch. Every wait is bounded in time: a block that gives up
 // sets CP_ERR_TIMEOUT and returns, and so does every other waiting block.
 
-__device__ __forceinline__ unsigned long long global_ns() {
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-
 // The last block of a step (thread 0): publish the scalars it has just
 // written, then release the step.
 __device__ __forceinline__ void grid_release(CgScalars* sc) {

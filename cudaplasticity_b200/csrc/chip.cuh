@@ -91,21 +91,30 @@ __device__ __forceinline__ void post(uint4* p, float2 v, unsigned int seq) {
 }
 __device__ __forceinline__ double word_value(const uint4& q) { return __hiloint2double(q.z, q.x); }
 
+// Of a wait that has taken some rounds: whether it has lasted longer than
+// limit nanoseconds since its first call (t0, 0 before).
+__device__ __forceinline__ bool waited(unsigned long long& t0, unsigned long long limit) {
+    const unsigned long long t = global_ns();
+    if (t0 == 0) t0 = t;
+    return t - t0 > limit;
+}
+
 // Polls N word pairs per lane until those of every lane of the warp carry seq;
-// false after `limit` rounds. The whole warp takes part, with valid addresses
+// false after `limit` nanoseconds (looked at every 256 rounds). The whole warp takes part, with valid addresses
 // in every lane: left to diverge, a warp of which some lanes polled and some
 // did not took 3700 cycles to come together again.
 template <int N>
-__device__ __forceinline__ bool poll(const uint4* p, size_t stride, unsigned int seq, unsigned int limit, uint4* c) {
-    for (unsigned int round = 0; round < limit; ++round) {
+__device__ __forceinline__ bool poll(const uint4* p, size_t stride, unsigned int seq, unsigned long long limit, uint4* c) {
+    unsigned long long t0 = 0;
+    for (unsigned int round = 1;; ++round) {
         bool ok = true;
 #pragma unroll
         for (int i = 0; i < N; ++i) c[i] = ld_words(p + i * stride);
 #pragma unroll
         for (int i = 0; i < N; ++i) ok = ok && c[i].y == seq && c[i].w == seq;
         if (__all_sync(0xffffffffu, ok)) return true;
+        if ((round & 255u) == 0u && __any_sync(0xffffffffu, waited(t0, limit))) return false;
     }
-    return false;
 }
 
 // A record (u, M w, M kp): pair i at p[i * stride].
@@ -208,7 +217,8 @@ struct Comm {
     unsigned int rec_base = 0;  // cluster: records [2][3][own]
     uint4 *ll_rec, *ll_part, *ll_step;
     size_t slots;
-    unsigned int poll_limit, seq_skew;
+    unsigned long long wait_ns;
+    unsigned int seq_skew;
     unsigned int seq = 0;
     int par = 1;             // parity of the last exchange
     unsigned int phase = 0;  // of the mbarriers' next wait
@@ -244,7 +254,10 @@ struct Comm {
     __device__ __forceinline__ void read_halo(unsigned int at, V2* q) {
         if constexpr (GRID) {
             uint4 c[NR];
-            if (!poll<NR>(ll_rec + (size_t)par * NR * slots + at, slots, seq, poll_limit, c)) failed = true;
+            if (failed || !poll<NR>(ll_rec + (size_t)par * NR * slots + at, slots, seq, wait_ns, c)) {
+                failed = true;  // (of a block that has given up: no further waits)
+                return;
+            }
             Record<T>::get(c, q);
         } else {
             const unsigned int s = at + (unsigned int)(par * 3 * own * sizeof(V2));
@@ -283,7 +296,7 @@ struct Comm {
         // mbarrier (whose waits acquire), from the warp farthest from the sums:
         // 0.06 us of an iteration at 4160 nodes, 0.02 at 1024.
         if constexpr (!GRID)
-            if (w == (nthr >> 5) - 1 && lane < ctas) bar_arrive_remote(mapa(smem_addr(&S.bar[par]), lane));
+            if (w == (nthr >> 5) - 1 && lane < ctas && seq_skew == 0u) bar_arrive_remote(mapa(smem_addr(&S.bar[par]), lane));
         // lane (g, j): slot j of the warps g, g + 4, ..; then over g
         const int j = lane & 7, g = lane >> 3;
         double s = 0.0;
@@ -299,7 +312,7 @@ struct Comm {
             if (w == 0 && (lane < 3 || lane == 4 || lane == 6)) post(pp + (size_t)val * ctas + rank, s, seq + seq_skew);
             if (w == 0) {
                 uint4 c[1];
-                if (!poll<1>(ll_step + par * 4 + min(lane, kStepWords - 1), 1, seq, poll_limit, c)) failed = true;
+                if (!poll<1>(ll_step + par * 4 + min(lane, kStepWords - 1), 1, seq, wait_ns, c)) failed = true;
                 const double q = word_value(c[0]);
                 if (lane == 0) S.step.alpha = q;
                 if (lane == 1) S.step.beta = q;
@@ -310,7 +323,7 @@ struct Comm {
             if (w == 0) {
                 // sums (0, 2), (1, 1), (3, 4) to every CTA
                 const double s2 = __shfl_sync(0xffffffffu, s, j == 4 ? 6 : j + 1);
-                if (!(j & 1) && j < 6) {
+                if (!(j & 1) && j < 6 && seq_skew == 0u) {
 #pragma unroll
                     for (int i = 0; i < 4; ++i)
                         if (g + 4 * i < ctas)
@@ -320,9 +333,9 @@ struct Comm {
             }
             {
                 const unsigned int ba = smem_addr(&S.bar[par]);
-                unsigned int round = 0;
+                unsigned long long t0 = 0;
                 while (!bar_try(ba, phase)) {
-                    if (++round > poll_limit) {
+                    if (__builtin_expect(waited(t0, wait_ns), 0)) {
                         failed = true;
                         break;
                     }
@@ -374,7 +387,7 @@ struct Comm {
             double t[kSums];
             uint4 ch[kSums];
             const int c = 32 * q + lane;
-            if (!poll<kSums>(pp + min(c, ctas - 1), ctas, seq, poll_limit, ch)) failed = true;
+            if (!poll<kSums>(pp + min(c, ctas - 1), ctas, seq, wait_ns, ch)) failed = true;
 #pragma unroll
             for (int i = 0; i < kSums; ++i) t[i] = c < ctas ? word_value(ch[i]) : 0.0;
             const double r5 = warp_sum5(t, lane);

@@ -132,6 +132,8 @@ struct BCtl {
     int n_chip[kBChipClasses], chip_at[kBChipClasses];  // on-chip instances per cluster size, in the chip list
     const volatile int* stop;  // host-mapped interrupt flag
     int go;                    // condition of the last trip (direct launches)
+    unsigned long long wait_ns;  // of the on-chip linear solve, as ChipArgs
+    unsigned int skew;
 };
 
 __device__ __forceinline__ void set_phase(BState* S, BCtl* c, int ph) {
@@ -606,7 +608,7 @@ __global__ void __launch_bounds__(kBChipThreads, 1) k_batch_chip(const BDesc* __
     const int count = c->n_chip[cls];
     if (count == 0) return;
     Comm<float, false> comm{cs, tid, kBChipThreads, tid & 31, w, rank, C, 0, 0u, nullptr, nullptr, nullptr, 0,
-                            kWaitNs, 0u};
+                            c->wait_ns, c->skew};
     comm.init();
     const int first_of_class = c->chip_at[cls];
     for (int it = blockIdx.x / C; it < count; it += ncl) {
@@ -772,8 +774,9 @@ __global__ void __launch_bounds__(kBChipThreads, 1) k_batch_chip(const BDesc* __
 #pragma unroll
                     for (int j = 0; j < 2; ++j)
                         if (n[j] >= 0) d.x[n[j]] = x[j];
-                    cluster_arrive_release();
-                    cluster_wait();
+                    // x to the other CTAs, by an exchange (chip.cuh, close())
+                    exchange([](const double*) -> Step { return {0.0, 0.0, NX_RES}; });
+                    if (comm.failed) break;
                 }
                 v[0] = v[1] = v[2] = v[3] = v[4] = 0.0;
 #pragma unroll
@@ -1210,6 +1213,7 @@ struct cp_batch {
     int* d_chip = nullptr;  // on-chip instances by cluster size (slots)
     int* h_chip = nullptr;  // pinned
     bool chip_ok = false;   // the GPU takes the on-chip kernel's clusters
+    unsigned long long test_wait_ns = 0;  // CUPLAST_TEST_BARRIER_NS, as cp_instance::test_barrier_ns
     cudaStream_t aux[kBChipClasses] = {};  // capture: the on-chip launches beside the tile kernels'
     cudaEvent_t fork = nullptr, join[kBChipClasses] = {};
     int tiles_cap = 0;
@@ -1542,6 +1546,7 @@ CP_API int cp_batch_create(cp_context* ctx, const cp_batch_opts* opts, cp_batch*
         CP_CUDA(cudaMalloc(&b->d_chip, sizeof(int) * (size_t)b->cap));
         CP_CUDA(cudaMallocHost(&b->h_chip, sizeof(int) * (size_t)b->cap));
         b->chip_ok = bchip_available();
+        if (const char* g = std::getenv("CUPLAST_TEST_BARRIER_NS")) b->test_wait_ns = std::strtoull(g, nullptr, 10);
         CP_CUDA(cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming));
         for (int k = 0; k < kBChipClasses; ++k) {
             CP_CUDA(cudaStreamCreateWithFlags(&b->aux[k], cudaStreamNonBlocking));
@@ -1757,6 +1762,8 @@ CP_API int cp_batch_launch(cp_batch* b, int until, long long max_trips) {
         c.trips = 0;
         c.max_trips = max_trips;
         c.stop = b->d_stop;
+        c.wait_ns = b->test_wait_ns ? b->test_wait_ns : kWaitNs;
+        c.skew = b->test_wait_ns ? 1 : 0;
         *b->h_ctl = c;
         *(volatile int*)b->h_stop = 0;
         if (nt > 0) CP_CUDA(cudaMemcpyAsync(b->d_tiles, b->h_tiles, sizeof(int4) * (size_t)nt, cudaMemcpyHostToDevice, s));

@@ -202,7 +202,7 @@ struct CommShared {
     __align__(16) double part[2][kMaxCluster][6];    // cluster: every CTA's sums (0, 2, 1, -, 3, 4), by parity
     __align__(8) unsigned long long bar[2];          // cluster: they have arrived, and the records are written
     Step step;
-    int fail;                                        // rank 0's: some CTA of the cluster gave up
+    int fail;                                        // cluster: some CTA of it gave up
 };
 
 // The exchange of one iteration: the own records and sums out, the halo
@@ -362,20 +362,16 @@ struct Comm {
     }
     // Cluster: at the end of a solve, whole cluster: all CTAs have read each
     // other's shared memory for the last time; whether any of them gave up.
+    // This and init() hold the only cluster barriers, so that a CTA that gives
+    // up meets the others here wherever they are (their next wait runs out
+    // too). The flag is sent to every CTA before the barrier and read from the
+    // own memory after it, when the others may have gone.
     __device__ __forceinline__ bool close() {
-        if (failed && tid == 0) {
-            const unsigned int f = mapa(smem_addr(&S.fail), 0);
-            asm volatile("st.shared::cluster.u32 [%0], 1;" ::"r"(f) : "memory");
-        }
+        if (failed && tid < ctas)
+            asm volatile("st.shared::cluster.u32 [%0], 1;" ::"r"(mapa(smem_addr(&S.fail), tid)) : "memory");
         cluster_arrive_release();
         cluster_wait();
-        int any;
-        asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(any) : "r"(mapa(smem_addr(&S.fail), 0)) : "memory");
-        if (any) {  // nobody goes while the flag is read
-            cluster_arrive_release();
-            cluster_wait();
-        }
-        return any != 0;
+        return *(volatile int*)&S.fail != 0;
     }
     // Grid: the adding CTA's side of one exchange.
     template <typename Decide>

@@ -11,7 +11,7 @@ import numpy as np
 import pytest
 
 import cudaplasticity_b200 as cp
-from test_gpu_chip import check, ctx, solve, strip  # noqa: F401
+from test_gpu_chip import EPS64, check, ctx, residual, solve, strip  # noqa: F401
 
 pytestmark = pytest.mark.gpu
 
@@ -60,3 +60,56 @@ def test_waits_are_limited_in_time(nx, ny, precision, ctx, monkeypatch):  # noqa
     assert 0.3 <= t <= 0.3 * 3 + 0.5  # a wait of each side of the exchange, and the set-up
     monkeypatch.delenv("CUPLAST_TEST_BARRIER_NS")
     check(p, *solve(ctx, p), 1e-11)
+
+
+# a cluster of 4, of 8 and of 16 CTAs
+@pytest.mark.parametrize("nx, ny", [(64, 26), (96, 60), (120, 80)])
+def test_batch_that_gives_up(nx, ny, ctx, monkeypatch):  # noqa: F811
+    """The same in a batch: each of its on-chip solves ends by itself with CP_ERR_TIMEOUT, and the context stays
+    usable."""
+    p = strip(nx, ny)
+    arrays, rp, mask = p
+    kw = dict(cg_tol=1e-11, outer_tol=1e300, inner_tol=1e-3, max_outer=1, max_cg=100000, precond=1)
+    for withheld in (True, False):
+        if withheld:
+            monkeypatch.setenv("CUPLAST_TEST_BARRIER_NS", "50000000")
+        batch = cp.Batch(ctx, max_instances=3)
+        monkeypatch.delenv("CUPLAST_TEST_BARRIER_NS", raising=False)
+        insts = [cp.Instance(ctx, arrays, cp.material(210000.0, 0.3)) for _ in range(3)]
+        for i in insts:
+            i.set_loads(rp, mask)
+            batch.add(i, **kw)
+        t = time.monotonic()
+        batch.run()
+        t = time.monotonic() - t
+        reps = [r for _, _, r in batch.harvest()]
+        assert len(reps) == 3
+        if withheld:
+            assert [r["status"] for r in reps] == [cp._capi.CP_ERR_TIMEOUT] * 3 and t <= 2.0
+        else:
+            for i, r in zip(insts, reps):
+                res, gap = residual(p, i.field("uv"), i.csr())
+                assert r["status"] == 0 and res <= 1e-11 + 2 * 20 * EPS64 * gap
+        for i in insts:
+            i.close()
+        batch.close()
+
+
+@pytest.mark.parametrize("nx, ny", [(64, 26), (96, 60), (120, 80)])
+def test_batch_residuals_are_of_the_whole_x(nx, ny, ctx):  # noqa: F811
+    """The FP64 residual of a batch's solve reads every CTA's x: with an inner tolerance that replaces it every few
+    iterations the result is the same bit for bit, alone and again."""
+    arrays, rp, mask = strip(nx, ny, "q4", 11)
+    out = []
+    for _ in range(6):
+        batch = cp.Batch(ctx, max_instances=1)
+        i = cp.Instance(ctx, arrays, cp.material(210000.0, 0.3))
+        i.set_loads(rp, mask)
+        batch.add(i, cg_tol=1e-10, outer_tol=1e300, inner_tol=0.3, max_outer=1, max_cg=100000, precond=1)
+        batch.run()
+        rep = batch.harvest()[0][2]
+        assert rep["status"] == 0 and rep["cg_rel_res"] <= 1e-10
+        out.append(i.field("uv"))
+        i.close()
+        batch.close()
+    assert all(np.array_equal(u, out[0]) for u in out)

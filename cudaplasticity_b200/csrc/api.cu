@@ -964,7 +964,7 @@ CP_API int cp_secant_update(cp_instance* I, double* rel_err) {
     if (I && I->in_batch) return CP_ERR_BUSY;  // owned by a batch until harvested
     if (!I) return CP_ERR_INVALID;
     return guarded(I->ctx, [&] {
-        cp::launch_update(I->mesh, I->mat, I->u, I->st, I->osc, I->partials, 0, 0, I->s(), I->sms());
+        cp::launch_update(I->mesh, I->mat, I->u, I->st, I->osc, I->partials, 0, 0, nullptr, I->s(), I->sms());
         CP_CUDA(cudaMemcpyAsync(I->osc_h, I->osc, sizeof(cp::OuterScalars), cudaMemcpyDeviceToHost, I->s()));
         CP_CUDA(cudaStreamSynchronize(I->s()));
         if (rel_err) *rel_err = I->osc_h->rel_err;
@@ -1091,11 +1091,14 @@ CP_API int cp_solve(cp_instance* I, const cp_solve_opts* opts, cp_solve_report* 
                     cg_mixed(I, eps, o.inner_tol, o.max_cg, &R.cg_iters, &R.fp64_spmv, &rr, o.precond ? 1 : 0);
                     R.cg_rel_res = rr;
                 }
-                cp::launch_update(I->mesh, I->mat, I->u, I->st, I->osc, I->partials, o.aitken, first, s, I->sms());
+                // (a linear solve whose outcome is not known here holds the update off where it failed)
+                const cp::CgScalars* pending = mg_deferred || chip_deferred ? I->sc : nullptr;
+                cp::launch_update(I->mesh, I->mat, I->u, I->st, I->osc, I->partials, o.aitken, first, pending, s,
+                                  I->sms());
                 I->launches += 1;
                 CP_CUDA(cudaMemcpyAsync(I->osc_h, I->osc, sizeof(cp::OuterScalars), cudaMemcpyDeviceToHost, s));
                 if (o.aitken) {  // the factor stays on the device
-                    cp::launch_aitken_relax(I->mesh, I->mat, I->st, I->osc, s, I->sms());
+                    cp::launch_aitken_relax(I->mesh, I->mat, I->st, I->osc, pending, s, I->sms());
                     I->launches += 1;
                 }
                 first = 0;

@@ -83,6 +83,10 @@ __global__ void __launch_bounds__(kAsmThreads) k_assemble(DevMesh m, DevCsr csr,
 }  // namespace
 constexpr int kElemThreads = 256;
 
+__device__ __forceinline__ bool solve_failed(const CgScalars* solve) {
+    return solve && (solve->status == CP_ERR_BREAKDOWN || solve->chip_err);
+}
+
 // strain4 + plastStress + exitNorm2 (src/PlasticitySolver.cu:1517-1549,
 // 1590-1610, 1664-1691) fused: element-mean strain, stress from the C of the
 // last assembly, stress intensity, secant update, and the two exit-norm sums
@@ -92,12 +96,15 @@ constexpr int kElemThreads = 256;
 // that fits once, so that the block sums and their fence are paid once per
 // block: 1,048,576 quads with Hollomon hardening, whole call 125 us at 2
 // blocks per SM with Newton's method on pow, 73 now (floor 26: 168 MB).
+// solve: a linear solve whose outcome the host has not seen yet; where it
+// failed, the elements keep their state.
 template <bool Q8>
 __global__ void __launch_bounds__(kElemThreads, 4) k_update(DevMesh m, MaterialDev M, const double2* __restrict__ u,
                                                          ElemState st, OuterScalars* sc, double* partials, int aitken,
-                                                         int first) {
+                                                         int first, const CgScalars* solve) {
     __shared__ double sh[2 * kElemThreads / 32];
     __shared__ bool last;
+    if (solve_failed(solve)) return;
     const int ne = m.c3 + m.c4 + m.c8;
     double s_num = 0.0, s_den = 0.0, s_an = 0.0, s_ad = 0.0;
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < ne; e += gridDim.x * blockDim.x)
@@ -140,8 +147,10 @@ namespace {
 
 // Aitken (Irons-Tuck) relaxation of the secant iteration on psi:
 // psi_{k+1} = psi_k + w_k r_k, w_k = -w_{k-1} (r_{k-1}, r_k - r_{k-1}) / |r_k - r_{k-1}|^2.
-// The fixed point (r = 0) is the reference's.
-__global__ void k_aitken(DevMesh m, MaterialDev M, ElemState st, const OuterScalars* sc) {
+// The fixed point (r = 0) is the reference's. Nothing moves after a failed
+// linear solve or an exit norm that is not finite, which the host has yet to see.
+__global__ void k_aitken(DevMesh m, MaterialDev M, ElemState st, const OuterScalars* sc, const CgScalars* solve) {
+    if (solve_failed(solve) || !(sc->rel_err - sc->rel_err == 0.0)) return;
     const int ne = m.c3 + m.c4 + m.c8;
     const double w = sc->aitken_omega;
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < ne; e += gridDim.x * blockDim.x)
@@ -197,19 +206,17 @@ int update_grid(int ne, int sm_count) {
 }
 
 void launch_update(const DevMesh& m, const MaterialDev& mat, const double2* u, ElemState& st, OuterScalars* sc,
-                   double* partials, int aitken, int first, cudaStream_t s, int sm_count) {
+                   double* partials, int aitken, int first, const CgScalars* solve, cudaStream_t s, int sm_count) {
     const int ne = m.c3 + m.c4 + m.c8;
-    if (m.c8)
-        k_update<true><<<update_grid(ne, sm_count), elem_threads(ne, sm_count), 0, s>>>(m, mat, u, st, sc, partials, aitken, first);
-    else
-        k_update<false><<<update_grid(ne, sm_count), elem_threads(ne, sm_count), 0, s>>>(m, mat, u, st, sc, partials, aitken, first);
+    const auto k = m.c8 ? k_update<true> : k_update<false>;
+    k<<<update_grid(ne, sm_count), elem_threads(ne, sm_count), 0, s>>>(m, mat, u, st, sc, partials, aitken, first, solve);
     CP_CUDA(cudaGetLastError());
 }
 
 void launch_aitken_relax(const DevMesh& m, const MaterialDev& mat, ElemState& st, const OuterScalars* sc,
-                         cudaStream_t s, int sm_count) {
+                         const CgScalars* solve, cudaStream_t s, int sm_count) {
     const int ne = m.c3 + m.c4 + m.c8;
-    k_aitken<<<update_grid(ne, sm_count), elem_threads(ne, sm_count), 0, s>>>(m, mat, st, sc);
+    k_aitken<<<update_grid(ne, sm_count), elem_threads(ne, sm_count), 0, s>>>(m, mat, st, sc, solve);
     CP_CUDA(cudaGetLastError());
 }
 
@@ -303,7 +310,7 @@ extern "C" CP_API int cp_secant_update_noalloc(void* stream, const cp_material* 
     es.psi = d_psi; es.E_c = d_E_c; es.nu_c = d_nu_c;
     const int threads = cp::elem_threads(count4, 148);
     const int grid = cp::update_grid(count4, 148);  // <= kNoAllocMaxBlocks
-    cp::k_update<false><<<grid, threads, 0, s>>>(m, M, reinterpret_cast<const double2*>(d_uv), es, sc, partials, 0, 0);
+    cp::k_update<false><<<grid, threads, 0, s>>>(m, M, reinterpret_cast<const double2*>(d_uv), es, sc, partials, 0, 0, nullptr);
     if (cudaGetLastError() != cudaSuccess) return CP_ERR_CUDA;
     double host_err = 0.0;
     if (cudaMemcpyAsync(&host_err, &sc->rel_err, sizeof(double), cudaMemcpyDeviceToHost, s) != cudaSuccess)

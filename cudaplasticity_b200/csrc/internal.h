@@ -126,9 +126,9 @@ struct MaterialDev {
 void launch_assemble(const DevMesh& m, const DevCsr& csr, const MaterialDev& mat, const double* E_c,
                      const double* nu_c, bool want64, bool want32, cudaStream_t s, int sm_count);
 void launch_update(const DevMesh& m, const MaterialDev& mat, const double2* u, ElemState& st, OuterScalars* sc,
-                   double* partials, int aitken, int first, cudaStream_t s, int sm_count);
+                   double* partials, int aitken, int first, const CgScalars* solve, cudaStream_t s, int sm_count);
 void launch_aitken_relax(const DevMesh& m, const MaterialDev& mat, ElemState& st, const OuterScalars* sc,
-                         cudaStream_t s, int sm_count);
+                         const CgScalars* solve, cudaStream_t s, int sm_count);
 void launch_plastic(const DevMesh& m, const MaterialDev& mat, ElemState& st, cudaStream_t s, int sm_count);
 
 }  // namespace cp

@@ -263,31 +263,34 @@ void run_cg_loop(cp_instance* I, const cp::CgArgs<T>& a, cudaGraphExec_t g) {
 // The upper half of K for the one-launch FP64 CG, its columns built on first
 // use; without room for it the iterations read all of K.
 void fused_half(cp_instance* I, cp::FusedArgs& a) {
-    if (!I->f_half_tried && cp::fused_wants_half(a.n, I->csr.max_width)) {
+    if (!I->f_half_tried && !I->persistent_fp64 && cp::fused_wants_half(a.n, I->csr.max_width)) {
         I->f_half_tried = true;
         cp::HalfK& h = a.half;
         const size_t nodes = 32 * (size_t)I->csr.n_slices;
-        const auto room = [I](auto*& p, size_t count) {
-            try {
-                p = I->alloc<std::remove_reference_t<decltype(*p)>>(count);
-            } catch (const Error&) {
-                (void)cudaGetLastError();
-                return false;
-            }
-            return true;
-        };
-        int *widths = nullptr, most[2];
-        if (!room(widths, 2) || !room(h.width, I->csr.n_slices)) return;
-        CP_CUDA(cudaMemsetAsync(widths, 0, 2 * sizeof(int), I->s()));
-        cp::fused_half_widths(a, widths, I->s());
-        CP_CUDA(cudaMemcpyAsync(most, widths, sizeof(most), cudaMemcpyDeviceToHost, I->s()));
-        CP_CUDA(cudaStreamSynchronize(I->s()));
-        h.u = most[0];
-        h.l = most[1];
-        if (!room(h.ucol, nodes * h.u) || !room(h.low, nodes * std::max(h.l, 1)) || !room(h.val, 2 * nodes * h.u)) return;
-        CP_CUDA(cudaMemsetAsync(h.val, 0, 2 * sizeof(double2) * nodes * h.u, I->s()));
-        cp::fused_half_columns(a, I->s());
-        I->f_half = h;
+        int* widths = I->alloc_if_room<int>(2);
+        int most[2] = {0, 0};
+        h.width = I->alloc_if_room<unsigned short>(I->csr.n_slices);
+        if (widths && h.width) {
+            CP_CUDA(cudaMemsetAsync(widths, 0, 2 * sizeof(int), I->s()));
+            cp::fused_half_widths(a, widths, I->s());
+            CP_CUDA(cudaMemcpyAsync(most, widths, sizeof(most), cudaMemcpyDeviceToHost, I->s()));
+            CP_CUDA(cudaStreamSynchronize(I->s()));
+            h.u = most[0];
+            h.l = most[1];
+            h.ucol = I->alloc_if_room<int>(nodes * h.u);
+            if (h.ucol) h.low = I->alloc_if_room<unsigned int>(nodes * h.l);
+            if (h.low) h.val = I->alloc_if_room<double2>(2 * nodes * h.u);
+        }
+        I->release(widths, 2);
+        if (h.val) {
+            CP_CUDA(cudaMemsetAsync(h.val, 0, 2 * sizeof(double2) * nodes * h.u, I->s()));
+            cp::fused_half_columns(a, I->s());
+            I->f_half = h;
+        } else {  // what did fit is given back
+            I->release(h.width, I->csr.n_slices);
+            I->release(h.ucol, nodes * h.u);
+            I->release(h.low, nodes * h.l);
+        }
     }
     a.half = I->f_half;
 }
@@ -330,27 +333,39 @@ cp::FusedArgs fused_args(cp_instance* I, int precond) {
 }
 
 // The on-chip CG's plan of this instance, built on first use; false when the
-// instance does not fit.
+// instance does not fit or the device has no room for the plan.
 bool chip_ready(cp_instance* I) {
     if (!I->on_chip) return false;
     if (I->chip_planned) return I->chip.ctas > 0;
     I->chip_planned = 1;
     for (const bool grid : {false, true}) {
         const cp::ChipShape sh = cp::chip_shape(I->n_nodes, I->csr.max_width, I->sms(), grid);
-        if (sh.ctas == 0) continue;
-        void* mem = I->alloc<unsigned char>(cp::chip_plan_bytes(sh, I->n_nodes));
-        cp::chip_build_plan(I->chip, sh, mem, I->n_nodes, I->mesh.xy, I->csr.slice_ptr, I->csr.scol, I->sms(), I->s());
-        if (I->chip.ctas == 0) continue;
+        if (!cp::instance_chip_plan(I, I->chip, sh, true)) continue;
         if (grid) {
             I->chip_ll_bytes = cp::chip_ll_bytes(sh);
-            I->chip_ll = I->alloc<unsigned char>(I->chip_ll_bytes);
-            I->chip_seq = I->alloc<unsigned int>(1);
+            I->chip_ll = I->alloc_if_room<unsigned char>(I->chip_ll_bytes);
+            I->chip_seq = I->alloc_if_room<unsigned int>(1);
+            if (!I->chip_ll || !I->chip_seq) {
+                I->release(I->chip_ll, I->chip_ll_bytes);
+                I->release(I->chip_seq, 1);
+                I->release(I->chip.mem, cp::chip_plan_bytes(sh, I->n_nodes));
+                I->chip.ctas = 0;
+                continue;
+            }
             CP_CUDA(cudaMemsetAsync(I->chip_ll, 0, I->chip_ll_bytes, I->s()));
             CP_CUDA(cudaMemsetAsync(I->chip_seq, 0, sizeof(unsigned int), I->s()));
         }
         break;
     }
     return I->chip.ctas > 0;
+}
+
+// The same for the mixed mode, which keeps u from before the linear solve.
+bool chip_ready_mixed(cp_instance* I) {
+    if (!chip_ready(I) || I->mix_tried) return chip_ready(I) && I->mix_u0;
+    I->mix_tried = true;
+    I->mix_u0 = I->alloc_if_room<double2>(I->n_nodes);
+    return I->mix_u0 != nullptr;
 }
 
 template <typename T>
@@ -579,9 +594,8 @@ void recycle_after(cp_instance* I, int m) {
 // began, the solve starts over from the same u with the two-kernel loop.
 void cg_mixed(cp_instance* I, double eps, double inner_tol, long long max_iter, long long* inner_total,
               long long* fp64_spmv, double* rel_res, int precond = 0) {
-    if (chip_ready(I)) {
+    if (chip_ready_mixed(I)) {
         const size_t ub = sizeof(double2) * (size_t)I->n_nodes;
-        if (!I->mix_u0) I->mix_u0 = I->alloc<double2>(I->n_nodes);
         CP_CUDA(cudaMemcpyAsync(I->mix_u0, I->u, ub, cudaMemcpyDeviceToDevice, I->s()));
         cp::ChipArgs<float> a = chip_args<float>(I, inner_tol * inner_tol, max_iter, precond);
         a.relative_to_r0 = 1;
@@ -633,6 +647,19 @@ void cp::instance_prepare_mixed(cp_instance* I, int precond) {
         CP_CUDA(cudaMemsetAsync(I->rec32b, 0, sizeof(float4) * I->n_nodes, I->s()));
     }
     if (precond) (void)I->cg_args<float>(1);  // allocates minv32 once
+}
+
+bool cp::instance_chip_plan(cp_instance* I, cp::ChipPlan& plan, const cp::ChipShape& sh, bool for_solve) {
+    if (sh.ctas == 0) return false;
+    const size_t nb = cp::chip_plan_bytes(sh, I->n_nodes);
+    plan.mem = I->alloc_if_room<unsigned char>(nb);
+    uint2* scratch = plan.mem ? I->alloc_if_room<uint2>(2 * (size_t)I->n_nodes) : nullptr;
+    if (scratch)
+        cp::chip_build_plan(plan, sh, scratch, I->n_nodes, I->mesh.xy, I->csr.slice_ptr, I->csr.scol, I->sms(), I->s(),
+                            for_solve);
+    I->release(scratch, 2 * (size_t)I->n_nodes);
+    if (plan.ctas == 0) I->release(plan.mem, nb);
+    return plan.ctas > 0;
 }
 
 // ------------------------------------------------------------------ C ABI --
@@ -751,6 +778,7 @@ CP_API int cp_instance_create(cp_context* ctx, const cp_mesh_view* mv, const cp_
         I->on_chip = std::strcmp(g, "cluster") == 0;
     }
     if (const char* g = std::getenv("CUPLAST_TEST_BARRIER_NS")) I->test_barrier_ns = std::strtoull(g, nullptr, 10);
+    if (const char* g = std::getenv("CUPLAST_TEST_NO_ROOM")) I->test_room = std::atoi(g);
     int rc = guarded(ctx, [&] {
         CP_CHECK(mv->node_count > 0 && mv->node_xy, CP_ERR_INVALID, "mesh: no nodes");
         CP_CHECK(mv->count3 >= 0 && mv->count4 >= 0 && mv->count8 >= 0 &&
@@ -1059,7 +1087,7 @@ CP_API int cp_solve(cp_instance* I, const cp_solve_opts* opts, cp_solve_report* 
                 if (!boost && o.adaptive_cg == 2 && rel_err > o.outer_tol)
                     eps = std::max(o.cg_tol, rule2_factor() * rel_err);
                 // the on-chip CG rounds K to FP32 as it loads it
-                assemble(I, prec == CP_PREC_MIXED && chip_ready(I) ? CP_PREC_FP64 : prec);
+                assemble(I, prec == CP_PREC_MIXED && chip_ready_mixed(I) ? CP_PREC_FP64 : prec);
                 // the multigrid graph loop and the on-chip CG leave their scalars
                 // for after the update: one wait of the host per outer iteration
                 const bool mg_deferred = prec == CP_PREC_FP64 && o.precond == 2 && I->use_graph;

@@ -1441,10 +1441,10 @@ void plan_bchip(cp_instance* I) {
         sh.npt = 2;
         sh.wmax = I->csr.max_width;
         if (sh.spc > 2 * kChipWarps) continue;
-        void* mem = I->alloc<unsigned char>(cp::chip_plan_bytes(sh, I->n_nodes));
-        cp::chip_build_plan(I->bchip, sh, mem, I->n_nodes, I->mesh.xy, I->csr.slice_ptr, I->csr.scol, I->sms(), I->s(),
-                            false);
-        if (I->bchip.ctas > 0 && bchip_smem(I->bchip) > kBChipSmem) I->bchip.ctas = 0;
+        if (cp::instance_chip_plan(I, I->bchip, sh, false) && bchip_smem(I->bchip) > kBChipSmem) {
+            I->bchip.ctas = 0;
+            I->release(I->bchip.mem, cp::chip_plan_bytes(sh, I->n_nodes));
+        }
         return;
     }
 }

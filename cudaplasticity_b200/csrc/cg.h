@@ -123,6 +123,7 @@ struct ChipPlan {
     bool grid = false;
     int ctas = 0, spc = 0, npt = 1, wmax = 0;
     int halo_cap = 0;                // most halo nodes of a CTA (rounded up)
+    unsigned char* mem = nullptr;    // chip_plan_bytes() bytes that hold the following
     int* order = nullptr;            // per slot (CTA, thread): its node, or -1
     unsigned short* lidx = nullptr;  // per block of a slot's row: index of its column in the CTA's U
     int* halo = nullptr;             // per CTA: the slots of its halo nodes
@@ -159,9 +160,10 @@ ChipShape chip_shape(int n, int wmax, int sm_count, bool grid);
 size_t chip_plan_bytes(const ChipShape& s, int n);
 size_t chip_ll_bytes(const ChipShape& s);
 void chip_ll_carve(const ChipPlan& p, void* mem, uint4** rec, uint4** part, uint4** step);
-// for_solve: checks that k_chip can run the plan (a batch brings its own kernel).
-void chip_build_plan(ChipPlan& p, const ChipShape& s, void* mem, int n, const double2* xy, const int* slice_ptr,
-                     const int* scol, int sm_count, cudaStream_t st, bool for_solve = true);
+// In p.mem; scratch: 2 n pairs. for_solve: checks that k_chip can run the plan
+// (a batch brings its own kernel).
+void chip_build_plan(ChipPlan& p, const ChipShape& s, uint2* scratch, int n, const double2* xy, const int* slice_ptr,
+                     const int* scol, int sm_count, cudaStream_t st, bool for_solve);
 template <typename T>
 void chip_launch(const ChipArgs<T>& a, cudaStream_t s);
 

@@ -651,7 +651,7 @@ void chip_ll_carve(const ChipPlan& p, void* mem, uint4** rec, uint4** part, uint
 }
 
 // Builds the plan on the device; plan.ctas = 0 when the instance does not fit.
-void chip_build_plan(ChipPlan& p, const ChipShape& s, void* mem, int n, const double2* xy, const int* slice_ptr,
+void chip_build_plan(ChipPlan& p, const ChipShape& s, uint2* scratch, int n, const double2* xy, const int* slice_ptr,
                      const int* scol, int sm_count, cudaStream_t st, bool for_solve) {
     const size_t slots = chip_slots(s);
     p.grid = s.grid;
@@ -659,15 +659,13 @@ void chip_build_plan(ChipPlan& p, const ChipShape& s, void* mem, int n, const do
     p.npt = s.npt;
     p.wmax = s.wmax;
     p.ctas = 0;
-    int* ints = static_cast<int*>(mem);
+    int* ints = reinterpret_cast<int*>(p.mem);
     p.order = ints;
     int* slot_of = ints + slots;
     p.halo = slot_of + n;
     p.halo_cnt = p.halo + (size_t)s.ctas * kHaloMax;
     p.lidx = reinterpret_cast<unsigned short*>(p.halo_cnt + s.ctas);
     p.pub = reinterpret_cast<unsigned char*>(p.lidx + slots * s.wmax);
-    uint2* scratch = nullptr;
-    CP_CUDA(cudaMallocAsync(&scratch, 2 * sizeof(uint2) * (size_t)n, st));
     CP_CUDA(cudaMemsetAsync(p.pub, 0, slots, st));
     constexpr int order_smem = kDigits * kOrderThreads * (int)sizeof(unsigned int);
     CP_CUDA(cudaFuncSetAttribute(k_chip_order, cudaFuncAttributeMaxDynamicSharedMemorySize, order_smem));
@@ -676,7 +674,6 @@ void chip_build_plan(ChipPlan& p, const ChipShape& s, void* mem, int n, const do
     k_chip_plan<<<s.ctas, kPlanThreads, 2 * sizeof(unsigned int) * (slots / 32), st>>>(
         (int)slots, s.spc * 32, s.wmax, slice_ptr, scol, p.order, slot_of, p.lidx, p.halo, p.halo_cnt, p.pub);
     CP_CUDA(cudaGetLastError());
-    CP_CUDA(cudaFreeAsync(scratch, st));
     std::vector<int> cnt(s.ctas);
     CP_CUDA(cudaMemcpyAsync(cnt.data(), p.halo_cnt, sizeof(int) * s.ctas, cudaMemcpyDeviceToHost, st));
     CP_CUDA(cudaStreamSynchronize(st));

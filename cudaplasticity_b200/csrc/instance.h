@@ -63,6 +63,9 @@ struct cp_instance {
     // never released, so every wait runs out and the solve ends with
     // CP_ERR_TIMEOUT
     unsigned long long test_barrier_ns = 0;
+    // CUPLAST_TEST_NO_ROOM=<k> (tests of the solves' forms without room): the
+    // k-th alloc_if_room and all after it find none (-1)
+    int test_room = 0;
     bool on_chip = true;           // the on-chip CG when the instance fits (CUPLAST_FP64_CG other than cluster: off)
     double2* pred_u = nullptr;     // level predictor (cp_solve_opts.predict): the last level's u and psi
     double* pred_psi = nullptr;
@@ -78,6 +81,7 @@ struct cp_instance {
     unsigned char* chip_ll = nullptr;  // its exchange buffers (grid form)
     size_t chip_ll_bytes = 0;
     unsigned int* chip_seq = nullptr;
+    bool mix_tried = false;
     double2* mix_u0 = nullptr;         // mixed mode on chip: u before the linear solve
     double2 *f_r = nullptr, *f_w = nullptr, *f_p = nullptr, *f_kp = nullptr, *f_g = nullptr;
     double* f_partials = nullptr;
@@ -113,6 +117,32 @@ struct cp_instance {
         return static_cast<T*>(p);
     }
 
+    // For what a solve can do without: null where the device has no room.
+    template <typename T>
+    T* alloc_if_room(size_t count) {
+        void* p = nullptr;
+        const size_t nb = std::max<size_t>(count, 1) * sizeof(T);
+        if (test_room > 0 && --test_room == 0) test_room = -1;
+        const cudaError_t e = test_room < 0 ? cudaErrorMemoryAllocation : cudaMallocAsync(&p, nb, ctx->stream);
+        if (e == cudaErrorMemoryAllocation) {
+            if (test_room >= 0) (void)cudaGetLastError();
+            return nullptr;
+        }
+        CP_CUDA(e);
+        allocs.push_back(p);
+        bytes += nb;
+        return static_cast<T*>(p);
+    }
+    // Gives back what alloc or alloc_if_room returned for count (or null).
+    template <typename T>
+    void release(T*& p, size_t count) {
+        if (!p) return;
+        allocs.erase(std::find(allocs.begin(), allocs.end(), (void*)p));
+        bytes -= std::max<size_t>(count, 1) * sizeof(T);
+        CP_CUDA(cudaFreeAsync(p, ctx->stream));
+        p = nullptr;
+    }
+
     cudaStream_t s() const { return ctx->stream; }
     int sms() const { return ctx->sm_count; }
 
@@ -126,4 +156,8 @@ namespace cp {
 // instance: FP32 values and recurrence vectors, and with precond the FP32
 // block-Jacobi vectors. Stream-ordered on the instance's context stream.
 void instance_prepare_mixed(cp_instance* I, int precond);
+// Builds a plan of the on-chip CG in memory of the instance's; false, with
+// nothing kept, where it does not fit or the device has no room. for_solve: as
+// chip_build_plan.
+bool instance_chip_plan(cp_instance* I, ChipPlan& plan, const ChipShape& sh, bool for_solve);
 }  // namespace cp

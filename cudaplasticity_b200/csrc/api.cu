@@ -267,21 +267,21 @@ void fused_half(cp_instance* I, cp::FusedArgs& a) {
         I->f_half_tried = true;
         cp::HalfK& h = a.half;
         const size_t nodes = 32 * (size_t)I->csr.n_slices;
-        int* widths = I->alloc_if_room<int>(2);
-        int most[2] = {0, 0};
+        cp::HalfCount* d_count = I->alloc_if_room<cp::HalfCount>(1);
+        cp::HalfCount count{};
         h.width = I->alloc_if_room<unsigned short>(I->csr.n_slices);
-        if (widths && h.width) {
-            CP_CUDA(cudaMemsetAsync(widths, 0, 2 * sizeof(int), I->s()));
-            cp::fused_half_widths(a, widths, I->s());
-            CP_CUDA(cudaMemcpyAsync(most, widths, sizeof(most), cudaMemcpyDeviceToHost, I->s()));
+        if (d_count && h.width) {
+            CP_CUDA(cudaMemsetAsync(d_count, 0, sizeof(count), I->s()));
+            cp::fused_half_widths(a, d_count, I->s());
+            CP_CUDA(cudaMemcpyAsync(&count, d_count, sizeof(count), cudaMemcpyDeviceToHost, I->s()));
             CP_CUDA(cudaStreamSynchronize(I->s()));
-            h.u = most[0];
-            h.l = most[1];
-            h.ucol = I->alloc_if_room<int>(nodes * h.u);
+            h.u = count.u;
+            h.l = count.l;
+            if (cp::fused_half_pays(count, a.n)) h.ucol = I->alloc_if_room<int>(nodes * h.u);
             if (h.ucol) h.low = I->alloc_if_room<unsigned int>(nodes * h.l);
             if (h.low) h.val = I->alloc_if_room<double2>(2 * nodes * h.u);
         }
-        I->release(widths, 2);
+        I->release(d_count, 1);
         if (h.val) {
             CP_CUDA(cudaMemsetAsync(h.val, 0, 2 * sizeof(double2) * nodes * h.u, I->s()));
             cp::fused_half_columns(a, I->s());

@@ -55,15 +55,21 @@ struct CgArgs {
 // Time limit of every wait between CTAs (an exchange takes microseconds).
 constexpr unsigned long long kWaitNs = 2000000000ull;
 
-// The upper half of K for cg_fused.cu's iterations: per slice of 32 nodes, up
-// to u blocks right of the diagonal (block 0 is the diagonal one) and up to l
-// left of it, in slots of the slice's widest row.
+// The upper half of K for cg_fused.cu's iterations: per slice of 32 nodes, u
+// slots of the diagonal block and of those right of it, and l of those left of
+// it, as many in every slice as the mesh's widest row takes.
 struct HalfK {
     int u = 0, l = 0;
     unsigned short* width = nullptr;  // per slice: upper blocks | lower blocks << 8
     int* ucol = nullptr;              // per upper slot: its column (the node itself: padding)
     unsigned int* low = nullptr;      // per lower slot: its column and its mirror's upper slot
     double2* val = nullptr;           // per upper slot: the block, rewritten by every solve's start; null: not in use
+};
+
+// Of a numbering: HalfK's u and l, and the slices whose rows are all within the
+// iterations' straight-line code.
+struct HalfCount {
+    int u, l, straight;
 };
 
 // The single-launch FP64 iteration of cg_fused.cu.
@@ -92,11 +98,12 @@ struct FusedArgs {
     unsigned int barrier_skew = 0;
 };
 
-// The upper half of K: whether the iterations of an instance read it, its
-// widths (widths: two ints, zero before; a.half.width is written), and, once
-// those are on the host, its columns.
+// The upper half of K: whether the iterations of an instance may read it, its
+// widths (count: zero before; a.half.width is written), whether they do in this
+// numbering, and, once it has its arrays, its columns.
 bool fused_wants_half(int n, int wmax);
-void fused_half_widths(const FusedArgs& a, int* widths, cudaStream_t s);
+bool fused_half_pays(const HalfCount& c, int n);
+void fused_half_widths(const FusedArgs& a, HalfCount* count, cudaStream_t s);
 void fused_half_columns(const FusedArgs& a, cudaStream_t s);
 void fused_launch_start(const FusedArgs& a, double eps2, long long max_iter, cudaStream_t s);
 void fused_launch_iteration(const FusedArgs& a, int parity, cudaStream_t s);

@@ -95,23 +95,42 @@ __device__ __forceinline__ double2 ld_other(const double2* p) {
 
 // ------------------------------------------------- the upper half of K --
 //
-// Above kHalfLeast nodes the iterations read K's upper half alone. A block left
+// Meshes of at least kHalfLeast nodes, numbered along rows, read K's upper half
+// alone in their iterations. A block left
 // of the diagonal is the transpose of its mirror in the row above (K is bitwise
 // symmetric), which the warps nearby read at about the same time: taken from
 // there, out of L2, it leaves 5 of a quad mesh's 9 blocks per node to device
 // memory (482 bytes per node and iteration in place of 614). The solve's first
 // kernel, which reads all of K, writes the upper blocks to slots of their own,
-// so that a mirror's address follows from its row and slot.
-// (99,856 nodes: 20.0 -> 18.9 us; below, the working set lies in L2 anyway.)
-constexpr int kHalfLeast = 100000;
+// as many for every node as the widest row has, so that a mirror's address
+// follows from its row and slot: 8 and 7 words for the generators' quads, 316
+// bytes per node.
+//
+// kHalfLeast: 147,456 nodes 21.2 us with all of K, 21.3 with the half (quads),
+// 20.7 and 21.1 (triangles); 179,776: 26.7, 24.5 and 23.9, 24.5; 197,136: 28.8,
+// 25.7 and 25.6, 24.4; 230,400: 37.4, 29.0 and 31.9, 26.8.
+// kHalfStraight: the share of slices of which no row has more than kChunk
+// blocks on a side. It is 0.95 and more in numberings along rows (rows of 40 to
+// 262,144 nodes), which gain 0.87-0.9 at 1,048,576 nodes. In any other a
+// slice's rows lie differently, and the half loses, by neighbours' records in
+// three arrays and rows with up to 8 blocks on a side: the same rows in random
+// order (share 0.35) 127.9 us with all of K, 136.7 with the half; along a
+// Hilbert curve (0.00) 122.9, 148.5; at random (0.00) 172, 255; 8-node quads
+// (0.00) 93.4 and 93.5 at 460,600 nodes, 180 and 170 at 994,752. At a share of
+// 0.9 a tenth of the worst of these is less than the rest's gain.
+// kHalfWidest: every node takes as many slots as the widest row has.
+constexpr int kHalfLeast = 190000;
+constexpr double kHalfStraight = 0.9;
+constexpr int kHalfWidest = 9;
 constexpr int kLowShift = 27;  // of a lower slot's word: column below, mirror's upper slot above
 constexpr int kHalfMax = 31;
+constexpr int kChunk = 4;      // blocks on a side in the iterations' straight-line code
 
 __device__ __forceinline__ size_t half_at(int w, int sl, int q, int lane) {
     return ((size_t)sl * w + q) * 32 + lane;
 }
 
-__global__ void k_f_half_widths(FusedArgs a, int* widths) {
+__global__ void k_f_half_widths(FusedArgs a, HalfCount* count) {
     CPF_SLICE_LOOP {
         const int n = 32 * sl + lane;
         const int base = a.slice_ptr[sl], wd = (a.slice_ptr[sl + 1] - base) >> 5;
@@ -126,8 +145,9 @@ __global__ void k_f_half_widths(FusedArgs a, int* widths) {
         l = __reduce_max_sync(0xffffffffu, l);
         if (lane == 0) {
             a.half.width[sl] = (unsigned short)(u | l << 8);
-            atomicMax(widths, u);
-            atomicMax(widths + 1, l);
+            atomicMax(&count->u, u);
+            atomicMax(&count->l, l);
+            if (u - 1 <= kChunk && l <= kChunk) atomicAdd(&count->straight, 1);
         }
     }
 }
@@ -360,8 +380,8 @@ __device__ __forceinline__ void iter_body(const FusedArgs& a, int parity, double
 // 27.1 us, 1,049,600 118 -> 101, 1,961,400 210 -> 177, triangles (1,049,600)
 // 110 -> 94, 8-node quads (461,824) 97 -> 95; 99,856 20.0 -> 18.9. (Mirrors
 // found through the slices' offsets instead of in slots of their own take 150
-// us at 1,049,600 nodes; chunks of 3, 3 blocks per SM, 1: 117, 117, 119.)
-constexpr int kChunk = 4;
+// us at 1,049,600 nodes; chunks of 3, 3 blocks per SM, 1: 117, 117, 119.) Below
+// kHalfLeast and for 8-node quads these were measured with the half forced.
 constexpr unsigned int kNoLow = 0xffffffffu;
 
 
@@ -718,8 +738,14 @@ bool fused_wants_half(int n, int wmax) {
     return (e ? e[0] == '1' : n >= kHalfLeast) && n < (1 << kLowShift) && wmax <= kHalfMax && form() == kDefaultForm;
 }
 
-void fused_half_widths(const FusedArgs& a, int* widths, cudaStream_t s) {
-    k_f_half_widths<<<std::min((a.n + kThreads - 1) / kThreads, a.sm_count * 8), kThreads, 0, s>>>(a, widths);
+bool fused_half_pays(const HalfCount& c, int n) {
+    const char* e = std::getenv("CUPLAST_HALF_K");
+    if (e && e[0] == '1') return true;
+    return 32.0 * c.straight >= kHalfStraight * n && c.u <= kHalfWidest && c.l <= kHalfWidest;
+}
+
+void fused_half_widths(const FusedArgs& a, HalfCount* count, cudaStream_t s) {
+    k_f_half_widths<<<std::min((a.n + kThreads - 1) / kThreads, a.sm_count * 8), kThreads, 0, s>>>(a, count);
     CP_CUDA(cudaGetLastError());
 }
 

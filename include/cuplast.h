@@ -203,9 +203,11 @@ CP_API int cp_bench_cg(cp_instance* inst, int precision, int precond, int iters,
  * current state, starts a (block-Jacobi with precond 1) CG from the current
  * uv and runs `iters` iterations as direct launches with CUDA events around
  * each. Outputs the mean duration of one iteration in milliseconds and the
- * algorithmic bytes one iteration moves: the values (above 100,000 nodes of
- * the diagonal blocks and those right of it) and one 4-byte column per 2x2
- * block, and per node the vectors read and written once. Leaves uv changed. */
+ * algorithmic bytes one iteration moves: the values (of the diagonal blocks
+ * and those right of it alone where the iterations read K's upper half: meshes
+ * of 190,000 nodes and more that are numbered along rows) and one 4-byte column
+ * per 2x2 block, and per node the vectors read and written once. Leaves uv
+ * changed. */
 CP_API int cp_bench_cg_fused(cp_instance* inst, int precond, int iters, double* ms_iter, double* bytes_iter);
 /* Measurement entry point: runs the assembly (fillGlobalStiffness) `iters`
  * times as direct launches with CUDA events around each, from the current

@@ -23,8 +23,9 @@
 // every (instance, tile) pair. Three persistent kernels walk that list, each
 // acting only on the tiles whose instance is in one of its phases:
 //   k_batch_cg    RES (FP64 residual), W (w = K u), ITER (one CG iteration)
-//   k_batch_chip  the three together, as phase CHIP, for instances of up to
-//                 12,288 nodes: one cluster each (not by tiles)
+//   k_batch_chip  the three together, as phase CHIP, for instances that a
+//                 cluster holds (12,288 nodes of 4-node meshes): one cluster
+//                 each (not by tiles)
 //   k_batch_asm   ASM (FP64 + FP32 values of K, node gather, no atomics)
 //   k_batch_elem  LEVEL, UPD (strain / stress / secant / exit norm),
 //                 RELAX (Aitken), PLASTIC
@@ -1426,8 +1427,9 @@ bool bchip_available() {
 }
 
 // The on-chip plan of an instance in a batch, built on its first add: the
-// smallest cluster of 4, 8 or 16 CTAs of up to 768 nodes that holds it
-// (12,288 nodes). CUPLAST_BATCH_CHIP=0 keeps the tile kernels (measurements).
+// smallest cluster of 4, 8 or 16 CTAs of up to 768 nodes whose shared memory
+// holds it (12,288 nodes with rows of up to 9 blocks, 8,192 with the 21 of
+// 8-node quads). CUPLAST_BATCH_CHIP=0 keeps the tile kernels (measurements).
 void plan_bchip(cp_instance* I) {
     if (I->bchip_planned) return;
     I->bchip_planned = 1;
@@ -1441,11 +1443,13 @@ void plan_bchip(cp_instance* I) {
         sh.npt = 2;
         sh.wmax = I->csr.max_width;
         if (sh.spc > 2 * kChipWarps) continue;
-        if (cp::instance_chip_plan(I, I->bchip, sh, false) && bchip_smem(I->bchip) > kBChipSmem) {
-            I->bchip.ctas = 0;
-            I->release(I->bchip.mem, cp::chip_plan_bytes(sh, I->n_nodes));
-        }
-        return;
+        cp::ChipPlan without_halo;
+        without_halo.spc = sh.spc;
+        without_halo.wmax = sh.wmax;
+        if (bchip_smem(without_halo) > kBChipSmem || !cp::instance_chip_plan(I, I->bchip, sh, false)) continue;
+        if (bchip_smem(I->bchip) <= kBChipSmem) return;
+        I->bchip.ctas = 0;
+        I->release(I->bchip.mem, cp::chip_plan_bytes(sh, I->n_nodes));
     }
 }
 

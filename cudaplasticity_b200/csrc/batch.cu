@@ -36,7 +36,8 @@
 // tiling, on the grid, or on the other instances in the batch.
 //
 // One CUDA graph drives a run: a WHILE node whose body is
-//   elem x E, asm, cg x C beside chip x 3 (cluster sizes), condition
+//   elem x E, asm, cg x C beside chip x 3 (cluster sizes; in runs with
+//   on-chip instances), condition
 // and every launch advances every instance in a matching phase by one step.
 #include <cuda_runtime.h>
 
@@ -1223,7 +1224,10 @@ struct cp_batch {
     BCtl* h_ctl = nullptr;  // pinned
     int* h_stop = nullptr;  // host-mapped
     int* d_stop = nullptr;
-    cudaGraphExec_t graph = nullptr;
+    // a trip, without and with the launches for on-chip instances; the
+    // listed ones decide which of them a run takes
+    cudaGraphExec_t graph[2] = {nullptr, nullptr};
+    bool chip_run = false;
     int grid_cg = 0, grid_elem = 0, grid_asm = 0;
     float2* d_sink = nullptr;           // autotuner probe output
     unsigned int* d_ptickets = nullptr;  // autotuner probe tickets (one per slot)
@@ -1263,6 +1267,13 @@ int default_tile(int bucket) {
     return bucket < 6 ? 4 : (bucket < 9 ? 8 : 16);
 }
 
+void drop_graphs(cp_batch* b) {
+    for (cudaGraphExec_t& g : b->graph) {
+        if (g) cudaGraphExecDestroy(g);
+        g = nullptr;
+    }
+}
+
 void ensure_tiles(cp_batch* b, int need) {
     if (need <= b->tiles_cap) return;
     int nc = std::max(need, 2 * b->tiles_cap);
@@ -1274,10 +1285,7 @@ void ensure_tiles(cp_batch* b, int need) {
     CP_CUDA(cudaMallocHost(&b->h_tiles, sizeof(int4) * (size_t)nc));
     b->tiles_cap = nc;
     // the graph holds the work-list pointer: rebuild it
-    if (b->graph) {
-        cudaGraphExecDestroy(b->graph);
-        b->graph = nullptr;
-    }
+    drop_graphs(b);
 }
 
 int tiles_of(const BDesc& d, int S) {
@@ -1370,7 +1378,7 @@ void launch_body(cp_batch* b, cudaStream_t s) {
     else
         k_batch_asm<false><<<b->grid_asm, kThreads, b->asm_smem, s>>>(b->d_desc, b->d_state, b->d_tiles, b->d_ctl,
                                                                       b->o.max_width);
-    if (b->chip_ok) {
+    if (b->chip_run) {
         CP_CUDA(cudaEventRecord(b->fork, s));
         for (int k = kBChipClasses - 1; k >= 0; --k) {
             const int C = 4 << k;
@@ -1394,7 +1402,7 @@ void launch_body(cp_batch* b, cudaStream_t s) {
     }
     for (int k = 0; k < b->o.cg_per_trip; ++k)
         batch_cg_kernel()<<<b->grid_cg, kThreads, 0, s>>>(b->d_desc, b->d_state, b->d_tiles, b->d_ctl);
-    if (b->chip_ok)
+    if (b->chip_run)
         for (int k = 0; k < kBChipClasses; ++k) CP_CUDA(cudaStreamWaitEvent(s, b->join[k], 0));
 }
 
@@ -1490,7 +1498,7 @@ void build_graph(cp_batch* b) {
         cudaGraphDestroy(g);
         CP_CUDA(e);
     }
-    e = cudaGraphInstantiate(&b->graph, g, 0);
+    e = cudaGraphInstantiate(&b->graph[b->chip_run], g, 0);
     cudaGraphDestroy(g);
     CP_CUDA(e);
 }
@@ -1593,7 +1601,7 @@ CP_API int cp_batch_destroy(cp_batch* b) {
     }
     for (int sl : b->listed)
         if (b->inst[sl]) b->inst[sl]->in_batch = false;
-    if (b->graph) cudaGraphExecDestroy(b->graph);
+    drop_graphs(b);
     if (b->d_desc) cudaFree(b->d_desc);
     if (b->d_state) cudaFree(b->d_state);
     if (b->d_tiles) cudaFree(b->d_tiles);
@@ -1646,10 +1654,7 @@ CP_API int cp_batch_add(cp_batch* b, cp_instance* I, const cp_solve_opts* opts, 
             // 8-node element, and capture the trip again with them
             b->q8 = true;
             element_grids<true>(b);
-            if (b->graph) {
-                cudaGraphExecDestroy(b->graph);
-                b->graph = nullptr;
-            }
+            drop_graphs(b);
         }
         instance_prepare_mixed(I, o.precond);
         BDesc d{};
@@ -1738,7 +1743,6 @@ CP_API int cp_batch_launch(cp_batch* b, int until, long long max_trips) {
         CP_CUDA(cudaSetDevice(b->ctx->device));
         const int nt = build_tiles(b, b->listed, true, nullptr, true);
         interleave_tiles(b, nt);
-        if (b->use_graph && !b->graph) build_graph(b);
         BCtl c{};
         c.n_tiles = nt;
         int active = 0, done = 0;
@@ -1760,6 +1764,8 @@ CP_API int cp_batch_launch(cp_batch* b, int until, long long max_trips) {
             c.n_chip[k] = (int)of.size();
             for (int sl : of) b->h_chip[at++] = sl;
         }
+        b->chip_run = at > 0;
+        if (b->use_graph && !b->graph[b->chip_run]) build_graph(b);
         c.active = active;
         c.done = 0;
         c.exit_on_done = until == CP_BATCH_RUN_ANY_DONE ? 1 : 0;
@@ -1777,7 +1783,7 @@ CP_API int cp_batch_launch(cp_batch* b, int until, long long max_trips) {
         b->timed = false;
         if (active > 0) {
             CP_CUDA(cudaEventRecord(b->ev0, s));
-            if (b->use_graph) CP_CUDA(cudaGraphLaunch(b->graph, s));
+            if (b->use_graph) CP_CUDA(cudaGraphLaunch(b->graph[b->chip_run], s));
             else run_direct(b);
             CP_CUDA(cudaEventRecord(b->ev1, s));
             b->timed = true;
@@ -1821,7 +1827,7 @@ CP_API int cp_batch_wait(cp_batch* b, int* active, int* done) {
         const long long trips = b->h_ctl->trips;
         b->trips += trips;
         b->launches +=
-            trips * (long long)(b->o.elem_per_trip + 1 + b->o.cg_per_trip + 1 + (b->chip_ok ? kBChipClasses : 0));
+            trips * (long long)(b->o.elem_per_trip + 1 + b->o.cg_per_trip + 1 + (b->chip_run ? kBChipClasses : 0));
         int a = 0, d = 0;
         for (int sl : b->listed) {
             b->state[sl] = b->h_state[sl];

@@ -4,7 +4,7 @@ import numpy as np
 import pytest
 
 import cudaplasticity_b200 as cp
-from test_gpu_chip import EPS64, ctx, residual  # noqa: F401
+from test_gpu_chip import EPS64, ctx, residual, strip  # noqa: F401
 
 pytestmark = pytest.mark.gpu
 
@@ -39,3 +39,24 @@ def test_8_node_meshes(n_c, n_r, on_chip, ctx, monkeypatch):  # noqa: F811
     # another order of the sums: equal bits only from the same form
     assert np.array_equal(u, tiles) != on_chip
     assert np.linalg.norm(u - tiles) <= 1e-6 * np.linalg.norm(tiles)
+
+
+def test_launches_per_trip(ctx):  # noqa: F811
+    """Runs without an instance on chip leave its launches out (three cluster sizes beside 3 + 1 + 16 + 1 others); a
+    batch takes both kinds of run in turn."""
+    batch, trips, launches = cp.Batch(ctx, max_instances=2), 0, 0
+    for sizes, per_trip in (([(140, 100)], 21), ([(64, 26)], 24), ([(140, 100), (64, 26)], 24), ([(140, 100)], 21)):
+        insts = []
+        for nx, ny in sizes:
+            arrays, rp, mask = strip(nx, ny)
+            insts.append(cp.Instance(ctx, arrays, cp.material(210000.0, 0.3)))
+            insts[-1].set_loads(rp, mask)
+            batch.add(insts[-1], cg_tol=1e-6, outer_tol=1e300, inner_tol=1e-3, max_outer=1, max_cg=20000, precond=1)
+        batch.run()
+        assert [r["status"] for _, _, r in batch.harvest()] == [0] * len(sizes)
+        s = batch.stats()
+        assert s["kernel_launches"] - launches == per_trip * (s["trips"] - trips)
+        trips, launches = s["trips"], s["kernel_launches"]
+        for i in insts:
+            i.close()
+    batch.close()

@@ -95,11 +95,15 @@ __device__ __forceinline__ bool solve_failed(const CgScalars* solve) {
 // 4 blocks per SM (64 registers) for the latency of the gathers, and a grid
 // that fits once, so that the block sums and their fence are paid once per
 // block: 1,048,576 quads with Hollomon hardening, whole call 125 us at 2
-// blocks per SM with Newton's method on pow, 73 now (floor 26: 168 MB).
+// blocks per SM with Newton's method on pow, 73 now (floor 26: 168 MB). With
+// the 8-node element 2 blocks per SM (128 registers): 64 registers spill 656
+// bytes a thread; 639,200 8-node quads, whole call with a linear and a
+// Hollomon diagram 125 and 137 us at 2, 150 and 174 at 1, 162 and 172 at 3, 174
+// and 175 at 4; 576 and 6144 of them 28.7 at each.
 // solve: a linear solve whose outcome the host has not seen yet; where it
 // failed, the elements keep their state.
 template <bool Q8>
-__global__ void __launch_bounds__(kElemThreads, 4) k_update(DevMesh m, MaterialDev M, const double2* __restrict__ u,
+__global__ void __launch_bounds__(kElemThreads, Q8 ? 2 : 4) k_update(DevMesh m, MaterialDev M, const double2* __restrict__ u,
                                                          ElemState st, OuterScalars* sc, double* partials, int aitken,
                                                          int first, const CgScalars* solve) {
     __shared__ double sh[2 * kElemThreads / 32];

@@ -116,6 +116,8 @@ cudaGraphExec_t fused_build_while_graph(const FusedArgs& a, int body_iters, cuda
 // CgScalars.status of an FP32 on-chip solve whose step lost its curvature
 // (internal: never returned to a caller).
 constexpr int CP_ERR_DEGENERATE = 100;
+// Of an on-chip solve that its budget of iterations has cut (internal too).
+constexpr int CP_CHIP_CUT = 101;
 
 // The whole linear solve on chip (cg_chip.cu): one thread-block cluster, or
 // a cooperative grid of up to one CTA per SM.
@@ -151,6 +153,13 @@ struct ChipArgs {
     double eps2 = 0.0, outer_eps2 = -1.0;  // as cg_launch_init
     long long max_iter = 0;
     int relative_to_r0 = 0;
+    // grid form: at most `budget` iterations. A solve that this cuts ends with
+    // CP_CHIP_CUT, its vectors in `state` (r, p, kp, w, u: 5 n pairs of T) and
+    // its last records in the exchange buffers, and another launch with resume
+    // = 1 goes on exactly where it was.
+    long long budget = 0x7fffffffLL;
+    void* state = nullptr;
+    int n = 0, resume = 0;
     // with inc: the solve's increment x - u0 is left there (recycle.h)
     const double2* u0 = nullptr;
     double2* inc = nullptr;

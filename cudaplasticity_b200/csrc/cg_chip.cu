@@ -323,6 +323,14 @@ __global__ void __launch_bounds__(kChipWarps * 32, 1) k_chip(ChipArgs<T> a) {
         v[0] += (double)r[j].x * (double)r[j].x + (double)r[j].y * (double)r[j].y;
         v[1] += bb.x * bb.x + bb.y * bb.y;
         v[2] += r0 * r0 + r1 * r1;
+        if (GRID && a.resume) {
+            const V2* st = static_cast<const V2*>(a.state) + nd;
+            r[j] = st[0];
+            p[j] = st[(size_t)a.n];
+            kp[j] = st[2 * (size_t)a.n];
+            wv[j] = st[3 * (size_t)a.n];
+            u[j] = st[4 * (size_t)a.n];
+        }
     }
     // ---- halo: thread nthr - 1 - tid takes the first halo nodes, so that the
     // warps that wait for the sums have few of them; past the last halo node a
@@ -331,12 +339,24 @@ __global__ void __launch_bounds__(kChipWarps * 32, 1) k_chip(ChipArgs<T> a) {
     const int* hl = P.halo + (size_t)rank * kHaloMax;
     const unsigned int ha = hc > 0 ? comm.halo_at(hl[min(h0, hc - 1)]) : 0u;
     V2 hr[3];
-    comm.seq = GRID ? *a.seq : 0u;
+    if constexpr (GRID) {
+        comm.seq = *a.seq;
+        comm.par = comm.seq & 1u;  // by the number, so that a solve that goes on finds its records
+    }
     // ---- the scalars of the solve: warp 0 (grid: of the adding CTA)
     double rr = 0.0, rho = 0.0, rho_inv = 0.0, bnorm2 = 0.0, res64 = 0.0, normB_inv = 0.0;
     int status = 0, converged = 0, lin_done = 0;
     int iter = 0;
-    const int max_iter = (int)(a.max_iter < 0x7fffffffLL ? a.max_iter : 0x7fffffffLL);
+    if (adder && a.resume) {
+        rho = a.sc->rho;
+        bnorm2 = a.sc->bb;
+        res64 = a.sc->res64;
+        normB_inv = a.sc->normB_inv;
+        iter = a.sc->iter;
+    }
+    const long long most = 0x7fffffffLL;
+    const int max_iter = (int)(a.max_iter < most ? a.max_iter : most);
+    const int cap = GRID ? (int)min((long long)max_iter, iter + a.budget) : max_iter;
     comm.init();
 
     auto apply_m = [&](int j, V2 q) { return make2<V2>(mi0[j] * q.x + mi1[j] * q.y, mi1[j] * q.x + mi2[j] * q.y); };
@@ -352,7 +372,7 @@ __global__ void __launch_bounds__(kChipWarps * 32, 1) k_chip(ChipArgs<T> a) {
         rho = g;
         rho_inv = den;  // the loop top replaces it
         iter += 1;
-        const int go = (int)(rr * normB_inv > a.eps2) & (int)(iter < max_iter) & (int)(den > 0.0) & (int)(g > 0.0);
+        const int go = (int)(rr * normB_inv > a.eps2) & (int)(iter < cap) & (int)(den > 0.0) & (int)(g > 0.0);
         return {an, b2, go};
     };
     auto decide_first = [&](const double* tot) -> Step {
@@ -387,7 +407,7 @@ __global__ void __launch_bounds__(kChipWarps * 32, 1) k_chip(ChipArgs<T> a) {
                 // in FP32 the step may degenerate before the residual does: the
                 // solve ends there and the caller takes the FP64 residual
                 status = sizeof(T) == 4 ? CP_ERR_DEGENERATE : CP_ERR_BREAKDOWN;
-            }
+            } else if (iter >= cap) status = CP_CHIP_CUT;
             if (!(rr == rr)) status = CP_ERR_BREAKDOWN;
         }
         sc->rr = rr;
@@ -438,7 +458,7 @@ __global__ void __launch_bounds__(kChipWarps * 32, 1) k_chip(ChipArgs<T> a) {
             comm.lead(decide_now);
             return cs.step.go != 0 && !comm.failed;
         };
-        if (lead(decide_init) && lead(decide_first)) {
+        if (a.resume || (lead(decide_init) && lead(decide_first))) {
             do {
                 rho_inv = __drcp_rn(rho);
             } while (lead(decide));
@@ -447,20 +467,30 @@ __global__ void __launch_bounds__(kChipWarps * 32, 1) k_chip(ChipArgs<T> a) {
         return;
     }
     // ---- (r, r), (b, b), and u to the neighbours
-    exchange(decide_init);
-    fill_u((T)0, (T)0);
-    bool go = cs.step.go != 0 && !comm.failed;
-    if (go) {
-        // ---- first step: w = K u; gamma = (r, u), delta = (w, u)
-        v[0] = v[1] = v[2] = 0.0;
-#pragma unroll
-        for (int j = 0; j < NPT; ++j) {
-            wv[j] = rows.gather(j);
-            v[0] += (double)r[j].x * (double)u[j].x + (double)r[j].y * (double)u[j].y;
-            v[1] += (double)wv[j].x * (double)u[j].x + (double)wv[j].y * (double)u[j].y;
-        }
-        exchange(decide_first);
+    bool go = true;
+    if (GRID && a.resume) {
+        // the last exchange's records are where they were, and the step that
+        // it made is in sc
+        if (tid == 0) cs.step = {a.sc->alpha, a.sc->beta, 1};
+        if (h_min < hc) comm.read_halo(ha, hr);
+        go = __syncthreads_or(comm.failed ? 1 : 0) == 0;
+        comm.failed = !go;
+    } else {
+        exchange(decide_init);
+        fill_u((T)0, (T)0);
         go = cs.step.go != 0 && !comm.failed;
+        if (go) {
+            // ---- first step: w = K u; gamma = (r, u), delta = (w, u)
+            v[0] = v[1] = v[2] = 0.0;
+#pragma unroll
+            for (int j = 0; j < NPT; ++j) {
+                wv[j] = rows.gather(j);
+                v[0] += (double)r[j].x * (double)u[j].x + (double)r[j].y * (double)u[j].y;
+                v[1] += (double)wv[j].x * (double)u[j].x + (double)wv[j].y * (double)u[j].y;
+            }
+            exchange(decide_first);
+            go = cs.step.go != 0 && !comm.failed;
+        }
     }
     // ---- iterations
     while (go) {
@@ -512,6 +542,14 @@ __global__ void __launch_bounds__(kChipWarps * 32, 1) k_chip(ChipArgs<T> a) {
             if (a.inc) {
                 const double2 b = a.u0[n[j]];
                 a.inc[n[j]] = make_double2(x[j].x - b.x, x[j].y - b.y);
+            }
+            if (GRID && a.state) {
+                V2* st = static_cast<V2*>(a.state) + n[j];
+                st[0] = r[j];
+                st[(size_t)a.n] = p[j];
+                st[2 * (size_t)a.n] = kp[j];
+                st[3 * (size_t)a.n] = wv[j];
+                st[4 * (size_t)a.n] = u[j];
             }
         }
     if (!GRID && rank == 0) finish();

@@ -11,6 +11,7 @@
 
 #include "cg.h"
 #include "internal.h"
+#include "lane_gate.h"
 #include "mg.h"
 #include "recycle.h"
 
@@ -24,6 +25,7 @@ struct cp_context {
     // cp_solve moves to this stream at its next outer iteration, after the
     // current one has drained.
     std::atomic<cudaStream_t> restream{nullptr};
+    cp::LaneGate* gate = nullptr;  // of the solve service whose lane this context is
 };
 
 struct cp_instance {
@@ -81,6 +83,8 @@ struct cp_instance {
     unsigned char* chip_ll = nullptr;  // its exchange buffers (grid form)
     size_t chip_ll_bytes = 0;
     unsigned int* chip_seq = nullptr;
+    bool chip_state_tried = false;
+    double2* chip_state = nullptr;     // vectors of a solve between its turns
     bool mix_tried = false;
     double2* mix_u0 = nullptr;         // mixed mode on chip: u before the linear solve
     double2 *f_r = nullptr, *f_w = nullptr, *f_p = nullptr, *f_kp = nullptr, *f_g = nullptr;

@@ -17,7 +17,8 @@
 // FP64 (and floatBoost) requests take the same admission path but are solved
 // by cp_solve, one request per lane thread; each lane has its own context
 // (stream), so the lanes' solves and the batch run concurrently. A small
-// request's CG occupies one cluster of up to 16 SMs, so several of them share the GPU.
+// request's CG occupies one cluster of up to 16 SMs, so several of them share
+// the GPU; larger ones take turns on it (lane_gate.h).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -95,6 +96,7 @@ struct cp_server {
     cp_server_stats st{};
     size_t inflight_bytes = 0;
     size_t total_mem = 0;
+    cp::LaneGate gate;  // the lanes' turns
 };
 
 namespace {
@@ -214,6 +216,7 @@ void lane(cp_server* s, int k) {
             r = s->lane_q.front();
             s->lane_q.pop_front();
             s->lane_cur[k] = r;
+            s->gate.busy += 1;
             if (!s->lane_streams.empty()) {
                 s->lane_level[k] = -1;
                 relevel(s);
@@ -239,6 +242,7 @@ void lane(cp_server* s, int k) {
         }
         std::lock_guard<std::mutex> lock(s->mu);
         s->lane_cur[k] = nullptr;
+        s->gate.busy -= 1;
         relevel(s);
         s->inflight_bytes -= r->footprint;
         if (rc != CP_OK) {
@@ -264,6 +268,7 @@ void scheduler(cp_server* s) {
             int active = 0, done = 0;
             const int rc = cp_batch_wait(s->batch, &active, &done);
             running = false;
+            s->gate.busy -= 1;
             std::lock_guard<std::mutex> lock(s->mu);
             s->st.busy_seconds += std::chrono::duration<double>(Clock::now() - t_launch).count();
             cp_batch_stats(s->batch, &s->st.trips, nullptr, nullptr);
@@ -322,6 +327,7 @@ void scheduler(cp_server* s) {
         if (active > 0) {
             if (cp_batch_launch(s->batch, CP_BATCH_RUN_ANY_DONE, s->o.trip_quantum) == CP_OK) {
                 running = true;
+                s->gate.busy += 1;
                 t_launch = Clock::now();
                 std::lock_guard<std::mutex> lock(s->mu);
                 s->st.runs += 1;
@@ -399,6 +405,7 @@ void scheduler(cp_server* s) {
                     int a = 0, d = 0;
                     cp_batch_wait(s->batch, &a, &d);
                     running = false;
+                    s->gate.busy -= 1;
                 }
                 for (auto& r : ready) r->status = CP_ERR_CANCELLED;
                 for (auto& r : s->lane_q) {
@@ -449,7 +456,10 @@ CP_API int cp_server_create(const cp_server_opts* opts, cp_server** out) {
     for (int k = 0; rc == CP_OK && k < o.fp64_lanes; ++k) {
         cp_context* c = nullptr;
         rc = cp_context_create(o.device, &c);
-        if (rc == CP_OK) s->lane_ctx.push_back(c);
+        if (rc == CP_OK) {
+            c->gate = &s->gate;
+            s->lane_ctx.push_back(c);
+        }
     }
     s->lane_cur.assign(s->lane_ctx.size(), nullptr);
     {

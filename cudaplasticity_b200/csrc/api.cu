@@ -770,21 +770,38 @@ CP_API int cp_context_synchronize(cp_context* ctx) {
 
 CP_API int cp_instance_footprint(const cp_mesh_view* m, int precision, size_t* bytes) {
     if (!m || !bytes || m->node_count <= 0 || m->count3 < 0 || m->count4 < 0 || m->count8 < 0) return CP_ERR_INVALID;
-    const size_t n = (size_t)m->node_count, ne = (size_t)m->count3 + (size_t)m->count4 + (size_t)m->count8;
-    const size_t incs = 3 * (size_t)m->count3 + 4 * (size_t)m->count4 + 8 * (size_t)m->count8;
-    // upper bound of the neighbour count: the reference's link capacity
-    const size_t nadj = 2 * (size_t)m->count3 + 3 * (size_t)m->count4 + 7 * (size_t)m->count8;
-    const size_t nadj_est = std::min(nadj, incs * 3);
-    const size_t nnz = 4 * (nadj_est + n);
-    size_t b = n * 16 + ne * 16 + (size_t)m->count8 * 16 + incs * (m->count8 ? 12 : 8) + (2 * n + 2) * 4 +
-               nadj_est * 4;                                                   // mesh + structure
-    b += nnz * 8;                                                              // K (FP64)
-    b += n * (16 * 8 + 2);                                                     // u, b, b_full, u_full, r, z, z, q, mask
-    b += ne * 18 * 8;                                                          // element state
-    b += n * 2 * 32;                                                           // (v, z) records, FP64 two-kernel form
-    if (precision != CP_PREC_FP64) b += nnz * 4 + n * 8 * 4 + n * 2 * 16;
-    b += n * 16 * (cp::kRecycleMax + 1);                                       // solution increments (recycle)
-    b += 1 << 20;                                                              // scalars, partials, graphs
+    const size_t n = (size_t)m->node_count, c3 = (size_t)m->count3, c4 = (size_t)m->count4, c8 = (size_t)m->count8;
+    const size_t ne = c3 + c4 + c8, incs = 3 * c3 + 4 * c4 + 8 * c8;
+    // neighbours of all nodes: every pair within an element, those along an
+    // edge shared by two (Euler: nodes + elements edges, holes apart)
+    const size_t nadj = std::min(6 * c3 + 12 * c4 + 56 * c8, (c8 ? 3 : 2) * (n + ne) + 4 * c4 + 32 * c8);
+    // blocks of K, rows padded to their slice's widest (21 and 13 in turn with
+    // 8-node quads, 5 to 9 in a triangle mesh)
+    const size_t blocks = (size_t)((double)(n + nadj) * (c8 || c3 ? 1.4 : 1.25));
+    const int width = c8 ? 24 : 12;
+    const int nodes = (int)std::min<size_t>(n, 1u << 30);
+    size_t b = 16 * n + 16 * (c3 + c4) + 32 * c8 + incs * (c8 ? 12 : 8) + 8 * (n + 1) + 4 * nadj;  // mesh + structure
+    b += 4 * (n / 32 + 2) + 36 * blocks;       // K (FP64), columns
+    b += n * (16 * 8 + 2);                     // u, b, b_full, u_full, r, z, z, q, mask
+    b += ne * 18 * 8;                          // element state
+    b += n * 16 * (cp::kRecycleMax + 1);       // solution increments (recycle)
+    b += 16 * n + 8 * ne;                      // the last level's u and psi (predict)
+    // The linear solve: on chip, its plan, exchange buffers and vectors
+    // between turns; else the vectors of the one-launch loop (of the two-kernel
+    // loop fewer) and the upper half of K at its widest.
+    size_t chip = 0;
+    for (const bool grid : {false, true}) {
+        const cp::ChipShape sh = cp::chip_shape(nodes, width, cp::kB200Sms, grid);
+        if (sh.ctas > 0) chip = std::max(chip, cp::chip_plan_bytes(sh, nodes) + cp::chip_ll_bytes(sh) + 80 * n);
+    }
+    const size_t loop = n * (160 + 32) + cp::fused_half_bytes(nodes);
+    b += std::max(chip, loop);
+    if (precision != CP_PREC_FP64) {
+        b += 16 * blocks + n * (56 + 16 + 16);         // K (FP32), vectors, block-Jacobi, u before the solve
+        b += 96 * n + 2 * (n + ne);                    // the batch's vectors, records and sums
+        b += cp::batch_plan_bytes(nodes, width);       // and its on-chip plan
+    }
+    b += 1 << 20;                                      // scalars, partials, graphs
     *bytes = b;
     return CP_OK;
 }

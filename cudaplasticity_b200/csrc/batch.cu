@@ -1434,6 +1434,17 @@ bool bchip_available() {
     return true;
 }
 
+// Of cluster size k; ctas = 0: too few threads.
+cp::ChipShape bchip_shape(int n_slices, int wmax, int k) {
+    const int C = 4 << k, per = (n_slices + C - 1) / C;
+    cp::ChipShape sh;
+    sh.spc = (per + 1) / 2 * 2;  // two nodes per thread
+    sh.npt = 2;
+    sh.wmax = wmax;
+    sh.ctas = sh.spc > 2 * kChipWarps ? 0 : C;
+    return sh;
+}
+
 // The on-chip plan of an instance in a batch, built on its first add: the
 // smallest cluster of 4, 8 or 16 CTAs of up to 768 nodes whose shared memory
 // holds it (12,288 nodes with rows of up to 9 blocks, 8,192 with the 21 of
@@ -1444,13 +1455,8 @@ void plan_bchip(cp_instance* I) {
     const char* e = std::getenv("CUPLAST_BATCH_CHIP");
     if (e && e[0] == '0') return;
     for (int k = 0; k < kBChipClasses; ++k) {
-        const int C = 4 << k, per = (I->csr.n_slices + C - 1) / C;
-        cp::ChipShape sh;
-        sh.ctas = C;
-        sh.spc = (per + 1) / 2 * 2;  // two nodes per thread
-        sh.npt = 2;
-        sh.wmax = I->csr.max_width;
-        if (sh.spc > 2 * kChipWarps) continue;
+        const cp::ChipShape sh = bchip_shape(I->csr.n_slices, I->csr.max_width, k);
+        if (sh.ctas == 0) continue;
         cp::ChipPlan without_halo;
         without_halo.spc = sh.spc;
         without_halo.wmax = sh.wmax;
@@ -1518,6 +1524,15 @@ cp_solve_report report_of(const BState& S) {
 }
 
 }  // namespace
+
+size_t cp::batch_plan_bytes(int n, int wmax) {
+    size_t most = 0;
+    for (int k = 0; k < kBChipClasses; ++k) {
+        const cp::ChipShape sh = bchip_shape((n + 31) / 32, wmax, k);
+        if (sh.ctas > 0) most = std::max(most, cp::chip_plan_bytes(sh, n));
+    }
+    return most;
+}
 
 extern "C" {
 

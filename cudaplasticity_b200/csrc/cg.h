@@ -103,6 +103,7 @@ struct FusedArgs {
 // numbering, and, once it has its arrays, its columns.
 bool fused_wants_half(int n, int wmax);
 bool fused_half_pays(const HalfCount& c, int n);
+size_t fused_half_bytes(int n);  // its arrays at their largest
 void fused_half_widths(const FusedArgs& a, HalfCount* count, cudaStream_t s);
 void fused_half_columns(const FusedArgs& a, cudaStream_t s);
 void fused_launch_start(const FusedArgs& a, double eps2, long long max_iter, cudaStream_t s);
@@ -182,6 +183,8 @@ void chip_build_plan(ChipPlan& p, const ChipShape& s, uint2* scratch, int n, con
                      const int* scol, int sm_count, cudaStream_t st, bool for_solve);
 template <typename T>
 void chip_launch(const ChipArgs<T>& a, cudaStream_t s);
+// The largest plan of an instance in a batch (batch.cu).
+size_t batch_plan_bytes(int n, int wmax);
 
 template <typename T>
 void cg_launch_init(const CgArgs<T>& a, const void* valA, bool valA_is_fp64, double eps2, long long max_iter,

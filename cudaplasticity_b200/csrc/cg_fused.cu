@@ -744,6 +744,12 @@ bool fused_half_pays(const HalfCount& c, int n) {
     return 32.0 * c.straight >= kHalfStraight * n && c.u <= kHalfWidest && c.l <= kHalfWidest;
 }
 
+size_t fused_half_bytes(int n) {
+    if (n < kHalfLeast) return 0;
+    const size_t slices = ((size_t)n + 31) / 32;
+    return slices * (32 * kHalfWidest * (sizeof(int) + sizeof(unsigned int) + 2 * sizeof(double2)) + 2);
+}
+
 void fused_half_widths(const FusedArgs& a, HalfCount* count, cudaStream_t s) {
     k_f_half_widths<<<std::min((a.n + kThreads - 1) / kThreads, a.sm_count * 8), kThreads, 0, s>>>(a, count);
     CP_CUDA(cudaGetLastError());

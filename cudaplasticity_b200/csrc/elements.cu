@@ -312,8 +312,8 @@ extern "C" CP_API int cp_secant_update_noalloc(void* stream, const cp_material* 
     es.sxx = d_fields + 4 * ne; es.syy = d_fields + 5 * ne; es.tau = d_fields + 6 * ne; es.sig_i = d_fields + 7 * ne;
     es.table_s = d_fields + 8 * ne;
     es.psi = d_psi; es.E_c = d_E_c; es.nu_c = d_nu_c;
-    const int threads = cp::elem_threads(count4, 148);
-    const int grid = cp::update_grid(count4, 148);  // <= kNoAllocMaxBlocks
+    const int threads = cp::elem_threads(count4, cp::kB200Sms);
+    const int grid = cp::update_grid(count4, cp::kB200Sms);  // <= kNoAllocMaxBlocks
     cp::k_update<false><<<grid, threads, 0, s>>>(m, M, reinterpret_cast<const double2*>(d_uv), es, sc, partials, 0, 0, nullptr);
     if (cudaGetLastError() != cudaSuccess) return CP_ERR_CUDA;
     double host_err = 0.0;

@@ -81,6 +81,8 @@ struct ElemState {
 };
 
 // Device-resident scalars of one linear solve.
+constexpr int kB200Sms = 148;  // where no context says how many SMs there are
+
 struct CgScalars {
     double rr;          // (r, r) of the recurrence residual
     double rho;         // (r, M^-1 r); equals rr without preconditioner

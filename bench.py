@@ -41,6 +41,7 @@ run N independent replicas ("replicas only"); value = solves of all ranks /
 max-over-ranks time.
 """
 import argparse
+import contextlib
 import json
 import os
 import statistics
@@ -1067,6 +1068,21 @@ CG_ONLY_KW = dict(cg_tol=1e-12, outer_tol=1e-9, max_outer=50, max_cg=5_000_000, 
                   inner_tol=1e-3)
 
 
+@contextlib.contextmanager
+def tile_kernels_only():
+    """Instances added to a batch inside run their linear solves in k_batch_cg, also those that a cluster holds (whose
+    iterations move nothing through HBM, and of which a launch makes up to 256)."""
+    old = os.environ.get("CUPLAST_BATCH_CHIP")
+    os.environ["CUPLAST_BATCH_CHIP"] = "0"
+    try:
+        yield
+    finally:
+        if old is None:
+            del os.environ["CUPLAST_BATCH_CHIP"]
+        else:
+            os.environ["CUPLAST_BATCH_CHIP"] = old
+
+
 def cg_kernel_roofline(ctx, n=512, warm_trips=3, trips=10, seed=20261203):
     """Live roofline of the batched CG iteration kernel (k_batch_cg, ITER
     phase): n resident batch-stream instances with tight, non-adaptive linear
@@ -1083,8 +1099,9 @@ def cg_kernel_roofline(ctx, n=512, warm_trips=3, trips=10, seed=20261203):
         inst.set_loads(w["rp"], w["mask"], w["uv"])
         insts.append(inst)
     b = cp.Batch(ctx, max_instances=n)
-    for inst in insts:
-        b.add(inst, levels=1, **CG_ONLY_KW)
+    with tile_kernels_only():
+        for inst in insts:
+            b.add(inst, levels=1, **CG_ONLY_KW)
     b.run(max_trips=warm_trips)
     b.autotune()
     cg0 = [b.progress(s)[2]["cg_iters"] for s in range(n)]
@@ -1132,8 +1149,9 @@ def batched_probe(n, trips):
         inst.set_loads(w["rp"], w["mask"], w["uv"])
         insts.append(inst)
     b = cp.Batch(ctx, max_instances=n)
-    for inst in insts:
-        b.add(inst, levels=1, **CG_ONLY_KW)
+    with tile_kernels_only():
+        for inst in insts:
+            b.add(inst, levels=1, **CG_ONLY_KW)
     b.run(max_trips=3)
     ms = b.autotune()
     t0 = time.perf_counter()

@@ -635,15 +635,16 @@ bool chip_schedulable(const ChipPlan& p, int sm_count) {
 //   cluster: about 13 CTAs, of at least 4 slices. 1024 nodes: 8 CTAs of 4
 //     slices 1.45 us per iteration, 16 of 2 1.9, 3 of 12 1.7; 4160 nodes: 13 of
 //     10 1.74, 11 of 12 1.8 (the whole solve in one cluster with every
-//     record read through distributed shared memory: 4.9 and 5.7). These are
-//     without the records' release, with which the forms taken have 1.47 and
-//     1.80.
+//     record read through distributed shared memory: 4.9 and 5.7). With the
+//     records' release the forms taken have 1.49 and 1.80.
 //   grid: about 128 CTAs, of at least 8 slices. 16104 nodes: 63 CTAs of 8
 //     slices 3.31 us, 126 of 4 3.7, 42 of 12 3.7 (one launch per iteration,
 //     cg_fused.cu: 10.2); 40200 nodes: 126 of 10 3.71, 105 of 12 3.8 (11.4).
 //     Above 147 CTAs of 12, two nodes per thread: 65536 nodes 86 CTAs of 24
 //     5.98 us (11.9); 99856 nodes 131 of 24 6.09 (16.3). At sizes that both
-//     hold the cluster is the faster one (4160 nodes: 3.2 as a grid).
+//     hold the cluster is the faster one (4160 nodes: 3.2 as a grid). With the
+//     waits limited by time the forms taken have 3.06 (16256 nodes), 3.31 and
+//     5.75.
 ChipShape chip_shape(int n, int wmax, int sm_count, bool grid) {
     const int n_slices = (n + 31) / 32;
     ChipShape s;

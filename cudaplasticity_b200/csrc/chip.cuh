@@ -70,7 +70,9 @@ __device__ __forceinline__ void cluster_wait() {
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-// Two words of (32 bits of data, sequence number).
+// Two words of (32 bits of data, sequence number): a word is its own flag, as in
+// the low-latency protocol of collective libraries (NCCL's LL). What it rests
+// on is that each 8-byte half of a 16-byte access is written and read whole.
 __device__ __forceinline__ uint4 ld_words(const uint4* p) {
     uint4 v;
     asm volatile("ld.volatile.global.v4.u32 {%0, %1, %2, %3}, [%4];"
@@ -100,9 +102,10 @@ __device__ __forceinline__ bool waited(unsigned long long& t0, unsigned long lon
 }
 
 // Polls N word pairs per lane until those of every lane of the warp carry seq;
-// false after `limit` nanoseconds (looked at every 256 rounds). The whole warp takes part, with valid addresses
-// in every lane: left to diverge, a warp of which some lanes polled and some
-// did not took 3700 cycles to come together again.
+// false after `limit` nanoseconds (looked at every 256 rounds). The whole warp
+// takes part, with valid addresses in every lane: left to diverge, a warp of
+// which some lanes polled and some did not took 3700 cycles to come together
+// again.
 template <int N>
 __device__ __forceinline__ bool poll(const uint4* p, size_t stride, unsigned int seq, unsigned long long limit, uint4* c) {
     unsigned long long t0 = 0;
@@ -411,8 +414,8 @@ struct Comm {
 // j nthr + t): the first kRegBlocks blocks of the first RN nodes in registers,
 // the other blocks in shared memory, upper and lower rows apart. WIDE: rows
 // may have more than kRegBlocks blocks; without, the first RN nodes' loops over
-// the rest are left out, for the length of the code: 4160 nodes take 1.74 us per
-// iteration so, 1.85 with them unrolled by 3.
+// the rest are left out, for the length of the code: 4160 nodes took 1.74 us per
+// iteration so, 1.85 with them unrolled by 3 (1.80 now).
 template <typename T, int NPT, int RN, bool WIDE>
 struct ChipRows {
     using V2 = typename Vec2<T>::type;

@@ -245,7 +245,9 @@ void launch_plastic(const DevMesh& m, const MaterialDev& mat, ElemState& st, cud
 // keeps until the process exits.
 namespace {
 
-constexpr int kNoAllocMaxBlocks = 4096;  // one partial-sum slot per block of 256 elements
+// Partial-sum slots. The call's limit, 1,048,576 elements, is one block of 256
+// per slot; the grid takes at most 4 blocks per SM of them.
+constexpr int kNoAllocMaxBlocks = 4096;
 constexpr int kNoAllocScalarBytes = 256;  // cp::OuterScalars, padded
 static_assert(sizeof(cp::OuterScalars) <= kNoAllocScalarBytes, "scalars do not fit the scratch header");
 

@@ -181,7 +181,9 @@ CP_API int cp_cg_solve(cp_instance* inst, double eps, long long max_iter, long l
 CP_API int cp_secant_update(cp_instance* inst, double* rel_err);
 /* Plastic strains: plastDeform (src/PlasticitySolver.cu:1641-1662). */
 CP_API int cp_plastic_strains(cp_instance* inst);
-/* The whole outer loop: solveCUDA (src/PlasticitySolver.cu:469-512). */
+/* The whole outer loop: solveCUDA (src/PlasticitySolver.cu:469-512). Where a
+ * linear solve fails (CP_ERR_BREAKDOWN, CP_ERR_TIMEOUT) the elements' fields are
+ * left as they were before it; the displacements are not. */
 CP_API void cp_solve_opts_default(cp_solve_opts* opts);
 CP_API int cp_solve(cp_instance* inst, const cp_solve_opts* opts, cp_solve_report* report);
 

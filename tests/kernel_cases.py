@@ -8,7 +8,7 @@ Cases (each prints one JSON line with its host-side facts):
   2.1M DOF), R launches (cp_bench_assemble: CUDA events around them);
 * ``update``     -- k_update (strain, stress, secant update, exit norm) on the
   same plate, R launches after one linear solve;
-* ``cg_cluster`` -- k_c_solve: R block-Jacobi PCG solves of the 64x64 O-grid
+* ``cg_cluster`` -- k_chip: R block-Jacobi PCG solves of the 64x64 O-grid
   plate (8320 DOF) from zero (with the assembly and the secant update of a
   one-iteration cp_solve around each), the whole solve in one thread-block
   cluster; prints the time per CG iteration;
@@ -17,8 +17,8 @@ Cases (each prints one JSON line with its host-side facts):
   visible to the profiler);
 * ``cg_large``   -- k_cg_p / k_cg_u on the 2.1M-DOF plate, R iterations
   (cp_bench_cg), FP64 values or (``--fp32``) the mixed mode's FP32 ones;
-* ``cg_fused_large`` -- k_f_iter, the FP64 form of instances too large for one
-  cluster: R iterations of one block-Jacobi PCG solve on the 2.1M-DOF plate
+* ``cg_fused_large`` -- k_f_iter_half, the FP64 form of large instances numbered
+  along rows: R iterations of one block-Jacobi PCG solve on the 2.1M-DOF plate
   (run with CUPLAST_NO_GRAPH=1 so that every launch is visible);
 * ``cg_mg``      -- the multigrid-preconditioned solve (cp_solve_opts.precond
   2: set-up kernels, then k_mg_p / k_mg_u / k_mg_restrict0 /

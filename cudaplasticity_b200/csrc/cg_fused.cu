@@ -106,9 +106,10 @@ __device__ __forceinline__ double2 ld_other(const double2* p) {
 // follows from its row and slot: 8 and 7 words for the generators' quads, 316
 // bytes per node.
 //
-// kHalfLeast: 147,456 nodes 21.2 us with all of K, 21.3 with the half (quads),
-// 20.7 and 21.1 (triangles); 179,776: 26.7, 24.5 and 23.9, 24.5; 197,136: 28.8,
-// 25.7 and 25.6, 24.4; 230,400: 37.4, 29.0 and 31.9, 26.8.
+// kHalfLeast: 135,424 nodes 20.8 us with all of K, 21.5 with the half (quads);
+// 144,400: 20.9, 21.0; 150,544: 22.3, 21.2; 160,000: 23.4, 23.1; 179,776: 25.7,
+// 25.0, triangles 24.4, 22.8 (147,456: 20.7, 21.1); 197,136: 28.8, 25.7 and 25.0,
+// 22.9; 230,400: 37.4, 29.0 and 31.9, 26.8.
 // kHalfStraight: the share of slices of which no row has more than kChunk
 // blocks on a side. It is 0.95 and more in numberings along rows (rows of 40 to
 // 262,144 nodes), which gain 0.87-0.9 at 1,048,576 nodes. In any other a
@@ -119,7 +120,7 @@ __device__ __forceinline__ double2 ld_other(const double2* p) {
 // (0.00) 93.4 and 93.5 at 460,600 nodes, 180 and 170 at 994,752. At a share of
 // 0.9 a tenth of the worst of these is less than the rest's gain.
 // kHalfWidest: every node takes as many slots as the widest row has.
-constexpr int kHalfLeast = 190000;
+constexpr int kHalfLeast = 150000;
 constexpr double kHalfStraight = 0.9;
 constexpr int kHalfWidest = 9;
 constexpr int kLowShift = 27;  // of a lower slot's word: column below, mirror's upper slot above

@@ -157,7 +157,8 @@ CP_API int cp_context_synchronize(cp_context* ctx);
  * (src/PlasticitySolver.cuh:236-338, src/PlasticitySolver.cu:469-485). */
 CP_API int cp_instance_create(cp_context* ctx, const cp_mesh_view* mesh, const cp_material* mat, cp_instance** out);
 CP_API int cp_instance_destroy(cp_instance* inst);
-/* Device bytes an instance of this mesh holds (for admission control). */
+/* Device bytes that an instance of this mesh holds at most, solves of every form
+ * but precond 2's among them (for admission control). */
 CP_API int cp_instance_footprint(const cp_mesh_view* mesh, int precision, size_t* bytes);
 CP_API int cp_instance_sizes(const cp_instance* inst, int* node_count, int* elem_count, long long* nnz,
                              long long* nadj);
@@ -207,7 +208,7 @@ CP_API int cp_bench_cg(cp_instance* inst, int precision, int precond, int iters,
  * each. Outputs the mean duration of one iteration in milliseconds and the
  * algorithmic bytes one iteration moves: the values (of the diagonal blocks
  * and those right of it alone where the iterations read K's upper half: meshes
- * of 190,000 nodes and more that are numbered along rows) and one 4-byte column
+ * of 150,000 nodes and more that are numbered along rows) and one 4-byte column
  * per 2x2 block, and per node the vectors read and written once. Leaves uv
  * changed. */
 CP_API int cp_bench_cg_fused(cp_instance* inst, int precond, int iters, double* ms_iter, double* bytes_iter);

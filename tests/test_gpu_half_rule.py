@@ -1,5 +1,5 @@
 """Which meshes the one-launch FP64 CG runs on the upper half of K: those
-numbered along rows, from 190,000 nodes, without rows far wider than the rest
+numbered along rows, from 150,000 nodes, without rows far wider than the rest
 (cp_bench_cg_fused reports the bytes of the form that ran). And what the form
 rests on: K is its transpose bit for bit, in any numbering."""
 import ctypes
@@ -61,8 +61,8 @@ def test_numbering(elem, kind, want, ctx):  # noqa: F811
 
 
 def test_size(ctx):  # noqa: F811
-    assert not runs_on_the_half(ctx, strip(380, 499))
-    assert runs_on_the_half(ctx, strip(380, 501))
+    assert not runs_on_the_half(ctx, strip(375, 399))
+    assert runs_on_the_half(ctx, strip(375, 400))
 
 
 def test_one_wide_row(ctx):  # noqa: F811
